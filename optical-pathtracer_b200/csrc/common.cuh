@@ -77,6 +77,15 @@ struct Frame {
 // A rigid transform p' = R p + t, row-major (src/owe/core/math.hpp:114-128).
 struct Xform {
     double m[12];
+    // One coordinate of point() and of vector().
+    template <class T>
+    OWEC_HD T pointRow(int r, const V3<T>& p) const {
+        return T(m[4 * r]) * p.x + T(m[4 * r + 1]) * p.y + T(m[4 * r + 2]) * p.z + T(m[4 * r + 3]);
+    }
+    template <class T>
+    OWEC_HD T vectorRow(int r, const V3<T>& v) const {
+        return T(m[4 * r]) * v.x + T(m[4 * r + 1]) * v.y + T(m[4 * r + 2]) * v.z;
+    }
     template <class T>
     OWEC_HD V3<T> point(const V3<T>& p) const {
         return {T(m[0]) * p.x + T(m[1]) * p.y + T(m[2]) * p.z + T(m[3]),

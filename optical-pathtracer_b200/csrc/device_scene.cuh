@@ -15,7 +15,8 @@ struct alignas(16) PrimRec {
     float bx, by, bz, bw;
     float cx, cy, cz, cw;
 };
-constexpr uint32_t kPrimTriangle = 0u, kPrimAnalytic = 1u;
+// (kPrimPlane: an analytic boundary that is a plane, which the lean traversal tests inline.)
+constexpr uint32_t kPrimTriangle = 0u, kPrimAnalytic = 1u, kPrimPlane = 2u;
 
 // The same triangle in FP64 for the all-FP64 instantiation (leaf order).
 struct alignas(16) PrimRec64 {

@@ -846,7 +846,7 @@ void uploadScene(owec_ctx& c, const owec_scene_desc& d) {
     c.nTriangles = uint32_t(c.primLo.size());
     for (uint32_t i = 0; i < d.n_boundaries; ++i) {
         if (d.boundaries[i].shape == OWEC_SHAPE_MESH) continue;
-        const uint32_t ids[3] = {i, 0u, kPrimAnalytic};
+        const uint32_t ids[3] = {i, 0u, d.boundaries[i].shape == OWEC_SHAPE_PLANE ? kPrimPlane : kPrimAnalytic};
         for (int k = 0; k < 3; ++k) {
             c.triRecs.push_back(make_float4(0.f, 0.f, 0.f, asF(ids[k])));
             for (int a = 0; a < 3; ++a) c.tri64.push_back(0.0);
@@ -1487,7 +1487,6 @@ int owec_open(int device, owec_ctx** out) {
         c->dStats.resize(1);
         c->dScene.resize(1);
         OWEC_CUDA(cudaMemsetAsync(c->dStats.get(), 0, sizeof(StatCounters), c->stream));
-        configureKernels();
         OWEC_CUDA(cudaStreamSynchronize(c->stream));
         *out = c.release();
     });

@@ -20,7 +20,13 @@
 
 namespace owec {
 
-constexpr int kStackDepth = 32;      // group entries per thread in shared memory: one per level
+#ifndef OWEC_STACK_DEPTH
+#define OWEC_STACK_DEPTH 16
+#endif
+// Group entries per thread in shared memory, one per level: 16 levels of eight children cover any tree
+// that is near balanced, and half the former 32 leaves the shared memory to the queries' cold records
+// and the L1.
+constexpr int kStackDepth = OWEC_STACK_DEPTH;
 constexpr int kDeepStackDepth = 96;  // the rare query of a deeper tree is traversed again with a stack
                                      // of this depth in local memory; beyond it the query ends and is
                                      // counted as a fault
@@ -68,6 +74,24 @@ struct HitRec {
     uint32_t slot;        // leaf-order primitive slot
     uint32_t flags;       // kHitFront, kHitAmbiguous (kept by the contact-resolving traversal only)
 };
+// The part of a query that the node loop does not touch: what a primitive test, an accepted
+// crossing or the query's end needs. The persistent kernels keep it in shared memory, one record per
+// thread, which leaves the registers to the node test (at 128 registers kIntersect's spill stores go
+// from 126 to 40 bytes and its local-memory reads to a fifth; 96 or 80 registers for five or six
+// blocks still spill in the node loop and run 10 to 18 % slower). The record is an odd number of
+// 8-byte words, so that a warp's accesses to one field spread over the banks.
+template <class T>
+struct ColdRay {
+    double od[3];
+    ShearedRay<T> sh;
+    T tmax, errN;
+    uint32_t depB, depP, region;
+    HitRec hit;           // written when a crossing is accepted
+    double pad;
+    __device__ __forceinline__ V3<double> origin() const { return V3<double>(od[0], od[1], od[2]); }
+};
+static_assert(sizeof(ColdRay<float>) % 16 == 8 && sizeof(ColdRay<double>) % 16 == 8, "an odd number of 8-byte words");
+
 // The crossing was met from its boundary's front side; it tied with another boundary's crossing that
 // the ray's region matches as well, which leaves their order undecided (NearestCrossing::offer,
 // src/owe/scene/world.cpp:515-550): the reference ends such a path.
@@ -95,18 +119,18 @@ __device__ __forceinline__ T behindWindow(const V3<T>& o) {
 // and not otherwise (a coplanar neighbour, met from behind: the root excludedRoot skips,
 // world.cpp:497-503); the far face of a plate thinner than the anchor's error is met the same way.
 template <class T>
-__device__ __forceinline__ bool acceptCrossing(const DeviceScene& sc, const RayQuery<T>& q, uint32_t b, uint32_t prim, bool mesh, T t,
-                            const V3<T>& n) {
-    if (mesh && b == q.depB && prim == q.depP) return false;
-    const T dn = dot(q.d, n);
+__device__ __forceinline__ bool acceptCrossing(const DeviceScene& sc, const V3<T>& d, T errN, uint32_t depB, uint32_t depP,
+                                               uint32_t region, uint32_t b, uint32_t prim, bool mesh, T t, const V3<T>& n) {
+    if (mesh && b == depB && prim == depP) return false;
+    const T dn = dot(d, n);
     const T nl = sqrt(dot(n, n));
-    const bool near = fabs(t * dn) <= q.errN * nl;
+    const bool near = fabs(t * dn) <= errN * nl;
     if (!near) return true;
-    if (b == q.depB && !mesh) return false;
-    if (q.region == kNone) return true;
+    if (b == depB && !mesh) return false;
+    if (region == kNone) return true;
     const DBoundary& bd = sc.boundaries[b];
     const uint32_t incident = dn < T(0) ? bd.front : bd.back;
-    return incident == q.region;
+    return incident == region;
 }
 
 // Relative widening of far planes against the rounding of the slab distances (a few ulps).
@@ -151,7 +175,7 @@ __device__ __forceinline__ bool analyticCandidate(const DeviceScene& sc, const R
         const AHit<Rr>& h = hits.get(i);
         const V3<T> nw = V3<T>(bd.toWorld.vector(h.n));
         if (Full && !(h.t > Rr(0)) && (b == q.depB || !(fabs(T(h.t) * dot(q.d, nw)) <= behindWindow(q.o)))) continue;
-        if (!acceptCrossing<T>(sc, qs, b, 0u, false, T(h.t), nw)) continue;
+        if (!acceptCrossing<T>(sc, q.d, qs.errN, q.depB, q.depP, q.region, b, 0u, false, T(h.t), nw)) continue;
         tOut = h.t;
         frontOut = dot(q.d, nw) < T(0);
         cosOut = float(fabs(dot(q.d, nw)));
@@ -188,6 +212,32 @@ __device__ __noinline__ AnalyticResult<Rr> analyticHit(const DeviceScene* scp, u
     r.cosAbs = 1.f;
     r.ok = analyticCandidate<R, Rr, T, Full>(*scp, q, b, best, r.t, r.front, r.cosAbs);
     return r;
+}
+
+// analyticCandidate for a plane boundary in the lean instantiation, inline: the crossing from the z
+// rows of the frame alone, and the aperture from the other two only when it lies in (0, best). Planes
+// (walls, floors, lamps, screens) are most of the analytic primitives met, and the out-of-line call with
+// its switch over the shapes costs several times this test. With the cold record in shared memory and
+// the node and primitive tests in one step, the closest-hit kernel takes 12.5 % fewer warp instructions:
+// 7.47 -> 6.97 ms of the 1920 x 1080 room's pass, and kShadowVis with the apply pass 4.61 -> 4.33 ms.
+template <class R, class Rr, class T>
+__device__ __forceinline__ bool planeCrossing(const DeviceScene& sc, const ColdRay<T>& c, const V3<T>& dir, uint32_t b, T best,
+                                              Rr& tOut) {
+    const DBoundary& bd = sc.boundaries[b];
+    const V3<Rr> od(c.origin()), d(dir);
+    const Rr oz = bd.toLocal.pointRow(2, od), dz = bd.toLocal.vectorRow(2, d);
+    if (dz == Rr(0)) return false;
+    const Rr t = -oz / dz;
+    if (t <= Rr(0) || t >= Rr(best)) return false;
+    const Rr px = bd.toLocal.pointRow(0, od) + bd.toLocal.vectorRow(0, d) * t;
+    const Rr py = bd.toLocal.pointRow(1, od) + bd.toLocal.vectorRow(1, d) * t;
+    if (!inPlaneAperture(int(bd.params[0]), Rr(bd.params[1]), Rr(bd.params[2]), Rr(0), Rr(0), V3<Rr>(px, py, Rr(0)))) return false;
+    T errN = c.errN;
+    if (b == c.depB && sizeof(Rr) > sizeof(R)) errN *= T(2.5e-7);
+    const V3<T> n(T(Rr(bd.toWorld.m[2])), T(Rr(bd.toWorld.m[6])), T(Rr(bd.toWorld.m[10])));
+    if (!acceptCrossing<T>(sc, dir, errN, c.depB, c.depP, c.region, b, 0u, false, T(t), n)) return false;
+    tOut = t;
+    return true;
 }
 
 // A wide node as the five 128-bit words it is loaded in (the WideNode layout of device_scene.cuh):
@@ -361,13 +411,12 @@ __device__ __forceinline__ uint32_t permuteSlots(uint32_t m, uint32_t x) {
 // (analyticCrossings).
 template <class T, class R, class Rr, bool AnyHit, class Stack = SharedStack, bool Count = true, bool Full = false>
 struct Traversal {
-    RayQuery<T> q;
+    V3<T> o, d;           // the ray, camera-relative
     V3<T> inv, oinv;
-    ShearedRay<T> sh;
     T best;
     T bestCos;            // contact-resolving instantiation: |cos| of the closest crossing's incidence
     double bestD;         // and its distance in the refinement's precision
-    HitRec hit;           // written when a crossing is accepted
+    ColdRay<T>* c;        // the rest of the query and the closest crossing so far
     Stack st;
     uint32_t nodeBase, nodeBits;  // the current node group (as a stack entry)
     uint32_t primBase, primBits;  // the current primitive group: primBase + bit, 24 bits
@@ -376,12 +425,23 @@ struct Traversal {
     int sp;
     bool found;
 
-    // `stack` is this thread's column of the block's shared-memory stack (stride = block size).
-    __device__ __forceinline__ void begin(const RayQuery<T>& query, StackEntry* stack, int stride) {
-        q = query;
-        inv = V3<T>(safeInverse(q.d.x), safeInverse(q.d.y), safeInverse(q.d.z));
-        oinv = V3<T>(q.o.x * inv.x, q.o.y * inv.y, q.o.z * inv.z);
-        sh = shearRay(q.d);
+    // `stack` is this thread's column of the block's shared-memory stack (stride = block size), `cold`
+    // this thread's record.
+    __device__ __forceinline__ void begin(const RayQuery<T>& q, StackEntry* stack, int stride, ColdRay<T>* cold) {
+        c = cold;
+        c->od[0] = q.od.x;
+        c->od[1] = q.od.y;
+        c->od[2] = q.od.z;
+        c->sh = shearRay(q.d);
+        c->tmax = q.tmax;
+        c->errN = q.errN;
+        c->depB = q.depB;
+        c->depP = q.depP;
+        c->region = q.region;
+        o = q.o;
+        d = q.d;
+        inv = V3<T>(safeInverse(d.x), safeInverse(d.y), safeInverse(d.z));
+        oinv = V3<T>(o.x * inv.x, o.y * inv.y, o.z * inv.z);
         best = q.tmax;
         bestCos = T(1);
         bestD = double(q.tmax);
@@ -391,7 +451,7 @@ struct Traversal {
         nodeVisits = primTests = 0;
         steps = 0;
         // bit k set: the ray runs towards +k, so it meets the children on the negative side first
-        first = ((q.d.x < T(0)) ? 0u : 1u) | ((q.d.y < T(0)) ? 0u : 2u) | ((q.d.z < T(0)) ? 0u : 4u);
+        first = ((d.x < T(0)) ? 0u : 1u) | ((d.y < T(0)) ? 0u : 2u) | ((d.z < T(0)) ? 0u : 4u);
         // the root as a group of one: position 0, an inner slot of rank 0
         nodeBase = 0;
         nodeBits = 1u | (1u << (8 + first));
@@ -399,51 +459,68 @@ struct Traversal {
         primBits = 0;
     }
 
-    // Advances by at most `budget` node or primitive visits: kTraceRunning, or the query's TraceStatus.
+    // The query as begin() took it.
+    __device__ __forceinline__ RayQuery<T> query() const {
+        RayQuery<T> q;
+        q.o = o;
+        q.d = d;
+        q.od = c->origin();
+        q.tmax = c->tmax;
+        q.depB = c->depB;
+        q.depP = c->depP;
+        q.region = c->region;
+        q.errN = c->errN;
+        return q;
+    }
+
+    // Advances by at most `budget` steps: kTraceRunning, or the query's TraceStatus. A step visits a
+    // node, unless primitives of the last one are left, and then tests one primitive: the lanes of a
+    // warp that just met a leaf go on with it in the same step instead of waiting for the others' nodes.
     __device__ __forceinline__ int run(const DeviceScene& sc, int budget) {
         if (sc.nNodes == 0) return kTraceMiss;
         for (int it = 0; it < budget; ++it) {
             if (++steps > kMaxTraversalSteps) return kTraceOverflow;
+            if (primBits == 0) {
+                if ((nodeBits & 0xFFu) == 0) {
+                    if (sp == 0) return found ? kTraceHit : kTraceMiss;
+                    --sp;
+                    const StackEntry e = st.get(sp);
+                    nodeBase = e.base;
+                    nodeBits = e.bits;
+                }
+                // the group's next child in visiting order; the rest of the group waits on the stack
+                const uint32_t pos = uint32_t(__ffs(nodeBits & 0xFFu) - 1);
+                nodeBits &= ~(1u << pos);
+                const uint32_t slot = pos ^ first;
+                const uint32_t node = nodeBase + uint32_t(__popc((nodeBits >> 8) & ((1u << slot) - 1u)));
+                if (nodeBits & 0xFFu) {
+                    if (sp >= Stack::kDepth) return kTraceOverflow;
+                    st.set(sp, {nodeBase, nodeBits});
+                    ++sp;
+                }
+                NodeWords nd;
+                loadNode(sc.nodes, node, nd);
+                if (Count) ++nodeVisits;
+                const uint32_t mask = intersectChildren(nd, inv, oinv, T(0), (Full && !AnyHit) ? tieLimit() : best);
+                const uint32_t inner = nd.a.w >> 24;
+                nodeBase = nd.b.x;
+                nodeBits = permuteSlots(mask & inner, first) | (inner << 8);
+                primBase = nd.b.y;
+                uint32_t pb = 0;
+                // the hit leaf slots' primitive ranges (meta: count << 5 | offset), one leaf at a time
+                for (uint32_t leaves = mask & ~inner; leaves; leaves &= leaves - 1u) {
+                    const uint32_t i = uint32_t(__ffs(leaves) - 1);
+                    const uint32_t meta = ((i < 4 ? nd.b.z : nd.b.w) >> (8 * (i & 3))) & 0xFFu;
+                    pb |= ((1u << (meta >> 5)) - 1u) << (meta & 31u);
+                }
+                primBits = pb;
+            }
             if (primBits) {
                 const uint32_t b = uint32_t(__ffs(primBits) - 1);
                 primBits &= primBits - 1u;
                 if (Count) ++primTests;
                 if (testPrim(sc, primBase + b) && AnyHit) return kTraceHit;
-                continue;
             }
-            if ((nodeBits & 0xFFu) == 0) {
-                if (sp == 0) return found ? kTraceHit : kTraceMiss;
-                --sp;
-                const StackEntry e = st.get(sp);
-                nodeBase = e.base;
-                nodeBits = e.bits;
-            }
-            // the group's next child in visiting order; the rest of the group waits on the stack
-            const uint32_t pos = uint32_t(__ffs(nodeBits & 0xFFu) - 1);
-            nodeBits &= ~(1u << pos);
-            const uint32_t slot = pos ^ first;
-            const uint32_t node = nodeBase + uint32_t(__popc((nodeBits >> 8) & ((1u << slot) - 1u)));
-            if (nodeBits & 0xFFu) {
-                if (sp >= Stack::kDepth) return kTraceOverflow;
-                st.set(sp, {nodeBase, nodeBits});
-                ++sp;
-            }
-            NodeWords nd;
-            loadNode(sc.nodes, node, nd);
-            if (Count) ++nodeVisits;
-            const uint32_t mask = intersectChildren(nd, inv, oinv, T(0), (Full && !AnyHit) ? tieLimit() : best);
-            const uint32_t inner = nd.a.w >> 24;
-            nodeBase = nd.b.x;
-            nodeBits = permuteSlots(mask & inner, first) | (inner << 8);
-            primBase = nd.b.y;
-            uint32_t pb = 0;
-            // the hit leaf slots' primitive ranges (meta: count << 5 | offset), one leaf at a time
-            for (uint32_t leaves = mask & ~inner; leaves; leaves &= leaves - 1u) {
-                const uint32_t i = uint32_t(__ffs(leaves) - 1);
-                const uint32_t meta = ((i < 4 ? nd.b.z : nd.b.w) >> (8 * (i & 3))) & 0xFFu;
-                pb |= ((1u << (meta >> 5)) - 1u) << (meta & 31u);
-            }
-            primBits = pb;
         }
         return kTraceRunning;
     }
@@ -455,23 +532,23 @@ struct Traversal {
 
     // The magnitude of the coordinates a crossing's distance is computed from (origin and hit point).
     __device__ __forceinline__ double coordScale() const {
-        return fmax(fmax(fabs(q.od.x), fabs(q.od.y)), fabs(q.od.z)) + fmin(fabs(bestD), 1e30);
+        return fmax(fmax(fabs(c->od[0]), fabs(c->od[1])), fabs(c->od[2])) + fmin(fabs(bestD), 1e30);
     }
 
     // The tie window of two crossings' distances: coincident faces' distances differ by the rounding
     // of their offsets over the cosine of incidence. With FP64 distances, the reference's contact
     // error, 64 ulps of the coordinates' magnitude (contactError, src/owe/core/math.hpp:15,
     // NearestCrossing::offer, src/owe/scene/world.cpp:526); plain FP32 keeps a relative window.
-    __device__ __forceinline__ double tieSpanD(T c) const {
-        if constexpr (kExactTies) return 64 * 2.220446049250313e-16 * fmax(coordScale(), 1e-3) / fmax(double(c), 1e-3);
-        else return fabs(bestD) * double(tieWindow<T>()) / fmax(double(c), 1e-3);
+    __device__ __forceinline__ double tieSpanD(T cs) const {
+        if constexpr (kExactTies) return 64 * 2.220446049250313e-16 * fmax(coordScale(), 1e-3) / fmax(double(cs), 1e-3);
+        else return fabs(bestD) * double(tieWindow<T>()) / fmax(double(cs), 1e-3);
     }
 
     // How far beyond the closest crossing the contact-resolving traversal still looks (node culling
     // and the crossings it admits): the tie window in the traversal's precision, and with FP64
     // decisions at least the FP64 window plus, for FP32 traversal, its distances' own rounding (a few
     // ulps of the coordinates' magnitude), so that every near tie reaches the FP64 test.
-    __device__ __forceinline__ T tieSpan(T c) const {
+    __device__ __forceinline__ T tieSpan(T cs) const {
         // |best|: a crossing just behind the anchor (a contact through it) may be the closest
         T s = fabs(best) * tieWindow<T>();
         if constexpr (kExactTies) {
@@ -479,25 +556,26 @@ struct Traversal {
             s += T(64 * 2.220446049250313e-16) * scale;
             if constexpr (sizeof(T) == sizeof(float)) s += T(1e-6) * scale;
         }
-        return s / fmax(c, T(1e-3));
+        return s / fmax(cs, T(1e-3));
     }
     __device__ __forceinline__ T tieLimit() const { return best + tieSpan(bestCos); }
 
-    // Whether boundary b's crossing at t, met from its front side when `front` at incidence |cos| c,
+    // Whether boundary b's crossing at t, met from its front side when `front` at incidence |cos| cs,
     // replaces the current closest (the contact-resolving instantiation; NearestCrossing::offer,
     // src/owe/scene/world.cpp:515-550). Crossings of different boundaries within the tie span are
     // one contact: the one met from the ray's region wins, matter wins over a zero-thickness
     // readout, then the lower boundary index; two that both match leave the order undecided
     // (kHitAmbiguous). `flags` receives the winner's flags.
-    __device__ __forceinline__ bool winsContact(const DeviceScene& sc, uint32_t b, double tD, bool front, T c,
+    __device__ __forceinline__ bool winsContact(const DeviceScene& sc, uint32_t b, double tD, bool front, T cs,
                                                 uint32_t& flags) {
         const uint32_t frontFlag = front ? kHitFront : 0u;
+        HitRec& hit = c->hit;
         // outside the tie window, or two crossings of one boundary: the nearer one
-        if (!found || b == hit.boundary || !(fabs(tD - bestD) <= tieSpanD(fmin(c, bestCos)))) {
+        if (!found || b == hit.boundary || !(fabs(tD - bestD) <= tieSpanD(fmin(cs, bestCos)))) {
             flags = frontFlag;
             return !found || tD < bestD;
         }
-        const bool hinted = q.region != kNone;
+        const bool hinted = c->region != kNone;
         auto incident = [&](uint32_t bb, bool fr) {
             const DBoundary& bd = sc.boundaries[bb];
             return fr ? bd.front : bd.back;
@@ -506,8 +584,8 @@ struct Traversal {
             const DBoundary& bd = sc.boundaries[bb];
             return sc.optics[bd.optics].type == OWEC_SURF_DETECTOR && bd.front == bd.back;
         };
-        const bool mNew = !hinted || incident(b, front) == q.region;
-        const bool mOld = !hinted || incident(hit.boundary, hit.flags & kHitFront) == q.region;
+        const bool mNew = !hinted || incident(b, front) == c->region;
+        const bool mOld = !hinted || incident(hit.boundary, hit.flags & kHitFront) == c->region;
         const bool rNew = readout(b), rOld = readout(hit.boundary);
         bool ambiguous = hit.flags & kHitAmbiguous;
         if (mNew && mOld && rNew != rOld) {
@@ -533,7 +611,7 @@ struct Traversal {
             const PrimRec64& p = sc.prims64[i];
             const V3<double> v0(p.v0[0], p.v0[1], p.v0[2]), v1(p.v1[0], p.v1[1], p.v1[2]), v2(p.v2[0], p.v2[1], p.v2[2]);
             const V3<double> n = triangleNormal(v0, v1, v2);
-            const double tD = dot(v0 - q.od, n) / dot(V3<double>(q.d), n);
+            const double tD = dot(v0 - c->origin(), n) / dot(V3<double>(d), n);
             return fabs(tD - double(t)) <= 1e-3 * (1 + fabs(double(t))) ? tD : double(t);
         } else {
             return double(t);
@@ -551,28 +629,34 @@ struct Traversal {
         const T limit = (Full && !AnyHit) ? tieLimit() : best;
         uint32_t flags = 0;
         if (kind == kPrimTriangle) {
-            const V3<T> a = v0 - q.o, bb = v1 - q.o, c = v2 - q.o;
-            if (!lineCrossesTriangle(sh, a, bb, c)) return false;
+            const V3<T> a0 = v0 - o, a1 = v1 - o, a2 = v2 - o;
+            if (!lineCrossesTriangle(c->sh, a0, a1, a2)) return false;
             const V3<T> n = triangleNormal(v0, v1, v2);
-            const T dn = dot(q.d, n);
-            const T t = -dot(q.o - v0, n) / dn;
+            const T dn = dot(d, n);
+            const T t = -dot(o - v0, n) / dn;
             // contacts: another boundary's face through the anchor may fall just behind it
-            if (!((Full ? t > T(0) || (b != q.depB && fabs(t * dn) <= behindWindow(q.o) * sqrt(dot(n, n))) : t > T(0)) &&
+            if (!((Full ? t > T(0) || (b != c->depB && fabs(t * dn) <= behindWindow(o) * sqrt(dot(n, n))) : t > T(0)) &&
                   t < limit))
                 return false;
-            if (!acceptCrossing<T>(sc, q, b, prim, true, t, n)) return false;
+            if (!acceptCrossing<T>(sc, d, c->errN, c->depB, c->depP, c->region, b, prim, true, t, n)) return false;
             if constexpr (Full) {
-                const T c = fabs(dn) / sqrt(dot(n, n));
+                const T cs = fabs(dn) / sqrt(dot(n, n));
                 const double tD = refinedTriangleT(sc, i, t);
-                if (!winsContact(sc, b, tD, dn < T(0), c, flags)) return false;
-                bestCos = c;
+                if (!winsContact(sc, b, tD, dn < T(0), cs, flags)) return false;
+                bestCos = cs;
                 bestD = tD;
             }
             best = t;
-            hit.t = double(t);
-            hit.prim = prim;
+            c->hit.t = double(t);
+            c->hit.prim = prim;
+        } else if (!Full && kind == kPrimPlane) {
+            Rr t;
+            if (!planeCrossing<R, Rr, T>(sc, *c, d, b, limit, t)) return false;
+            best = T(t);
+            c->hit.t = double(t);
+            c->hit.prim = 0;
         } else {
-            const AnalyticResult<Rr> ar = analyticHit<T, R, Rr, Full>(sc.self, b, q.od, q.d, limit, q.depB, q.region, q.errN);
+            const AnalyticResult<Rr> ar = analyticHit<T, R, Rr, Full>(sc.self, b, c->origin(), d, limit, c->depB, c->region, c->errN);
             if (!ar.ok) return false;
             if constexpr (Full) {
                 if (!winsContact(sc, b, double(ar.t), ar.front, T(ar.cosAbs), flags)) return false;
@@ -580,12 +664,12 @@ struct Traversal {
                 bestD = double(ar.t);
             }
             best = T(ar.t);
-            hit.t = double(ar.t);
-            hit.prim = 0;
+            c->hit.t = double(ar.t);
+            c->hit.prim = 0;
         }
-        if constexpr (Full) hit.flags = flags;
-        hit.boundary = b;
-        hit.slot = i;
+        if constexpr (Full) c->hit.flags = flags;
+        c->hit.boundary = b;
+        c->hit.slot = i;
         found = true;
         return true;
     }
@@ -603,14 +687,15 @@ template <class T, class R, class Rr, bool AnyHit, bool Full = false>
 __device__ __noinline__ DeepResult traceRayDeep(const DeviceScene* scp, RayQuery<T> q, HitRec hitIn) {
     const DeviceScene& sc = *scp;
     Traversal<T, R, Rr, AnyHit, LocalStack, true, Full> tr;
-    tr.begin(q, nullptr, 0);
-    tr.hit = hitIn;
+    ColdRay<T> cold;
+    tr.begin(q, nullptr, 0, &cold);
+    cold.hit = hitIn;
     int s;
     do {
         s = tr.run(sc, 1 << 30);
     } while (s == kTraceRunning);
     DeepResult r;
-    r.hit = tr.hit;
+    r.hit = cold.hit;
     r.status = s;
     r.visits = tr.nodeVisits;
     r.tests = tr.primTests;
@@ -622,8 +707,9 @@ template <class T, class R, class Rr, bool AnyHit, bool Full = false>
 __device__ __forceinline__ int traceRay(const DeviceScene& sc, const RayQuery<T>& q, StackEntry* stack, int stride, HitRec& hit,
                                         uint32_t* visits = nullptr, uint32_t* tests = nullptr) {
     Traversal<T, R, Rr, AnyHit, SharedStack, true, Full> tr;
-    tr.begin(q, stack, stride);
-    tr.hit = hit;
+    ColdRay<T> cold;
+    tr.begin(q, stack, stride, &cold);
+    cold.hit = hit;
     int s;
     do {
         s = tr.run(sc, 1 << 30);
@@ -636,7 +722,7 @@ __device__ __forceinline__ int traceRay(const DeviceScene& sc, const RayQuery<T>
         nv += d.visits;
         nt += d.tests;
     } else {
-        hit = tr.hit;
+        hit = cold.hit;
     }
     if (visits) *visits += nv;
     if (tests) *tests += nt;

@@ -56,10 +56,11 @@ __global__ void __launch_bounds__(256) kGenerate(DeviceScene sc, PassParams pp, 
 }
 
 // ------------------------------------------------------------------ intersect
-// Visits a lane makes between two refills of its warp: small enough that a finished lane does not
-// idle long, large enough to amortise the refill's vote, atomic and ray load.
+// Steps (a node and a primitive) a lane makes between two refills of its warp: small enough that a
+// finished lane does not idle long, large enough to amortise the refill's vote, atomic and ray load.
+// The 1920 x 1080 room's pass: 4 steps 16.91 ms, 6 16.83, 8 16.97, 12 17.61.
 #ifndef OWEC_REFILL_BUDGET
-#define OWEC_REFILL_BUDGET 8
+#define OWEC_REFILL_BUDGET 6
 #endif
 constexpr int kRefillBudget = OWEC_REFILL_BUDGET;
 // Resident blocks per SM the traversal kernels are compiled for (a register cap of
@@ -93,6 +94,12 @@ __device__ __forceinline__ uint32_t refillLanes(bool idle, uint32_t* fetch, uint
     return idle ? base + uint32_t(__popc(need & ((1u << lane) - 1u))) : n;
 }
 
+// This thread's record behind the block's traversal stacks (persistentSharedBytes).
+template <class R>
+__device__ __forceinline__ ColdRay<R>* coldRay(StackEntry* stackMem) {
+    return reinterpret_cast<ColdRay<R>*>(stackMem + size_t(kStackDepth) * blockDim.x) + threadIdx.x;
+}
+
 // Adds a per-lane count to a counter, one atomic per warp (all lanes of the warp present).
 __device__ __forceinline__ void warpFlush(unsigned long long* counter, uint32_t v) {
     const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, v);
@@ -108,6 +115,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kIntersect(DeviceScene sc, PathBuffers<RT<
     using R = RT<M>;
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
+    ColdRay<R>* cold = coldRay<R>(stackMem);
     const uint32_t n = q.counts[cur];
     Traversal<R, typename Mode<M>::Ro, typename Mode<M>::Rr, false, SharedStack, Count, Full> tr;
     uint32_t path = 0, segments = 0, faults = 0;
@@ -126,19 +134,19 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kIntersect(DeviceScene sc, PathBuffers<RT<
             rq.depP = ray.depP;
             rq.region = ray.region;
             rq.errN = R(ray.errN);
-            tr.begin(rq, stack, blockDim.x);
+            tr.begin(rq, stack, blockDim.x, cold);
             alive = true;
         }
         if (__ballot_sync(0xFFFFFFFFu, alive) == 0) break;
         if (alive) {
             int s = tr.run(sc, kRefillBudget);
             if (s != kTraceRunning) {
-                HitRec h = tr.hit;
+                HitRec h = cold->hit;
                 uint32_t nv = tr.nodeVisits, nt = tr.primTests;
                 if (s == kTraceOverflow) {
                     h.boundary = kNone;
                     h.t = INFINITY;
-                    const DeepResult d = traceRayDeep<R, typename Mode<M>::Ro, typename Mode<M>::Rr, false, Full>(sc.self, tr.q, h);
+                    const DeepResult d = traceRayDeep<R, typename Mode<M>::Ro, typename Mode<M>::Rr, false, Full>(sc.self, tr.query(), h);
                     s = d.status;
                     h = d.hit;
                     nv += d.visits;
@@ -566,6 +574,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadow(DeviceScene sc, PassParams pp, Pat
     using Rr = typename Mode<M>::Rr;
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
+    ColdRay<R>* cold = coldRay<R>(stackMem);
     const uint32_t n = q.counts[3];
     Traversal<R, Ro, Rr, AnyHit, SharedStack, Count, Full> tr;
     // the light point's identity decides (the Full instantiation's next-event rays)
@@ -605,11 +614,11 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadow(DeviceScene sc, PassParams pp, Pat
         if (!begin) {
             int s = tr.run(sc, kRefillBudget);
             if (s == kTraceRunning) continue;
-            HitRec h = tr.hit;
+            HitRec h = cold->hit;
             uint32_t nv = tr.nodeVisits, nt = tr.primTests;
             if (s == kTraceOverflow) {
                 h.boundary = kNone;
-                const DeepResult d = traceRayDeep<R, Ro, Rr, AnyHit, Full>(sc.self, tr.q, h);
+                const DeepResult d = traceRayDeep<R, Ro, Rr, AnyHit, Full>(sc.self, tr.query(), h);
                 s = d.status;
                 h = d.hit;
                 nv += d.visits;
@@ -651,15 +660,15 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadow(DeviceScene sc, PassParams pp, Pat
                         } else {
                             // pass the null boundary, if met from this region
                             PathRay<R> tmp;
-                            tmp.o[0] = tr.q.od.x; tmp.o[1] = tr.q.od.y; tmp.o[2] = tr.q.od.z;
-                            tmp.d[0] = tr.q.d.x; tmp.d[1] = tr.q.d.y; tmp.d[2] = tr.q.d.z;
+                            for (int j = 0; j < 3; ++j) tmp.o[j] = cold->od[j];
+                            tmp.d[0] = tr.d.x; tmp.d[1] = tr.d.y; tmp.d[2] = tr.d.z;
                             const SurfacePoint<R> gp = hitGeometry<R, Ro, Rr, Full>(sc, tmp, h);
-                            const bool ff = dot(tr.q.d, gp.n) < R(0);
+                            const bool ff = dot(tr.d, gp.n) < R(0);
                             if ((ff ? bd.front : bd.back) != region) {
                                 outcome = 2;
                             } else {
                                 region = ff ? bd.back : bd.front;
-                                rq = tr.q;
+                                rq = tr.query();
                                 rq.od = gp.p;
                                 if (Mode<M>::plainOrigin) rq.od = V3<double>(V3<float>(gp.p));
                                 rq.o = V3<R>(rq.od);
@@ -686,7 +695,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadow(DeviceScene sc, PassParams pp, Pat
             } else {
                 rq.tmax = R(tq);
                 rq.region = region;
-                tr.begin(rq, stack, blockDim.x);
+                tr.begin(rq, stack, blockDim.x, cold);
             }
         }
         if (outcome != 0) {
@@ -721,6 +730,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadowVis(DeviceScene sc, PathBuffers<RT<
     using Rr = typename Mode<M>::Rr;
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
+    ColdRay<R>* cold = coldRay<R>(stackMem);
     const uint32_t n = q.counts[3];
     Traversal<R, Ro, Rr, true, SharedStack, Count, Full> tr;
     uint32_t job = 0;
@@ -746,7 +756,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadowVis(DeviceScene sc, PathBuffers<RT<
                 rq.errN = R(sr.errN);
                 rq.tmax = R(tq);
                 rq.region = sr.region;
-                tr.begin(rq, stack, blockDim.x);
+                tr.begin(rq, stack, blockDim.x, cold);
                 alive = true;
             }
         }
@@ -756,9 +766,9 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadowVis(DeviceScene sc, PathBuffers<RT<
         if (s == kTraceRunning) continue;
         uint32_t nv = tr.nodeVisits, nt = tr.primTests;
         if (s == kTraceOverflow) {
-            HitRec h = tr.hit;
+            HitRec h = cold->hit;
             h.boundary = kNone;
-            const DeepResult d = traceRayDeep<R, Ro, Rr, true, Full>(sc.self, tr.q, h);
+            const DeepResult d = traceRayDeep<R, Ro, Rr, true, Full>(sc.self, tr.query(), h);
             s = d.status;
             nv += d.visits;
             nt += d.tests;
@@ -997,6 +1007,9 @@ __global__ void __launch_bounds__(256) kResolve(const double* film, const double
 
 // ------------------------------------------------------------------ launchers
 size_t traversalSharedBytes(int block) { return size_t(block) * kStackDepth * sizeof(StackEntry); }
+// The persistent kernels': the stacks and the queries' cold records.
+template <int M>
+size_t persistentSharedBytes(int block) { return traversalSharedBytes(block) + size_t(block) * sizeof(ColdRay<RT<M>>); }
 
 template <int M>
 void launchGenerate(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
@@ -1006,7 +1019,7 @@ void launchGenerate(const DeviceScene& sc, const PassParams& pp, const PathBuffe
 template <int M>
 void launchIntersect(const DeviceScene& sc, const PathBuffers<RT<M>>& pb, const Queues& q, int cur, StatCounters* st,
                      uint32_t* fetch, int grid, cudaStream_t s) {
-    const size_t smem = traversalSharedBytes(128);
+    const size_t smem = persistentSharedBytes<M>(128);
     if (sc.fullFeatures) {
         if (sc.travCounters) kIntersect<M, true, true><<<grid, 128, smem, s>>>(sc, pb, q, cur, st, fetch);
         else kIntersect<M, false, true><<<grid, 128, smem, s>>>(sc, pb, q, cur, st, fetch);
@@ -1036,7 +1049,7 @@ void launchSurface(const DeviceScene& sc, const PassParams& pp, const PathBuffer
 template <int M, bool Splat, bool Count, bool Full>
 void shadowKernelsOf(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
                      StatCounters* st, uint32_t* fetch, uint8_t* vis, const SplatTarget& film, int grid, cudaStream_t s) {
-    const size_t smem = traversalSharedBytes(128);
+    const size_t smem = persistentSharedBytes<M>(128);
     // next-event rays of a scene with contacts take the ordered walk, where the light point's
     // identity decides what lies at its end
     if (pp.anyHitShadows && !(Full && !Splat)) {
@@ -1101,16 +1114,6 @@ void launchMaterialize(const uint32_t* leafOrder, uint32_t n, const float4* tri,
                        PrimRec64* prims64, cudaStream_t s) {
     kMaterialize<<<(n + 255) / 256, 256, 0, s>>>(leafOrder, n, tri, tri64, prims, prims64);
 }
-void configureKernels() {
-    const int smem = int(traversalSharedBytes(128));
-    cudaFuncSetAttribute(kIntersect<0, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(kIntersect<1, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(kIntersect<2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(kIntersect<0, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(kIntersect<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(kIntersect<2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-}
-
 #define OWEC_INSTANTIATE(M)                                                                                         \
     template void launchGenerate<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&, \
                                     StatCounters*, cudaStream_t);                                                   \

@@ -12,7 +12,6 @@ template <int M>
 using ModeR = typename Mode<M>::R;
 
 size_t traversalSharedBytes(int block);
-void configureKernels();
 
 template <int M>
 void launchGenerate(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&, StatCounters*,
