@@ -65,17 +65,23 @@ __global__ void kCentroidBounds(const float4* lo, const float4* hi, uint32_t n, 
         const float c[3] = {0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z)};
         for (int k = 0; k < 3; ++k) { mn[k] = fminf(mn[k], c[k]); mx[k] = fmaxf(mx[k], c[k]); }
     }
+    // one set of atomics per block: with one per warp the six addresses took most of the kernel's time
+    __shared__ int part[6][8];
     for (int k = 0; k < 3; ++k) {
-        for (int off = 16; off > 0; off >>= 1) {
-            mn[k] = fminf(mn[k], __shfl_xor_sync(0xFFFFFFFFu, mn[k], off));
-            mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xFFFFFFFFu, mx[k], off));
+        const int l = __reduce_min_sync(0xFFFFFFFFu, floatToOrdered(mn[k]));
+        const int h = __reduce_max_sync(0xFFFFFFFFu, floatToOrdered(mx[k]));
+        if ((threadIdx.x & 31) == 0) {
+            part[k][threadIdx.x >> 5] = l;
+            part[3 + k][threadIdx.x >> 5] = h;
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-        for (int k = 0; k < 3; ++k) {
-            atomicMin(bounds + k, floatToOrdered(mn[k]));
-            atomicMax(bounds + 3 + k, floatToOrdered(mx[k]));
-        }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int k = threadIdx.x, warps = int(blockDim.x >> 5);
+        int v = part[k][0];
+        for (int w = 1; w < warps; ++w) v = k < 3 ? min(v, part[k][w]) : max(v, part[k][w]);
+        if (k < 3) atomicMin(bounds + k, v);
+        else atomicMax(bounds + k, v);
     }
 }
 
@@ -193,6 +199,11 @@ __device__ __forceinline__ uint32_t scaleExponent(float ext) {
     return uint32_t(biased);
 }
 
+// The build's counters: [0] wide nodes allocated, [1] primitives placed, [2 + level] the wide nodes of
+// a level still to be made from their binary nodes.
+constexpr uint32_t kMaxLevels = 4096;
+constexpr uint32_t kCounters = 2 + kMaxLevels + 2;
+
 struct CollapseArgs {
     const int2* children;
     const int2* ranges;
@@ -200,133 +211,225 @@ struct CollapseArgs {
     const float4* boxHi;
     const uint32_t* counts;
     const uint32_t* vals;
+    const uint32_t* errors;  // kBottomUp's report: nothing is collapsed from a malformed tree
     int n;
     WideNode* nodes;
     uint32_t* leafOrder;
-    uint32_t* counters;  // [0] nodes allocated, [1] primitives placed, [2] next work count
-    uint2* work;         // (binary node, wide node)
-    uint2* next;
+    uint32_t* counters;
 };
 
-__global__ void kCollapse(CollapseArgs a, uint32_t nWork) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= nWork) return;
-    const uint2 item = a.work[w];
+// Sets what the build's kernels start from: the empty bounds, the counters and the root's work item.
+__global__ void kBeginBuild(int* bounds, uint32_t* counters, uint2* work) {
+    for (uint32_t i = threadIdx.x; i < kCounters; i += blockDim.x) counters[i] = i == 0 || i == 2 ? 1u : 0u;
+    if (threadIdx.x < 6) bounds[threadIdx.x] = threadIdx.x < 3 ? 0x7F800000 : int(0x807FFFFFu);  // +inf, -inf
+    // the binary root: inner node 0, or with one primitive its leaf (combined index n - 1 = 0)
+    if (threadIdx.x == 0) work[0] = make_uint2(0u, 0u);
+}
+
+// One level of wide nodes, eight lanes to a node, a lane to a child. The widest levels hold n / 8 nodes
+// and the first ones 1, 8, 64: with one thread per node a level lasted as long as its node's chain of
+// dependent loads, eight openings and the 8 x 8 auction from local memory (about 50 us), whatever its
+// width. The level's node count is read on the device, so the host queues levels without waiting.
+// owec_set_heightfield of a 256 x 256 heightfield (262,141 primitives in the scene): 9.80 -> 0.56 ms with
+// kDeformHeightfield; the seven levels alone were 0.40 ms of kernel time and a host round trip each.
+__global__ void __launch_bounds__(128) kCollapse(CollapseArgs a, int level, const uint2* work, uint2* next) {
+    // work: the (binary node, wide node) pairs of this level, next: those of the one below
+    const uint32_t nWork = *a.errors >= 0x10000u ? 0u : a.counters[2 + level];
     const int n = a.n;
-    int c[8];
-    int nc;
-    if (int(item.x) >= n - 1) {  // a single-leaf root
-        c[0] = int(item.x);
-        nc = 1;
-    } else {
-        const int2 ch = a.children[item.x];
-        c[0] = ch.x;
-        c[1] = ch.y;
-        nc = 2;
+    const uint32_t lane = threadIdx.x & 7u;
+    const uint32_t group = 0xFFu << (threadIdx.x & 24u);  // the node's eight lanes
+    const int lead = int(threadIdx.x & 24u);              // their first lane
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; w < nWork; w += (gridDim.x * blockDim.x) >> 3) {
+        const uint2 item = work[w];
+        int c = -1;  // this lane's child
+        int nc;
+        if (int(item.x) >= n - 1) {  // a single-leaf root
+            if (lane == 0) c = int(item.x);
+            nc = 1;
+        } else {
+            const int2 ch = a.children[item.x];
+            if (lane < 2) c = lane == 0 ? ch.x : ch.y;
+            nc = 2;
+        }
+        float4 l = make_float4(INFINITY, INFINITY, INFINITY, 0.f), h = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+        uint32_t cnt = 0;
+        if (c >= 0) { l = a.boxLo[c]; h = a.boxHi[c]; cnt = a.counts[c]; }
+        // open the largest openable child (the first of equals) until there are eight
         while (nc < 8) {
-            int best = -1;
-            float bestArea = -1.f;
-            for (int i = 0; i < nc; ++i) {
-                if (c[i] >= n - 1 || a.counts[c[i]] <= kLeafMax) continue;
-                const float ar = halfArea(a.boxLo[c[i]], a.boxHi[c[i]]);
-                if (ar > bestArea) { bestArea = ar; best = i; }
-            }
-            if (best < 0) break;
-            const int2 ch2 = a.children[c[best]];
-            c[best] = ch2.x;
-            c[nc++] = ch2.y;
+            float area = c >= 0 && c < n - 1 && cnt > kLeafMax ? halfArea(l, h) : -1.f;
+            if (!(area > -1.f)) area = -1.f;
+            float best = area;
+            for (int off = 4; off > 0; off >>= 1) best = fmaxf(best, __shfl_xor_sync(group, best, off));
+            if (!(best > -1.f)) break;
+            const int src = __ffs(__ballot_sync(group, area == best) & group) - 1;
+            const int2 ch = a.children[__shfl_sync(group, c, src)];
+            if (int(threadIdx.x & 31u) == src) c = ch.x;
+            else if (int(lane) == nc) c = ch.y;
+            if (int(threadIdx.x & 31u) == src || int(lane) == nc) { l = a.boxLo[c]; h = a.boxHi[c]; cnt = a.counts[c]; }
+            ++nc;
         }
-    }
-    float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-    uint32_t nInner = 0, nLeafPrims = 0;
-    for (int i = 0; i < nc; ++i) {
-        const float4 l = a.boxLo[c[i]], h = a.boxHi[c[i]];
-        lo = make_float4(fminf(lo.x, l.x), fminf(lo.y, l.y), fminf(lo.z, l.z), 0.f);
-        hi = make_float4(fmaxf(hi.x, h.x), fmaxf(hi.y, h.y), fmaxf(hi.z, h.z), 0.f);
-        const uint32_t cnt = a.counts[c[i]];
-        if (cnt > kLeafMax) ++nInner; else nLeafPrims += cnt;
-    }
-    // slot auction: repeatedly give the free slot and unplaced child with the largest projection of
-    // the child's centre (relative to the node's) on the slot's octant diagonal to each other
-    int childAt[8];
-    for (int k = 0; k < 8; ++k) childAt[k] = -1;
-    {
-        float cost[8][8];
+        float4 lo = l, hi = h;
+        for (int off = 4; off > 0; off >>= 1) {
+            lo.x = fminf(lo.x, __shfl_xor_sync(group, lo.x, off));
+            lo.y = fminf(lo.y, __shfl_xor_sync(group, lo.y, off));
+            lo.z = fminf(lo.z, __shfl_xor_sync(group, lo.z, off));
+            hi.x = fmaxf(hi.x, __shfl_xor_sync(group, hi.x, off));
+            hi.y = fmaxf(hi.y, __shfl_xor_sync(group, hi.y, off));
+            hi.z = fmaxf(hi.z, __shfl_xor_sync(group, hi.z, off));
+        }
+        // slot auction: repeatedly give the free slot and unplaced child with the largest projection of
+        // the child's centre (relative to the node's) on the slot's octant diagonal to each other; of
+        // equals the first child, then the first slot
         const float px = 0.5f * (lo.x + hi.x), py = 0.5f * (lo.y + hi.y), pz = 0.5f * (lo.z + hi.z);
-        for (int i = 0; i < nc; ++i) {
-            const float4 l = a.boxLo[c[i]], h = a.boxHi[c[i]];
-            const float cx = 0.5f * (l.x + h.x) - px, cy = 0.5f * (l.y + h.y) - py, cz = 0.5f * (l.z + h.z) - pz;
-            for (int k = 0; k < 8; ++k)
-                cost[i][k] = ((k & 1) ? -cx : cx) + ((k & 2) ? -cy : cy) + ((k & 4) ? -cz : cz);
-        }
-        uint32_t placed = 0;
+        const float cx = 0.5f * (l.x + h.x) - px, cy = 0.5f * (l.y + h.y) - py, cz = 0.5f * (l.z + h.z) - pz;
+        int slot = -1;
+        uint32_t taken = 0;
         for (int round = 0; round < nc; ++round) {
-            int bi = -1, bk = -1;
+            int bk = -1;
             float bc = -INFINITY;
-            for (int i = 0; i < nc; ++i) {
-                if (placed & (1u << i)) continue;
-                for (int k = 0; k < 8; ++k)
-                    if (childAt[k] < 0 && (bi < 0 || cost[i][k] > bc)) { bc = cost[i][k]; bi = i; bk = k; }
+            if (c >= 0 && slot < 0) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float cost = ((k & 1) ? -cx : cx) + ((k & 2) ? -cy : cy) + ((k & 4) ? -cz : cz);
+                    if (!(taken >> k & 1u) && (bk < 0 || cost > bc)) { bc = cost; bk = k; }
+                }
+                if (!(bc > -INFINITY)) bc = -INFINITY;
             }
-            childAt[bk] = bi;
-            placed |= 1u << bi;
+            float best = bc;
+            for (int off = 4; off > 0; off >>= 1) best = fmaxf(best, __shfl_xor_sync(group, best, off));
+            const int src = __ffs(__ballot_sync(group, bk >= 0 && bc == best) & group) - 1;
+            const int k = __shfl_sync(group, bk, src);
+            if (int(threadIdx.x & 31u) == src) slot = k;
+            taken |= 1u << k;
         }
-    }
-    const uint32_t childBase = nInner ? atomicAdd(&a.counters[0], nInner) : 0u;
-    const uint32_t primBase = nLeafPrims ? atomicAdd(&a.counters[1], nLeafPrims) : 0u;
-    WideNode nd;
-    nd.ox = lo.x;
-    nd.oy = lo.y;
-    nd.oz = lo.z;
-    const uint32_t ex = scaleExponent(hi.x - lo.x), ey = scaleExponent(hi.y - lo.y), ez = scaleExponent(hi.z - lo.z);
-    nd.ex = uint8_t(ex);
-    nd.ey = uint8_t(ey);
-    nd.ez = uint8_t(ez);
-    const float sx = __uint_as_float(ex << 23), sy = __uint_as_float(ey << 23), sz = __uint_as_float(ez << 23);
-    nd.imask = 0;
-    nd.child_base = childBase;
-    nd.prim_base = primBase;
-    // inner children are stored in slot order, so that the k-th inner slot's node is child_base + k
-    uint32_t innerK = 0, leafOff = 0;
-    for (int i = 0; i < 8; ++i) {
-        if (childAt[i] < 0) {
-            nd.meta[i] = 0;
-            nd.qlox[i] = nd.qloy[i] = nd.qloz[i] = 255;
-            nd.qhix[i] = nd.qhiy[i] = nd.qhiz[i] = 0;
-            continue;
+        // the lanes without a child take the empty slots in order: a lane to a slot from here on
+        if (c < 0) {
+            uint32_t empty = ~taken & 0xFFu;
+            for (int k = nc; k < int(lane); ++k) empty &= empty - 1u;
+            slot = __ffs(empty) - 1;
         }
-        const int ci = c[childAt[i]];
-        const float4 l = a.boxLo[ci], h = a.boxHi[ci];
+        const bool inner = c >= 0 && cnt > kLeafMax;
+        const uint32_t leafCnt = c >= 0 && !inner ? cnt : 0u;
+        const uint32_t imask = __reduce_or_sync(group, inner ? 1u << slot : 0u);
+        const uint32_t leafCounts = __reduce_or_sync(group, leafCnt << (4 * slot));  // by slot
+        const uint32_t nInner = uint32_t(__popc(imask)), nLeafPrims = __reduce_add_sync(group, leafCnt);
+        // inner children are stored in slot order, so that the k-th inner slot's node is child_base + k
+        const uint32_t innerK = uint32_t(__popc(imask & ((1u << slot) - 1u)));
+        uint32_t leafOff = 0;
+        for (int k = 0; k < slot; ++k) leafOff += (leafCounts >> (4 * k)) & 15u;
+        uint32_t childBase = 0, primBase = 0, nextBase = 0;
+        if (lane == 0) {
+            if (nInner) {
+                childBase = atomicAdd(&a.counters[0], nInner);
+                nextBase = atomicAdd(&a.counters[2 + level + 1], nInner);
+            }
+            if (nLeafPrims) primBase = atomicAdd(&a.counters[1], nLeafPrims);
+        }
+        childBase = __shfl_sync(group, childBase, lead);
+        primBase = __shfl_sync(group, primBase, lead);
+        nextBase = __shfl_sync(group, nextBase, lead);
+        const uint32_t ex = scaleExponent(hi.x - lo.x), ey = scaleExponent(hi.y - lo.y), ez = scaleExponent(hi.z - lo.z);
+        const float sx = __uint_as_float(ex << 23), sy = __uint_as_float(ey << 23), sz = __uint_as_float(ez << 23);
         auto qlo = [](float v, float o, float s) {
             return uint8_t(fminf(fmaxf(floorf(__fsub_rd(v, o) / s), 0.f), 255.f));
         };
         auto qhi = [](float v, float o, float s) {
             return uint8_t(fminf(fmaxf(ceilf(__fsub_ru(v, o) / s), 0.f), 255.f));
         };
-        nd.qlox[i] = qlo(l.x, lo.x, sx);
-        nd.qloy[i] = qlo(l.y, lo.y, sy);
-        nd.qloz[i] = qlo(l.z, lo.z, sz);
-        nd.qhix[i] = qhi(h.x, lo.x, sx);
-        nd.qhiy[i] = qhi(h.y, lo.y, sy);
-        nd.qhiz[i] = qhi(h.z, lo.z, sz);
-        const uint32_t cnt = a.counts[ci];
-        if (cnt > kLeafMax) {
-            nd.imask |= uint8_t(1u << i);
-            nd.meta[i] = uint8_t(8u | innerK);
-            const uint32_t slot = atomicAdd(&a.counters[2], 1u);
-            a.next[slot] = make_uint2(uint32_t(ci), childBase + innerK);
-            ++innerK;
+        WideNode& nd = a.nodes[item.y];
+        if (lane == 0) {
+            nd.ox = lo.x;
+            nd.oy = lo.y;
+            nd.oz = lo.z;
+            nd.ex = uint8_t(ex);
+            nd.ey = uint8_t(ey);
+            nd.ez = uint8_t(ez);
+            nd.imask = uint8_t(imask);
+            nd.child_base = childBase;
+            nd.prim_base = primBase;
+        }
+        if (c < 0) {  // an empty slot's box is inverted: no ray passes it
+            nd.meta[slot] = 0;
+            nd.qlox[slot] = nd.qloy[slot] = nd.qloz[slot] = 255;
+            nd.qhix[slot] = nd.qhiy[slot] = nd.qhiz[slot] = 0;
         } else {
-            nd.meta[i] = uint8_t((cnt << 5) | leafOff);
-            const int first = ci >= n - 1 ? ci - (n - 1) : a.ranges[ci].x;
-            for (uint32_t k = 0; k < cnt; ++k) a.leafOrder[primBase + leafOff + k] = a.vals[first + k];
-            leafOff += cnt;
+            nd.qlox[slot] = qlo(l.x, lo.x, sx);
+            nd.qloy[slot] = qlo(l.y, lo.y, sy);
+            nd.qloz[slot] = qlo(l.z, lo.z, sz);
+            nd.qhix[slot] = qhi(h.x, lo.x, sx);
+            nd.qhiy[slot] = qhi(h.y, lo.y, sy);
+            nd.qhiz[slot] = qhi(h.z, lo.z, sz);
+            if (inner) {
+                nd.meta[slot] = uint8_t(8u | innerK);
+                next[nextBase + innerK] = make_uint2(uint32_t(c), childBase + innerK);
+            } else {
+                nd.meta[slot] = uint8_t((cnt << 5) | leafOff);
+                const int first = c >= n - 1 ? c - (n - 1) : a.ranges[c].x;
+                for (uint32_t k = 0; k < cnt; ++k) a.leafOrder[primBase + leafOff + k] = a.vals[first + k];
+            }
         }
     }
-    a.nodes[item.y] = nd;
+}
+
+// ------------------------------------------------------------------ deformed heightfields
+// One triangle of a heightfield whose vertices moved to z = baseZ + height: its FP64 and FP32 vertices
+// and its padded box, as the scene upload computes them on the host, operation by operation (no
+// contraction), so that a heightfield set on the device is the mesh uploaded with those heights.
+__device__ __forceinline__ double frameRow(const double* m, double x, double y, double z) {
+    return __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(m[0], x), __dmul_rn(m[1], y)), __dmul_rn(m[2], z)), m[3]);
+}
+// Bound by its 152 bytes written a triangle; the host's loop over them and four copies, with every
+// triangle of the scene uploaded again in FP64, were most of owec_set_heightfield's 9.80 ms (kCollapse).
+__global__ void __launch_bounds__(128) kDeformHeightfield(HeightfieldMesh m, const double* heights, float4* tri,
+                                                          double* tri64, float4* primLo, float4* primHi) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= m.nTriangles) return;
+    double w[3][3];
+    float f[3][3];
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t v = m.tris[3 * size_t(t) + k];
+        const double x = m.verts[3 * size_t(v)], y = m.verts[3 * size_t(v) + 1], z = __dadd_rn(m.baseZ, heights[v]);
+        for (int a = 0; a < 3; ++a) {
+            w[k][a] = frameRow(m.toWorld.m + 4 * a, x, y, z);
+            f[k][a] = float(w[k][a]);
+        }
+    }
+    const size_t p = size_t(m.firstPrim) + t;
+    const uint32_t ids[3] = {m.boundary, t, kPrimTriangle};
+    double lo[3], hi[3], ext = 0, mag = 0;
+    for (int k = 0; k < 3; ++k) {
+        tri[3 * p + k] = make_float4(f[k][0], f[k][1], f[k][2], __uint_as_float(ids[k]));
+        for (int a = 0; a < 3; ++a) tri64[9 * p + 3 * k + a] = w[k][a];
+    }
+    for (int a = 0; a < 3; ++a) {
+        const double v[6] = {f[0][a], f[1][a], f[2][a], w[0][a], w[1][a], w[2][a]};
+        lo[a] = hi[a] = v[0];
+        for (int k = 1; k < 6; ++k) {
+            if (v[k] < lo[a]) lo[a] = v[k];
+            if (hi[a] < v[k]) hi[a] = v[k];
+        }
+        const double e = __dadd_rn(hi[a], -lo[a]);
+        if (ext < e) ext = e;
+        if (mag < fabs(lo[a])) mag = fabs(lo[a]);
+        if (mag < fabs(hi[a])) mag = fabs(hi[a]);
+    }
+    const double pad = __dadd_rn(__dmul_rn(1e-6, __dadd_rn(mag, ext)), 1e-9);
+    float bl[3], bh[3];
+    for (int a = 0; a < 3; ++a) {
+        bl[a] = nextafterf(float(__dadd_rn(lo[a], -pad)), -INFINITY);
+        bh[a] = nextafterf(float(__dadd_rn(hi[a], pad)), INFINITY);
+    }
+    primLo[p] = make_float4(bl[0], bl[1], bl[2], 0.f);
+    primHi[p] = make_float4(bh[0], bh[1], bh[2], 0.f);
 }
 
 }  // namespace
+
+void launchDeformHeightfield(const HeightfieldMesh& m, const double* heights, float4* tri, double* tri64, float4* primLo,
+                             float4* primHi, cudaStream_t s) {
+    if (m.nTriangles == 0) return;
+    kDeformHeightfield<<<(m.nTriangles + 127) / 128, 128, 0, s>>>(m, heights, tri, tri64, primLo, primHi);
+}
 
 uint32_t buildWideBvh(const float4* primLo, const float4* primHi, uint32_t n, BvhScratch& s, DBuf<WideNode>& nodes,
                       DBuf<uint32_t>& leafOrder, cudaStream_t stream) {
@@ -345,14 +448,12 @@ uint32_t buildWideBvh(const float4* primLo, const float4* primHi, uint32_t n, Bv
     s.flags.reserve(n);
     s.work.reserve(n);
     s.next.reserve(n);
-    s.counters.reserve(8);
+    s.counters.reserve(kCounters);
     s.bounds.reserve(8);
     nodes.reserve(std::max<uint32_t>(1, n));
     leafOrder.reserve(n);
 
-    // +inf and -inf in the ordered integer image
-    const int init[6] = {0x7F800000, 0x7F800000, 0x7F800000, int(0x807FFFFFu), int(0x807FFFFFu), int(0x807FFFFFu)};
-    OWEC_CUDA(cudaMemcpyAsync(s.bounds.get(), init, sizeof(init), cudaMemcpyHostToDevice, stream));
+    kBeginBuild<<<1, 256, 0, stream>>>(s.bounds.get(), s.counters.get(), s.work.get());
     const int T = 256;
     kCentroidBounds<<<std::min<uint32_t>((n + T - 1) / T, 1184), T, 0, stream>>>(primLo, primHi, n, s.bounds.get());
     kMorton<<<(n + T - 1) / T, T, 0, stream>>>(primLo, primHi, n, s.bounds.get(), s.keys.get(), s.vals.get());
@@ -373,34 +474,33 @@ uint32_t buildWideBvh(const float4* primLo, const float4* primHi, uint32_t n, Bv
     kBottomUp<<<(n + T - 1) / T, T, 0, stream>>>(primLo, primHi, vals, int(n), s.children.get(), s.parents.get(),
                                                   s.boxLo.get(), s.boxHi.get(), s.counts.get(), s.flags.get());
 
-    {
-        uint32_t err = 0;  // flags[n - 1] is no inner node's: it collects malformed-tree reports
+    CollapseArgs a{s.children.get(), s.ranges.get(), s.boxLo.get(), s.boxHi.get(), s.counts.get(), vals,
+                   s.flags.get() + (n - 1),  // no inner node's: it collects malformed-tree reports
+                   int(n), nodes.get(), leafOrder.get(), s.counters.get()};
+    uint2 *work = s.work.get(), *next = s.next.get();
+    // Levels are queued a batch at a time, a tree of full nodes' depth and a few more first, and the host
+    // looks at the counters once per batch: a level past the last one finds no work.
+    int batch = 4;
+    for (uint64_t full = 1; full < n; full *= 8) ++batch;
+    uint64_t width = 1;  // nodes the level can hold
+    for (int level = 0;;) {
+        for (int k = 0; k < batch; ++k, ++level) {
+            const uint64_t items = std::min<uint64_t>(width, n);
+            kCollapse<<<int(std::min<uint64_t>((items * 8 + 127) / 128, 2368)), 128, 0, stream>>>(a, level, work, next);
+            std::swap(work, next);
+            width = std::min<uint64_t>(width * 8, n);
+        }
+        std::vector<uint32_t> h(3 + level);
+        uint32_t err = 0;
+        OWEC_CUDA(cudaMemcpyAsync(h.data(), s.counters.get(), h.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
         OWEC_CUDA(cudaMemcpyAsync(&err, s.flags.get() + (n - 1), sizeof(err), cudaMemcpyDeviceToHost, stream));
         OWEC_CUDA(cudaStreamSynchronize(stream));
         if (err >= 0x10000u) throw std::runtime_error("BVH build: malformed radix tree");
-    }
-    const uint32_t counters[4] = {1u, 0u, 0u, 0u};  // the root is wide node 0
-    OWEC_CUDA(cudaMemcpyAsync(s.counters.get(), counters, sizeof(counters), cudaMemcpyHostToDevice, stream));
-    // the binary root: inner node 0, or with one primitive its leaf (combined index n - 1 = 0)
-    const uint2 root = make_uint2(0u, 0u);
-    OWEC_CUDA(cudaMemcpyAsync(s.work.get(), &root, sizeof(root), cudaMemcpyHostToDevice, stream));
-    CollapseArgs a{s.children.get(), s.ranges.get(), s.boxLo.get(), s.boxHi.get(), s.counts.get(), vals, int(n),
-                   nodes.get(), leafOrder.get(), s.counters.get(), s.work.get(), s.next.get()};
-    uint32_t nWork = 1;
-    for (int level = 0; nWork > 0; ++level) {
-        if (level > 4096) throw std::runtime_error("BVH collapse did not terminate");
-        kCollapse<<<(nWork + 127) / 128, 128, 0, stream>>>(a, nWork);
-        uint32_t h[4];
-        OWEC_CUDA(cudaMemcpyAsync(h, s.counters.get(), sizeof(h), cudaMemcpyDeviceToHost, stream));
-        OWEC_CUDA(cudaStreamSynchronize(stream));
-        nWork = h[2];
-        const uint32_t zero = 0;
-        OWEC_CUDA(cudaMemcpyAsync(s.counters.get() + 2, &zero, sizeof(zero), cudaMemcpyHostToDevice, stream));
-        std::swap(a.work, a.next);
         s.nodeCount = h[0];
         s.placedPrims = h[1];
+        if (h[2 + level] == 0) break;
+        if (level + batch > int(kMaxLevels)) throw std::runtime_error("BVH collapse did not terminate");
     }
-    OWEC_CUDA(cudaStreamSynchronize(stream));
     if (s.placedPrims != n) throw std::runtime_error("BVH collapse placed " + std::to_string(s.placedPrims) +
                                                      " of " + std::to_string(n) + " primitives");
     return s.nodeCount;

@@ -26,4 +26,18 @@ struct BvhScratch {
 uint32_t buildWideBvh(const float4* primLo, const float4* primHi, uint32_t n, BvhScratch& s, DBuf<WideNode>& nodes,
                       DBuf<uint32_t>& leafOrder, cudaStream_t stream);
 
+// A mesh boundary whose vertices' heights are set: its rest vertices and triangles in its own frame
+// (device memory), that frame, and where its primitives lie.
+struct HeightfieldMesh {
+    const double* verts;
+    const uint32_t* tris;
+    uint32_t nTriangles, boundary, firstPrim;
+    double baseZ;
+    Xform toWorld;
+};
+// Moves the mesh's vertices to z = baseZ + heights[vertex]: rewrites its triangles' FP32 and FP64
+// vertices and boxes (indexed by primitive).
+void launchDeformHeightfield(const HeightfieldMesh& m, const double* heights, float4* tri, double* tri64, float4* primLo,
+                             float4* primHi, cudaStream_t s);
+
 }  // namespace owec

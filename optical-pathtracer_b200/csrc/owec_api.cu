@@ -414,7 +414,7 @@ struct owec_ctx {
     DBuf<PrimRec> dPrims;
     DBuf<PrimRec64> dPrims64;
     uint32_t nNodes = 0;
-    bool prims64Ready = false;
+    bool prims64Ready = false, tri64Ready = false;
 
     // rendering
     owec_settings settings{1, 64, 6, OWEC_WAVELENGTHS_HERO4, OWEC_PRECISION_MIXED, 380, 780, 0, OWEC_INTEGRATOR_PATH, 0};
@@ -452,6 +452,7 @@ struct owec_ctx {
     uint64_t hfVertices = 0;
     double lastPathAdjointSeconds = 0;
     DBuf<uint32_t> dHfTris;
+    DBuf<double> dHfVerts, dHfHeights;
     struct MeshCopy {
         std::vector<double> verts;    // shape-frame vertices as uploaded
         std::vector<uint32_t> tris;
@@ -1038,6 +1039,7 @@ void uploadScene(owec_ctx& c, const owec_scene_desc& d) {
     c.hasScene = true;
     c.bvhDirty = true;
     c.prims64Ready = false;
+    c.tri64Ready = false;
     // a new scene has no heightfield until owec_set_heightfield names one of its boundaries
     c.hf.boundary = kNone;
     c.hfVertices = 0;
@@ -1049,7 +1051,28 @@ void uploadScene(owec_ctx& c, const owec_scene_desc& d) {
     c.particles = 0;
 }
 
-void ensurePrims64(owec_ctx& c);
+// The FP64 vertices on the device, uploaded once per scene (a heightfield's are rewritten there).
+void ensureTri64(owec_ctx& c) {
+    if (c.tri64Ready) return;
+    c.dTri64.upload(c.tri64.data(), c.tri64.size(), c.stream);
+    c.tri64Ready = true;
+}
+
+// The primitive records in leaf order, with the FP64 ones the mixed and FP64 modes read.
+void materializePrims(owec_ctx& c, bool with64) {
+    c.dPrims.reserve(c.nPrims);
+    if (with64) {
+        ensureTri64(c);
+        c.dPrims64.reserve(c.nPrims);
+    }
+    launchMaterialize(c.dLeafOrder.get(), c.nPrims, c.dTri.get(), with64 ? c.dTri64.get() : nullptr, c.dPrims.get(),
+                      with64 ? c.dPrims64.get() : nullptr, c.stream);
+    checkLaunch();
+    OWEC_CUDA(cudaStreamSynchronize(c.stream));
+    c.ds.prims = c.dPrims.get();
+    if (with64) c.ds.prims64 = c.dPrims64.get();
+    c.prims64Ready = with64;
+}
 
 void buildBvh(owec_ctx& c) {
     require(c.hasScene, "no scene uploaded", OWEC_E_STATE);
@@ -1067,29 +1090,16 @@ void buildBvh(owec_ctx& c) {
         return;
     }
     c.nNodes = buildWideBvh(c.dPrimLo.get(), c.dPrimHi.get(), c.nPrims, c.scratch, c.dNodes, c.dLeafOrder, c.stream);
-    c.dPrims.reserve(c.nPrims);
-    launchMaterialize(c.dLeafOrder.get(), c.nPrims, c.dTri.get(), nullptr, c.dPrims.get(), nullptr, c.stream);
-    checkLaunch();
-    OWEC_CUDA(cudaStreamSynchronize(c.stream));
     c.ds.nodes = c.dNodes.get();
-    c.ds.prims = c.dPrims.get();
     c.ds.nNodes = c.nNodes;
     c.ds.nPrims = c.nPrims;
+    materializePrims(c, c.settings.precision != OWEC_PRECISION_FP32);
     c.bvhDirty = false;
-    c.prims64Ready = false;
-    if (c.settings.precision != OWEC_PRECISION_FP32) ensurePrims64(c);
 }
 
 void ensurePrims64(owec_ctx& c) {
     if (c.prims64Ready || c.nPrims == 0) return;
-    c.dTri64.upload(c.tri64.data(), c.tri64.size(), c.stream);
-    c.dPrims64.reserve(c.nPrims);
-    launchMaterialize(c.dLeafOrder.get(), c.nPrims, c.dTri.get(), c.dTri64.get(), c.dPrims.get(), c.dPrims64.get(),
-                      c.stream);
-    checkLaunch();
-    OWEC_CUDA(cudaStreamSynchronize(c.stream));
-    c.ds.prims64 = c.dPrims64.get();
-    c.prims64Ready = true;
+    materializePrims(c, true);
 }
 
 // Copies the scene description to its device copy, which the out-of-line traversal functions read
@@ -1981,37 +1991,18 @@ int owec_set_heightfield(owec_ctx* ctx, uint32_t boundary, uint64_t n_vertices, 
         require(n_vertices == m.verts.size() / 3, "one height per vertex of the mesh");
         OWEC_CUDA(cudaSetDevice(ctx->device));
         const DBoundary& bd = ctx->boundaries[boundary];
-        auto asF = [](uint32_t v) { float f; std::memcpy(&f, &v, 4); return f; };
-        const uint32_t base = ctx->triBase[boundary];
-        const size_t nt = m.tris.size() / 3;
-        for (size_t t = 0; t < nt; ++t) {
-            double w[3][3];
-            for (int k = 0; k < 3; ++k) {
-                const uint32_t v = m.tris[3 * t + k];
-                const double local[3] = {m.verts[3 * v], m.verts[3 * v + 1], base_z + heights[v]};
-                xfPoint(bd.toWorld.m, local, w[k]);
-            }
-            const size_t p = base + t;
-            const uint32_t ids[3] = {boundary, uint32_t(t), kPrimTriangle};
-            double lo[3], hi[3];
-            for (int k = 0; k < 3; ++k) {
-                ctx->triRecs[3 * p + k] = make_float4(float(w[k][0]), float(w[k][1]), float(w[k][2]), asF(ids[k]));
-                for (int a = 0; a < 3; ++a) ctx->tri64[9 * p + 3 * k + a] = w[k][a];
-            }
-            for (int a = 0; a < 3; ++a) {
-                const float f0 = float(w[0][a]), f1 = float(w[1][a]), f2 = float(w[2][a]);
-                lo[a] = std::min({double(f0), double(f1), double(f2), w[0][a], w[1][a], w[2][a]});
-                hi[a] = std::max({double(f0), double(f1), double(f2), w[0][a], w[1][a], w[2][a]});
-            }
-            padPrimBox(lo, hi, ctx->primLo[p], ctx->primHi[p]);
+        if (ctx->hf.boundary != boundary) {  // the first heights of this boundary: its rest mesh
+            ctx->hf.boundary = kNone;
+            ctx->dHfTris.upload(m.tris.data(), m.tris.size(), ctx->stream);
+            ctx->dHfVerts.upload(m.verts.data(), m.verts.size(), ctx->stream);
         }
-        OWEC_CUDA(cudaMemcpyAsync(ctx->dTri.get() + 3 * size_t(base), ctx->triRecs.data() + 3 * size_t(base),
-                                  3 * nt * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
-        OWEC_CUDA(cudaMemcpyAsync(ctx->dPrimLo.get() + base, ctx->primLo.data() + base, nt * sizeof(float4),
-                                  cudaMemcpyHostToDevice, ctx->stream));
-        OWEC_CUDA(cudaMemcpyAsync(ctx->dPrimHi.get() + base, ctx->primHi.data() + base, nt * sizeof(float4),
-                                  cudaMemcpyHostToDevice, ctx->stream));
-        ctx->dHfTris.upload(m.tris.data(), m.tris.size(), ctx->stream);
+        ensureTri64(*ctx);
+        ctx->dHfHeights.upload(heights, n_vertices, ctx->stream);
+        HeightfieldMesh hm{ctx->dHfVerts.get(), ctx->dHfTris.get(), uint32_t(m.tris.size() / 3), boundary,
+                           ctx->triBase[boundary], base_z, bd.toWorld};
+        launchDeformHeightfield(hm, ctx->dHfHeights.get(), ctx->dTri.get(), ctx->dTri64.get(), ctx->dPrimLo.get(),
+                                ctx->dPrimHi.get(), ctx->stream);
+        checkLaunch();
         buildBvh(*ctx);
         ctx->hf.boundary = boundary;
         ctx->hf.tris = ctx->dHfTris.get();
