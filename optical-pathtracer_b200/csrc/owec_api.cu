@@ -1449,7 +1449,7 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
 // library holds these 10.5 MB until the process exits; every call of that entry point shares them.
 constexpr size_t kNoAllocMaxBins = 512 * 512;      // walk film bins (width x height)
 constexpr size_t kNoAllocMaxHeights = 1u << 20;    // heightfield vertices
-constexpr size_t kNoAllocStatsWords = 8;           // walk counters (5 used)
+constexpr size_t kNoAllocStatsWords = 8;           // walk counters (kWalkStatWords used)
 static __device__ __align__(256) double gAdjointScratch[kNoAllocMaxBins + kNoAllocMaxHeights + kNoAllocStatsWords];
 
 namespace {
@@ -1934,7 +1934,7 @@ int owec_walk(owec_ctx* ctx, const owec_walk_desc* w, uint64_t first, uint64_t n
             ctx->hasWalk = true;
             ctx->walks = 0;
             ctx->dWalkBins.resize(size_t(w->width) * w->height);
-            ctx->dWalkStats.resize(5);
+            ctx->dWalkStats.resize(kWalkStatWords);
             OWEC_CUDA(cudaMemsetAsync(ctx->dWalkBins.get(), 0, ctx->dWalkBins.bytes(), ctx->stream));
             OWEC_CUDA(cudaMemsetAsync(ctx->dWalkStats.get(), 0, ctx->dWalkStats.bytes(), ctx->stream));
         }
@@ -2025,10 +2025,10 @@ int owec_walk_adjoint(owec_ctx* ctx, const owec_walk_desc* w, uint64_t first, ui
         ensureReady(*ctx);
         const size_t nb = size_t(w->width) * w->height, nh = ctx->hfVertices;
         DBuf<double> dG(nb), dDH(nh);
-        DBuf<unsigned long long> st(5);
+        DBuf<unsigned long long> st(kWalkStatWords);
         OWEC_CUDA(cudaMemcpyAsync(dG.get(), g, nb * 8, cudaMemcpyHostToDevice, ctx->stream));
         OWEC_CUDA(cudaMemsetAsync(dDH.get(), 0, nh * 8, ctx->stream));
-        OWEC_CUDA(cudaMemsetAsync(st.get(), 0, 5 * 8, ctx->stream));
+        OWEC_CUDA(cudaMemsetAsync(st.get(), 0, st.bytes(), ctx->stream));
         double measure;
         if (w->source_kind == OWEC_SOURCE_POINT) measure = 2 * kPi * (1 - std::cos(w->extent));
         else if (w->source_kind == OWEC_SOURCE_COLLIMATED) measure = kPi * w->extent * w->extent;

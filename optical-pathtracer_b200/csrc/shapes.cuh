@@ -71,11 +71,11 @@ OWEC_HD void quadricCoeffs(int kind, T qa, T qb, T qc, const V3<T>& o, const V3<
 
 // The root t (from precision R) refined in precision Rr, if it may lie in (tmin, tmax) and does
 // once refined (refineRoot / mayLieIn / refinedRootIn, surfaces.hpp:75-101).
-template <class R, class Rr>
-OWEC_HD bool refinedRootIn(int kind, Rr qa, Rr qb, const V3<Rr>& o, const V3<Rr>& d, Rr t, Rr tmin, Rr tmax, Rr& tr,
-                           Rr qc = Rr(0)) {
+template <class Rr>
+OWEC_HD bool refinedRootIn(int kind, Rr qa, Rr qb, const V3<Rr>& o, const V3<Rr>& d, Rr t, Rr tmin, Rr tmax, Rr& tr, Rr qc,
+                           Rr refine) {
     tr = t;
-    const Rr m = Rr(Tol<R>::refine) * (Rr(1) + fabs(t));
+    const Rr m = refine * (Rr(1) + fabs(t));
     if (t + m <= tmin || t - m >= tmax) return false;
     Rr A, B, C, u0, u1;
     quadricCoeffs(kind, qa, qb, qc, o + d * t, d, A, B, C);
@@ -84,6 +84,12 @@ OWEC_HD bool refinedRootIn(int kind, Rr qa, Rr qb, const V3<Rr>& o, const V3<Rr>
         if (fabs(du) < m) tr = t + du;
     }
     return tr > tmin && tr < tmax;
+}
+
+template <class R, class Rr>
+OWEC_HD bool refinedRootIn(int kind, Rr qa, Rr qb, const V3<Rr>& o, const V3<Rr>& d, Rr t, Rr tmin, Rr tmax, Rr& tr,
+                           Rr qc = Rr(0)) {
+    return refinedRootIn(kind, qa, qb, o, d, t, tmin, tmax, tr, qc, Rr(Tol<R>::refine));
 }
 
 // A crossing of an analytic surface in its frame.
@@ -160,7 +166,7 @@ OWEC_HD bool nearSphere(const DBoundary& b, const V3<double>& od) {
 // The sphere's crossings in (tmin, tmax) for such a ray, in the world frame (a sphere's roots do not
 // depend on its frame's rotation): od - c exact as a double-double, the quadratic's coefficients in
 // double-double, the roots in the numerically stable form. Points and normals in the sphere's local
-// frame, as classicCrossings gives them (the normal from the exact od - c; the point converted from
+// frame, as classicPoint and classicNormal give them (the normal from the exact od - c; the point converted from
 // the world point od + t d). Out of line, its result by value: the callers' own hits stay in registers.
 OWEC_HD_COLD AHits<double> nearSphereCrossings(const DBoundary& b, V3<double> od, V3<double> d, double tmin,
                                                double tmax) {
@@ -328,72 +334,76 @@ OWEC_HD bool domeSolid(T R, T azimuth, T width, T top, const V3<T>& p) {
     return fabs(sin(dAz)) * R * cos(el) >= width / T(2) || cos(dAz) < T(0);
 }
 
-// The crossings of the shapes every scene had before the trimmed, lathe and aspheric ones: spheres,
-// conic sags, disk, rectangle and ellipse apertures and cylinders (the lean traversal's
-// analyticCrossings; see there).
-template <class R, class Rr>
-OWEC_HD int classicCrossings(const DBoundary& b, const V3<Rr>& o, const V3<Rr>& d, Rr tmin, Rr tmax, AHits<Rr>& out) {
-    out.n = 0;
+// Spheres, conic sags, plain apertures and cylinders (the lean instantiations' shapes): the distances of
+// up to two crossings in (tmin, tmax), ascending, each inside the shape's trim. The roots come in
+// precision R (a sphere's in the refinement's: a ray leaving a large sphere, a moon, a planet, a dome,
+// has |o| near R, where FP32 loses c = |o|^2 - R^2 entirely, and a root the refinement cannot pull back
+// within its window would survive as a false crossing) and are refined in Rr by one loop for all the
+// quadrics. Points and normals are left to classicPoint and classicNormal, which the caller asks for the
+// one crossing it takes: both crossings' normals in full, every shape with its own unrolled pair, were
+// half of a lens walk's FP64 work. Rolled: the loop stays a loop, for the one-lane-per-walk kernels,
+// whose code overflows the instruction cache (277 KB of it, and 8 of a warp's 13.6 cycles per instruction
+// spent waiting for the next one); the traversal kernels, which fit, are 8 % faster on spheres unrolled.
+template <class R, class Rr, bool Rolled>
+OWEC_HD int classicRoots(const DBoundary& b, const V3<Rr>& o, const V3<Rr>& d, Rr tmin, Rr tmax, Rr& first, Rr& second) {
     const double* P = b.params;
+    int kind = -1;  // -1: a plane, one root and no refinement
+    Rr qa = Rr(0), qb = Rr(0), s0 = Rr(0), s1 = Rr(0), refine = Rr(Tol<R>::refine);
+    bool both = true;
     switch (b.shape) {
         case OWEC_SHAPE_SPHERE: {
-            // Sphere roots in the refinement's precision: a ray leaving a large sphere (a moon, a
-            // planet, a dome) has |o| near R, where FP32 loses c = |o|^2 - R^2 entirely, and a root
-            // the refinement cannot pull back within its window would survive as a false crossing.
             const Rr Rad = Rr(P[0]);
-            Rr t0, t1;
-            if (!sphereRoots(o, d, Rad, t0, t1)) return 0;
-            const Rr ts[2] = {t0, t1};
-            for (int i = 0; i < 2; ++i) {
-                Rr tr;
-                if (!refinedRootIn<Rr, Rr>(kQuadSphere, Rad * Rad, Rr(0), o, d, ts[i], tmin, tmax, tr)) continue;
-                const V3<Rr> p = o + d * tr;
-                out.add({tr, p, normalize(p / Rad)});
-            }
+            if (!sphereRoots(o, d, Rad, s0, s1)) return 0;
+            kind = kQuadSphere;
+            qa = Rad * Rad;
+            refine = Rr(Tol<Rr>::refine);
             break;
         }
         case OWEC_SHAPE_SAG: {
-            const Rr c = Rr(P[0]), k = Rr(P[1]), rMax = Rr(P[2]), rMin = Rr(P[3]);
-            auto solid = [&](const V3<Rr>& p) {
-                const Rr r2 = p.x * p.x + p.y * p.y;
-                return r2 <= rMax * rMax && r2 >= rMin * rMin &&
-                       (c == Rr(0) || (Rr(1) + k) * c * p.z <= Rr(1) + Rr(Tol<R>::relTol));
-            };
-            auto normal = [&](const V3<Rr>& p) {
-                const Rr r = sqrt(p.x * p.x + p.y * p.y);
-                if (r < Tol<Rr>::tiny) return V3<Rr>(0, 0, 1);
-                const Rr s = conicSlope(c, k, r);
-                return normalize(V3<Rr>(-s * p.x / r, -s * p.y / r, Rr(1)));
-            };
-            if (c == Rr(0)) {
-                if (d.z == Rr(0)) return 0;
-                const Rr t = -o.z / d.z;
-                if (t <= tmin || t >= tmax) return 0;
-                const V3<Rr> p = o + d * t;
-                if (!solid(p)) return 0;
-                out.add({t, p, normal(p)});
+            const Rr c = Rr(P[0]), k = Rr(P[1]);
+            if (c != Rr(0)) {
+                R A, B, C, t0, t1;
+                quadricCoeffs(kQuadSag, R(c), R(c * (Rr(1) + k)), R(0), V3<R>(o), V3<R>(d), A, B, C);
+                if (solveQuadratic(A, B, C, t0, t1) <= 0) return 0;
+                kind = kQuadSag;
+                qa = c;
+                qb = c * (Rr(1) + k);
+                s0 = Rr(t0);
+                s1 = Rr(t1);
+                both = t1 != t0;  // a sag's double root counts once
                 break;
             }
-            R A, B, C, t0, t1;
-            quadricCoeffs(kQuadSag, R(c), R(c * (Rr(1) + k)), R(0), V3<R>(o), V3<R>(d), A, B, C);
-            if (solveQuadratic(A, B, C, t0, t1) <= 0) return 0;
-            const R ts[2] = {t0, t1};
-            for (int i = 0; i < 2; ++i) {
-                if (i == 1 && t1 == t0) break;
-                Rr tr;
-                if (!refinedRootIn<R, Rr>(kQuadSag, c, c * (Rr(1) + k), o, d, Rr(ts[i]), tmin, tmax, tr)) continue;
-                const V3<Rr> p = o + d * tr;
-                if (!solid(p)) continue;
-                out.add({tr, p, normal(p)});
-            }
+        }
+        // a flat sag is a plane
+        case OWEC_SHAPE_PLANE:
+            if (d.z == Rr(0)) return 0;
+            s0 = -o.z / d.z;
+            both = false;
+            break;
+        case OWEC_SHAPE_CYLINDER: {
+            R t0, t1;
+            if (!cylinderRoots(V3<R>(o), V3<R>(d), R(P[0]), t0, t1)) return 0;
+            kind = kQuadCylinder;
+            qa = Rr(P[0]) * Rr(P[0]);
+            s0 = Rr(t0);
+            s1 = Rr(t1);
             break;
         }
-        case OWEC_SHAPE_PLANE: {
-            if (d.z == Rr(0)) return 0;
-            const Rr t = -o.z / d.z;
-            if (t <= tmin || t >= tmax) return 0;
-            V3<Rr> p = o + d * t;
-            p.z = Rr(0);
+        default: return 0;
+    }
+    int n = 0;
+#pragma unroll(Rolled ? 1 : 2)
+    for (int i = 0; i < 2; ++i) {
+        if (i == 1 && !both) break;
+        const Rr t = i == 0 ? s0 : s1;
+        Rr tr = t;
+        if (kind < 0) {
+            if (t <= tmin || t >= tmax) continue;
+        } else if (!refinedRootIn(kind, qa, qb, o, d, t, tmin, tmax, tr, Rr(0), refine)) {
+            continue;
+        }
+        const V3<Rr> p = o + d * tr;
+        if (b.shape == OWEC_SHAPE_PLANE) {
             const int ap = int(P[0]);
             const Rr a = Rr(P[1]), bb = Rr(P[2]);
             bool in;
@@ -405,33 +415,46 @@ OWEC_HD int classicCrossings(const DBoundary& b, const V3<Rr>& o, const V3<Rr>& 
             } else {
                 in = sqr(p.x / a) + sqr(p.y / bb) <= Rr(1);
             }
-            if (!in) return 0;
-            out.add({t, p, V3<Rr>(0, 0, 1)});
-            break;
+            if (!in) continue;
+        } else if (b.shape == OWEC_SHAPE_SAG) {
+            const Rr c = Rr(P[0]), k = Rr(P[1]), rMax = Rr(P[2]), rMin = Rr(P[3]);
+            const Rr r2 = p.x * p.x + p.y * p.y;
+            if (!(r2 <= rMax * rMax && r2 >= rMin * rMin && (c == Rr(0) || (Rr(1) + k) * c * p.z <= Rr(1) + Rr(Tol<R>::relTol))))
+                continue;
+        } else if (b.shape == OWEC_SHAPE_CYLINDER) {
+            if (p.z < Rr(P[1]) || p.z > Rr(P[2])) continue;
         }
-        case OWEC_SHAPE_CYLINDER: {
-            const Rr Rad = Rr(P[0]), z0 = Rr(P[1]), z1 = Rr(P[2]);
-            R t0, t1;
-            if (!cylinderRoots(V3<R>(o), V3<R>(d), R(P[0]), t0, t1)) return 0;
-            const R ts[2] = {t0, t1};
-            for (int i = 0; i < 2; ++i) {
-                Rr tr;
-                if (!refinedRootIn<R, Rr>(kQuadCylinder, Rad * Rad, Rr(0), o, d, Rr(ts[i]), tmin, tmax, tr)) continue;
-                const V3<Rr> p = o + d * tr;
-                if (p.z < z0 || p.z > z1) continue;
-                out.add({tr, p, normalize(V3<Rr>(p.x, p.y, Rr(0)))});
-            }
-            break;
-        }
-        default: break;
+        if (n == 0) first = tr;
+        else second = tr;
+        ++n;
     }
-    if (out.n == 2 && out.h1.t < out.h0.t) { const AHit<Rr> tmp = out.h0; out.h0 = out.h1; out.h1 = tmp; }
-    return out.n;
+    if (n == 2 && second < first) { const Rr tmp = first; first = second; second = tmp; }
+    return n;
+}
+// The point at distance t of a local ray on a classicRoots shape, and the shape's unit normal there.
+template <class Rr>
+OWEC_HD V3<Rr> classicPoint(const DBoundary& b, const V3<Rr>& o, const V3<Rr>& d, Rr t) {
+    V3<Rr> p = o + d * t;
+    if (b.shape == OWEC_SHAPE_PLANE) p.z = Rr(0);
+    return p;
+}
+template <class Rr>
+OWEC_HD V3<Rr> classicNormal(const DBoundary& b, const V3<Rr>& p) {
+    const double* P = b.params;
+    if (b.shape == OWEC_SHAPE_SPHERE) return normalize(p / Rr(P[0]));
+    if (b.shape == OWEC_SHAPE_CYLINDER) return normalize(V3<Rr>(p.x, p.y, Rr(0)));
+    if (b.shape == OWEC_SHAPE_SAG) {
+        const Rr r = sqrt(p.x * p.x + p.y * p.y);
+        if (r < Tol<Rr>::tiny) return V3<Rr>(0, 0, 1);
+        const Rr s = conicSlope(Rr(P[0]), Rr(P[1]), r);
+        return normalize(V3<Rr>(-s * p.x / r, -s * p.y / r, Rr(1)));
+    }
+    return V3<Rr>(0, 0, 1);
 }
 
 // Up to two crossings found numerically, ascending. The root finders below are out of line and
 // return by value: they need many registers and run only for the rare aspheres and torus patches,
-// so they must not raise the register count of the traversal that inlines analyticCrossings.
+// so they must not raise the register count of the traversal that inlines fullCrossings.
 template <class Rr>
 struct NumericRoots {
     Rr t[2];
@@ -700,14 +723,20 @@ OWEC_HD void quadricHits(int kind, Rr qa, Rr qb, Rr qc, const V3<Rr>& o, const V
     }
 }
 
-// The crossings of every shape (analyticCrossings with Full).
+// Up to two crossings of boundary b's shape, any shape, by the local ray (o, d) in (tmin, tmax),
+// ascending, each inside the shape's trim; returns how many. data: the shape's run of the scene's shape
+// data. departed: the ray leaves this boundary (a torus patch then resolves the start of its bracket
+// finely; a wave surface skips the crossings within depWindow of the origin along their normal).
+// nearWindow: the origin's error along a surface normal (a wave surface looks for a second crossing only
+// behind a first one within it). The kernels of a scene without the shapes beyond classicRoots' keep the
+// registers they need for those alone.
 template <class R, class Rr>
 OWEC_HD int fullCrossings(const DBoundary& b, const double* data, const V3<Rr>& o, const V3<Rr>& d, Rr tmin, Rr tmax,
-                          bool departed, AHits<Rr>& out, Rr depWindow, Rr nearWindow) {
+                          bool departed, AHits<Rr>& out, Rr depWindow = Rr(0), Rr nearWindow = Rr(0)) {
     out.n = 0;
     const double* P = b.params;
     switch (b.shape) {
-        case OWEC_SHAPE_SPHERE: {  // roots in the refinement's precision, as classicCrossings
+        case OWEC_SHAPE_SPHERE: {  // roots in the refinement's precision, as classicRoots
             const Rr Rad = Rr(P[0]);
             Rr t0, t1;
             if (!sphereRoots(o, d, Rad, t0, t1)) return 0;
@@ -830,21 +859,6 @@ OWEC_HD int fullCrossings(const DBoundary& b, const double* data, const V3<Rr>& 
     }
     if (out.n == 2 && out.h1.t < out.h0.t) { const AHit<Rr> tmp = out.h0; out.h0 = out.h1; out.h1 = tmp; }
     return out.n;
-}
-
-// Up to two crossings of boundary b's shape by the local ray (o, d) in (tmin, tmax), ascending,
-// each inside the shape's trim. data: the shape's run of the scene's shape data. departed: the ray
-// leaves this boundary (a torus patch then resolves the start of its bracket finely; a wave surface
-// skips the crossings within depWindow of the origin along their normal). nearWindow: the origin's
-// error along a surface normal (a wave surface looks for a second crossing only behind a first one
-// within it). Returns how many. Full = false compiles only the spheres, conic sags, plain apertures
-// and cylinders: the kernels of a scene without the other shapes keep the registers they need for
-// those alone.
-template <class R, class Rr, bool Full>
-OWEC_HD int analyticCrossings(const DBoundary& b, const double* data, const V3<Rr>& o, const V3<Rr>& d, Rr tmin, Rr tmax,
-                              bool departed, AHits<Rr>& out, Rr depWindow = Rr(0), Rr nearWindow = Rr(0)) {
-    if constexpr (Full) return fullCrossings<R, Rr>(b, data, o, d, tmin, tmax, departed, out, depWindow, nearWindow);
-    else return classicCrossings<R, Rr>(b, o, d, tmin, tmax, out);
 }
 
 // The unit normal of a shape found by a numeric crossing (aspheres, torus patches, wave surfaces) at

@@ -20,14 +20,15 @@ OWEC_HD T planck(T lambdaNm, T kelvin) {
     return T(1e6) * c1 / (l2 * l2 * l * (exp(c2 / (l * kelvin)) - T(1)));
 }
 
-// Spectrum::eval (spectrum.cpp:131-148) for the kinds a scene description carries.
+// Spectrum::eval (spectrum.cpp:131-148) for the kinds a scene description carries. A black body and a
+// table are evaluated out of line: the shading kernels ask for a spectrum at dozens of places, most
+// spectra are constants, and inlined the rest made kMedium 165 KB of code, of which the instruction
+// cache held too little.
 template <class T>
-OWEC_HD T evalSpectrum(const DeviceScene& s, int32_t idx, T lambda) {
-    if (idx < 0) return T(0);
-    const owec_spectrum sp = s.spectra[idx];
-    if (sp.kind == OWEC_SPEC_CONSTANT) return T(sp.a);
+OWEC_HD_COLD T evalVaryingSpectrum(const DeviceScene* s, int32_t idx, T lambda) {
+    const owec_spectrum sp = s->spectra[idx];
     if (sp.kind == OWEC_SPEC_BLACKBODY) return T(sp.scale) * planck(lambda, T(sp.a));
-    const double* t = s.table + 2 * sp.table_offset;
+    const double* t = s->table + 2 * sp.table_offset;
     const int n = sp.table_count;
     if (lambda <= T(t[0])) return T(sp.scale * t[1]);
     if (lambda >= T(t[2 * (n - 1)])) return T(sp.scale * t[2 * (n - 1) + 1]);
@@ -39,6 +40,13 @@ OWEC_HD T evalSpectrum(const DeviceScene& s, int32_t idx, T lambda) {
     const T l0 = T(t[2 * lo]), l1 = T(t[2 * hi]);
     const T u = (lambda - l0) / (l1 - l0);
     return T(sp.scale) * (T(t[2 * lo + 1]) * (T(1) - u) + T(t[2 * hi + 1]) * u);
+}
+template <class T>
+OWEC_HD T evalSpectrum(const DeviceScene& s, int32_t idx, T lambda) {
+    if (idx < 0) return T(0);
+    const owec_spectrum& sp = s.spectra[idx];
+    if (sp.kind == OWEC_SPEC_CONSTANT) return T(sp.a);
+    return evalVaryingSpectrum(s.self, idx, lambda);
 }
 
 // Standard dry air, Ciddor (1996) two-term form, l2 in um^2 (spectra.hpp:55-58).

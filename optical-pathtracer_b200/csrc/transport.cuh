@@ -72,7 +72,7 @@ __device__ __forceinline__ double refineTriangleT(const DeviceScene& sc, uint32_
 }
 
 // Full: the scene may hold shapes beyond spheres, conic sags, plain apertures and cylinders
-// (analyticCrossings).
+// (fullCrossings).
 template <class R, class Ro, class Rr, bool Full>
 __device__ SurfacePoint<R> hitGeometry(const DeviceScene& sc, const PathRay<R>& ray, const HitRec& h) {
     SurfacePoint<R> sp;
@@ -132,8 +132,10 @@ __device__ SurfacePoint<R> hitGeometry(const DeviceScene& sc, const PathRay<R>& 
     }
     AHits<Rr> hits;
     const Rr slack = Rr(1e-6) * (Rr(1) + fabs(t));
-    const int n = analyticCrossings<Ro, Rr, Full>(bd, data, lo, ld, Rr(0), t + slack, ray.depB == h.boundary, hits);
-    const AHit<Rr>& hb = (n == 2 && fabs(hits.h1.t - t) < fabs(hits.h0.t - t)) ? hits.h1 : hits.h0;
+    int n;
+    if constexpr (Full) n = fullCrossings<Ro, Rr>(bd, data, lo, ld, Rr(0), t + slack, ray.depB == h.boundary, hits);
+    else n = classicRoots<Ro, Rr, true>(bd, lo, ld, Rr(0), t + slack, hits.h0.t, hits.h1.t);
+    const bool secondNearer = n == 2 && fabs(hits.h1.t - t) < fabs(hits.h0.t - t);
     if (n == 0) {  // not found again (rounding at a trim edge): the point on the ray
         sp.p = od + V3<double>(d) * h.t;
         sp.pLocal = bd.toLocal.point(sp.p);
@@ -141,8 +143,15 @@ __device__ SurfacePoint<R> hitGeometry(const DeviceScene& sc, const PathRay<R>& 
         sp.n = V3<R>(normalize(bd.toWorld.vector(sp.nLocal)));
         return sp;
     }
-    sp.pLocal = V3<double>(hb.p);
-    sp.nLocal = V3<double>(hb.n);
+    if constexpr (Full) {
+        const AHit<Rr>& hb = secondNearer ? hits.h1 : hits.h0;
+        sp.pLocal = V3<double>(hb.p);
+        sp.nLocal = V3<double>(hb.n);
+    } else {
+        const V3<Rr> p = classicPoint(bd, lo, ld, secondNearer ? hits.h1.t : hits.h0.t);
+        sp.pLocal = V3<double>(p);
+        sp.nLocal = V3<double>(classicNormal(bd, p));
+    }
     sp.p = bd.toWorld.point(sp.pLocal);
     sp.n = V3<R>(normalize(bd.toWorld.vector(sp.nLocal)));
     return sp;

@@ -139,7 +139,7 @@ template <> __device__ __forceinline__ float farWiden<float>() { return 4e-7f; }
 template <> __device__ __forceinline__ double farWiden<double>() { return 4e-16; }
 
 // The analytic boundary b's first acceptable crossing in (0, best); FP64 refinement when Rr = double.
-template <class R, class Rr, class T, bool Full>
+template <class R, class Rr, class T, bool Full, bool Rolled>
 __device__ __forceinline__ bool analyticCandidate(const DeviceScene& sc, const RayQuery<T>& q, uint32_t b, T best, Rr& tOut,
                                                   bool& frontOut, float& cosOut) {
     const DBoundary& bd = sc.boundaries[b];
@@ -165,18 +165,23 @@ __device__ __forceinline__ bool analyticCandidate(const DeviceScene& sc, const R
         }
     }
     if (solved) {
-    } else if constexpr (Full)
-        n = analyticCrossings<R, Rr, true>(bd, sc.shapeData + bd.dataOffset, lo, ld, tLow, Rr(best), b == q.depB, hits,
-                                           Rr(qs.errN), Rr(q.errN));
-    else n = analyticCrossings<R, Rr, false>(bd, nullptr, lo, ld, Rr(0), Rr(best), false, hits);
-#pragma unroll
+    } else if constexpr (Full) {
+        n = fullCrossings<R, Rr>(bd, sc.shapeData + bd.dataOffset, lo, ld, tLow, Rr(best), b == q.depB, hits, Rr(qs.errN),
+                                 Rr(q.errN));
+    } else {
+        n = classicRoots<R, Rr, Rolled>(bd, lo, ld, Rr(0), Rr(best), hits.h0.t, hits.h1.t);
+    }
+#pragma unroll(Rolled ? 1 : 2)
     for (int i = 0; i < 2; ++i) {
         if (i >= n) break;
-        const AHit<Rr>& h = hits.get(i);
-        const V3<T> nw = V3<T>(bd.toWorld.vector(h.n));
-        if (Full && !(h.t > Rr(0)) && (b == q.depB || !(fabs(T(h.t) * dot(q.d, nw)) <= behindWindow(q.o)))) continue;
-        if (!acceptCrossing<T>(sc, q.d, qs.errN, q.depB, q.depP, q.region, b, 0u, false, T(h.t), nw)) continue;
-        tOut = h.t;
+        const Rr t = i == 0 ? hits.h0.t : hits.h1.t;
+        V3<Rr> nl;
+        if constexpr (Full) nl = hits.get(i).n;
+        else nl = classicNormal(bd, classicPoint(bd, lo, ld, t));
+        const V3<T> nw = V3<T>(bd.toWorld.vector(nl));
+        if (Full && !(t > Rr(0)) && (b == q.depB || !(fabs(T(t) * dot(q.d, nw)) <= behindWindow(q.o)))) continue;
+        if (!acceptCrossing<T>(sc, q.d, qs.errN, q.depB, q.depP, q.region, b, 0u, false, T(t), nw)) continue;
+        tOut = t;
         frontOut = dot(q.d, nw) < T(0);
         cosOut = float(fabs(dot(q.d, nw)));
         return true;
@@ -194,7 +199,7 @@ struct AnalyticResult {
     bool front;  // met from the boundary's front side
     float cosAbs;  // |cos| between the ray and the surface normal there
 };
-template <class T, class R, class Rr, bool Full>
+template <class T, class R, class Rr, bool Full, bool Rolled>
 __device__ __noinline__ AnalyticResult<Rr> analyticHit(const DeviceScene* scp, uint32_t b, V3<double> od, V3<T> d, T best,
                                                         uint32_t depB, uint32_t region, T errN) {
     RayQuery<T> q;
@@ -210,7 +215,7 @@ __device__ __noinline__ AnalyticResult<Rr> analyticHit(const DeviceScene* scp, u
     r.t = Rr(0);
     r.front = false;
     r.cosAbs = 1.f;
-    r.ok = analyticCandidate<R, Rr, T, Full>(*scp, q, b, best, r.t, r.front, r.cosAbs);
+    r.ok = analyticCandidate<R, Rr, T, Full, Rolled>(*scp, q, b, best, r.t, r.front, r.cosAbs);
     return r;
 }
 
@@ -406,9 +411,10 @@ __device__ __forceinline__ uint32_t permuteSlots(uint32_t m, uint32_t x) {
 // Closest (AnyHit = false) or first (AnyHit = true) acceptable crossing in (0, q.tmax), as a state
 // machine that a persistent kernel can advance a few visits at a time and then hand the thread a
 // new query when this one ends. R / Rr: precision of analytic roots and of their refinement.
-// Count: keep the per-query visit and test counts (the counting pass; the timed kernels leave them out).
+// Count: keep the per-query visit and test counts (the counting pass and the whole queries of traceRay;
+// the timed persistent kernels leave them out, and take the analytic roots unrolled).
 // Full: the scene has shapes beyond spheres, conic sags, plain apertures and cylinders
-// (analyticCrossings).
+// (fullCrossings).
 template <class T, class R, class Rr, bool AnyHit, class Stack = SharedStack, bool Count = true, bool Full = false>
 struct Traversal {
     V3<T> o, d;           // the ray, camera-relative
@@ -656,7 +662,7 @@ struct Traversal {
             c->hit.t = double(t);
             c->hit.prim = 0;
         } else {
-            const AnalyticResult<Rr> ar = analyticHit<T, R, Rr, Full>(sc.self, b, c->origin(), d, limit, c->depB, c->region, c->errN);
+            const AnalyticResult<Rr> ar = analyticHit<T, R, Rr, Full, Count>(sc.self, b, c->origin(), d, limit, c->depB, c->region, c->errN);
             if (!ar.ok) return false;
             if constexpr (Full) {
                 if (!winsContact(sc, b, double(ar.t), ar.front, T(ar.cosAbs), flags)) return false;

@@ -1,9 +1,10 @@
 // Forward light walks (the reference's Tracer::walk, src/owe/transport/transport.cpp:531-595),
-// one thread per walk, binned where they end on a target boundary; and their path-replay adjoint
+// one lane per walk, binned where they end on a target boundary; and their path-replay adjoint
 // with respect to the heights of a refractive heightfield.
 //
-// A walk is short (a lens: a handful of crossings and the odd ghost; a slab: three), so each thread
-// loops over its own events with the same wide-BVH traversal as the camera paths. Bins accumulate
+// A walk is short (a lens: a handful of crossings and the odd ghost; a slab: three), so each lane
+// steps through its walk's events with the same wide-BVH traversal as the camera paths, and takes
+// another walk when it ends. Bins accumulate
 // in 64-bit fixed point (2^-32 per unit throughput), so the film is the same whatever order the
 // walks finish in.
 //
@@ -13,6 +14,9 @@
 // (the hit point moves within its surface), of refraction and reflection, of the Fresnel weight,
 // of Beer-Lambert attenuation, and finally of the bilinear splat on the target. Nothing of the
 // forward pass is stored.
+#include <algorithm>
+
+#include "dbuf.hpp"
 #include "tangents.cuh"
 #include "transport.cuh"
 #include "walk.hpp"
@@ -77,15 +81,28 @@ struct Tangents {
     bool valid;
 };
 
-template <int M, bool ADJ, bool Full>
-__device__ void walkOne(const DeviceScene& sc, const WalkParams& P, uint64_t walkIndex, StackEntry* stack, int stride,
-                        unsigned long long* bins, unsigned long long* stats, const double* g, double* dH) {
+// A walk between two events.
+template <class R>
+struct WalkState {
+    Pcg32 rng;
+    double lambda;
+    PathRay<R> ray;
+    R beta;
+    int events;
+};
+
+// How walkEvent leaves a walk.
+enum WalkEnd : int { kWalkGoes = 0, kWalkEnds = 1, kWalkBinned = 2, kWalkEscaped = 3, kWalkFault = 4 };
+
+// Walk walkIndex leaves its source.
+template <int M>
+__device__ __forceinline__ void startWalk(const DeviceScene& sc, const WalkParams& P, uint64_t walkIndex,
+                                          WalkState<typename Mode<M>::R>& ws) {
     using R = typename Mode<M>::R;
-    using Ro = typename Mode<M>::Ro;
-    using Rr = typename Mode<M>::Rr;
     const owec_walk_desc& w = P.w;
-    Pcg32 rng = Pcg32::seeded(hashCombine(w.seed, walkIndex), w.stream);
-    const double lambda = w.lambda_min + (w.lambda_max - w.lambda_min) * rng.uniform();
+    Pcg32& rng = ws.rng;
+    rng = Pcg32::seeded(hashCombine(w.seed, walkIndex), w.stream);
+    ws.lambda = w.lambda_min + (w.lambda_max - w.lambda_min) * rng.uniform();
     // emission
     const Draw2<double> e(rng);
     const V3<double> S(P.srcFrame[0], P.srcFrame[1], P.srcFrame[2]), T(P.srcFrame[3], P.srcFrame[4], P.srcFrame[5]),
@@ -112,21 +129,32 @@ __device__ void walkOne(const DeviceScene& sc, const WalkParams& P, uint64_t wal
         o = o + (S * (2 * e.u1 - 1) + T * (2 * e.u2 - 1)) * w.extent;
         dir = Ax;
     }
-    PathRay<R> ray;
+    PathRay<R>& ray = ws.ray;
     ray.o[0] = o.x; ray.o[1] = o.y; ray.o[2] = o.z;
     ray.d[0] = R(dir.x); ray.d[1] = R(dir.y); ray.d[2] = R(dir.z);
     ray.region = w.region;
     ray.depB = kNone;
     ray.depP = kNone;
     ray.errN = 0.f;
-    R beta = R(1);
-    Tangents tg;
-    tg.n = 0;
-    tg.valid = ADJ;
-    bool binned = false, escaped = false, fault = false;
-    int events = 0;
-    for (int ev = 0; ev < w.max_events; ++ev) {
-        ++events;
+    ws.beta = R(1);
+    ws.events = 0;
+}
+
+// One event of a walk: the segment to the closest crossing and what happens there.
+template <int M, bool ADJ, bool Full>
+__device__ __forceinline__ WalkEnd walkEvent(const DeviceScene& sc, const WalkParams& P, WalkState<typename Mode<M>::R>& ws,
+                                             Tangents& tg, StackEntry* stack, int stride, unsigned long long* bins,
+                                             const double* g, double* dH) {
+    using R = typename Mode<M>::R;
+    using Ro = typename Mode<M>::Ro;
+    using Rr = typename Mode<M>::Rr;
+    const owec_walk_desc& w = P.w;
+    Pcg32& rng = ws.rng;
+    const double lambda = ws.lambda;
+    PathRay<R>& ray = ws.ray;
+    R& beta = ws.beta;
+    {
+        ++ws.events;
         RayQuery<R> rq;
         rq.od = V3<double>(ray.o[0], ray.o[1], ray.o[2]);
         rq.o = V3<R>(rq.od);
@@ -138,8 +166,8 @@ __device__ void walkOne(const DeviceScene& sc, const WalkParams& P, uint64_t wal
         rq.errN = R(ray.errN);
         HitRec h;
         const int s = traceRay<R, Ro, Rr, false, Full>(sc, rq, stack, stride, h);
-        if (s == kTraceOverflow) { fault = true; break; }
-        if (s != kTraceHit) { escaped = true; break; }
+        if (s == kTraceOverflow) return kWalkFault;
+        if (s != kTraceHit) return kWalkEscaped;
         const owec_medium med = sc.media[sc.regionMedium[ray.region]];
         const DBoundary bd = sc.boundaries[h.boundary];
         const SurfacePoint<R> gp = hitGeometry<R, Ro, Rr, Full>(sc, ray, h);
@@ -220,7 +248,7 @@ __device__ void walkOne(const DeviceScene& sc, const WalkParams& P, uint64_t wal
             ray.region = other;
             ray.o[0] = gp.p.x; ray.o[1] = gp.p.y; ray.o[2] = gp.p.z;
             ray.depB = h.boundary; ray.depP = h.prim; ray.errN = errN;
-            continue;
+            return ws.events < w.max_events ? kWalkGoes : kWalkEnds;
         }
         if (op.type == OWEC_SURF_ABSORBER || op.type == OWEC_SURF_DETECTOR ||
             (w.mode == OWEC_WALK_PRIMARY_TRANSMISSION && op.type == OWEC_SURF_DIFFUSE)) {
@@ -244,9 +272,9 @@ __device__ void walkOne(const DeviceScene& sc, const WalkParams& P, uint64_t wal
                         atomicAdd(dH + tg.vert[k], acc * P.scale);
                     }
                 }
-                binned = nb > 0;
+                if (nb > 0) return kWalkBinned;
             }
-            break;
+            return kWalkEnds;
         }
         Interface<R> it;
         it.o = op;
@@ -280,7 +308,7 @@ __device__ void walkOne(const DeviceScene& sc, const WalkParams& P, uint64_t wal
             const Draw3<R> u(rng);
             ok = sampleScatter(sc, it, d, u.u1, u.u2, u.u3, false, ss);
         }
-        if (!ok) break;
+        if (!ok) return kWalkEnds;
         if (ADJ && tg.valid && tg.n > 0) {
             const V3<double> dd(d), n(gp.n);
             if (op.type == OWEC_SURF_DIELECTRIC && ss.delta && w.mode == OWEC_WALK_PRIMARY_TRANSMISSION) {
@@ -330,25 +358,82 @@ __device__ void walkOne(const DeviceScene& sc, const WalkParams& P, uint64_t wal
         ray.depB = h.boundary;
         ray.depP = h.prim;
         ray.errN = errN;
-    }
-    if (!ADJ) {
-        atomicAdd(stats + 0, 1ull);
-        if (binned) atomicAdd(stats + 1, 1ull);
-        if (escaped) atomicAdd(stats + 2, 1ull);
-        atomicAdd(stats + 3, (unsigned long long)events);
-        if (fault) atomicAdd(stats + 4, 1ull);
-    } else if (fault || (!tg.valid && tg.n > 0)) {
-        atomicAdd(stats + 4, 1ull);
+        return ws.events < w.max_events ? kWalkGoes : kWalkEnds;
     }
 }
 
+// Resident blocks per SM the lean kernels are compiled for: 128 registers with a little spilling
+// against 166 without (three blocks): 9.3 against 10.3 ms for 4.2 M lens walks, 4.4 either way for the
+// caustic slab's, 6.75 against 6.86 ms for their adjoint; two blocks 14.0, 5.6 and 7.9 ms. The Full
+// kernels spill far more and take what registers they need.
+#ifndef OWEC_WALK_MIN_BLOCKS
+#define OWEC_WALK_MIN_BLOCKS 4
+#endif
+
+// Adds a per-lane count to a counter, one atomic per warp (all lanes of the warp present).
+__device__ __forceinline__ void flushCount(unsigned long long* counter, uint32_t v) {
+    const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, v);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(counter, (unsigned long long)sum);
+}
+
+// Persistent: a lane whose walk ends takes the next one before its warp's next event, so that a warp
+// does not run its longest walk (a ghost's many reflections) with the others' lanes idle, and the
+// counters are summed per lane and added once per warp at the end instead of with four atomics on one
+// line per walk. The kernel is bound by FP64 arithmetic of few lanes and by instruction fetch (its code
+// exceeds the instruction cache). 4.2 M walks: the cemented achromat 24.1 -> 9.3 ms with the analytic
+// roots taken lazily (classicRoots), the caustic slab 4.73 -> 4.40 ms, its adjoint 7.49 -> 6.75 ms;
+// refilling only when 8 or 32 lanes are idle: 22 and 25 ms for the lens.
 template <int M, bool ADJ, bool Full>
-__global__ void __launch_bounds__(128) kWalk(DeviceScene sc, WalkParams P, unsigned long long* bins,
-                                             unsigned long long* stats, const double* g, double* dH) {
+__global__ void __launch_bounds__(128, Full ? 1 : OWEC_WALK_MIN_BLOCKS) kWalk(DeviceScene sc, WalkParams P, unsigned long long* bins,
+                                                                   unsigned long long* stats, const double* g, double* dH,
+                                                                   unsigned long long* fetch) {
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
-    for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < P.n; k += uint64_t(gridDim.x) * blockDim.x)
-        walkOne<M, ADJ, Full>(sc, P, P.first + k, stack, blockDim.x, bins, stats, g, dH);
+    const uint32_t lane = threadIdx.x & 31u;
+    WalkState<typename Mode<M>::R> ws;
+    Tangents tg;
+    uint32_t nWalks = 0, nBinned = 0, nEscaped = 0, nEvents = 0, nFaults = 0;
+    bool alive = false, exhausted = false;
+    auto flush = [&] {
+        if (!ADJ) {
+            flushCount(stats + 0, nWalks);
+            flushCount(stats + 1, nBinned);
+            flushCount(stats + 2, nEscaped);
+            flushCount(stats + 3, nEvents);
+        }
+        flushCount(stats + 4, nFaults);
+        nWalks = nBinned = nEscaped = nEvents = nFaults = 0;
+    };
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !alive);
+        if (!exhausted && idle) {
+            if (__any_sync(0xFFFFFFFFu, nEvents > (1u << 24))) flush();  // a warp's sum stays within 32 bits
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(fetch, (unsigned long long)__popc(idle));
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            exhausted = base + __popc(idle) >= P.n;
+            const uint64_t k = base + __popc(idle & ((1u << lane) - 1u));
+            if (!alive && k < P.n && P.w.max_events > 0) {
+                startWalk<M>(sc, P, P.first + k, ws);
+                tg.n = 0;
+                tg.valid = ADJ;
+                alive = true;
+            }
+        }
+        if (__ballot_sync(0xFFFFFFFFu, alive) == 0) break;
+        if (alive) {
+            const WalkEnd e = walkEvent<M, ADJ, Full>(sc, P, ws, tg, stack, blockDim.x, bins, g, dH);
+            if (e != kWalkGoes) {
+                alive = false;
+                ++nWalks;
+                nBinned += e == kWalkBinned;
+                nEscaped += e == kWalkEscaped;
+                nEvents += uint32_t(ws.events);
+                nFaults += e == kWalkFault || (ADJ && !tg.valid && tg.n > 0);
+            }
+        }
+    }
+    flush();
 }
 
 // kWalk for the scene's shapes (the lean traversal unless the scene needs the full set).
@@ -356,8 +441,17 @@ template <int M, bool ADJ>
 void walkKernel(const DeviceScene& sc, const WalkParams& P, unsigned long long* bins, unsigned long long* stats,
                 const double* g, double* dH, int grid, cudaStream_t s) {
     const size_t smem = traversalSharedBytes(128);
-    if (sc.fullFeatures) kWalk<M, ADJ, true><<<grid, 128, smem, s>>>(sc, P, bins, stats, g, dH);
-    else kWalk<M, ADJ, false><<<grid, 128, smem, s>>>(sc, P, bins, stats, g, dH);
+    unsigned long long* fetch = stats + kWalkFetchWord;
+    OWEC_CUDA(cudaMemsetAsync(fetch, 0, sizeof(*fetch), s));
+    grid = int(std::min<uint64_t>(uint64_t(grid), (P.n + 127) / 128));
+    if (grid == 0) return;
+    if (sc.fullFeatures) kWalk<M, ADJ, true><<<grid, 128, smem, s>>>(sc, P, bins, stats, g, dH, fetch);
+    else kWalk<M, ADJ, false><<<grid, 128, smem, s>>>(sc, P, bins, stats, g, dH, fetch);
+}
+
+__global__ void __launch_bounds__(256) kResolveWalk(const unsigned long long* bins, size_t n, double scale, double* out) {
+    const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (i < n) out[i] = double(bins[i]) * scale;
 }
 
 WalkParams makeParams(const owec_walk_desc& w, const Xform& targetToLocal, uint64_t first, uint64_t n, double scale,
@@ -389,6 +483,10 @@ void launchWalk(int mode, const DeviceScene& sc, const owec_walk_desc& w, const 
     if (mode == OWEC_PRECISION_FP64) walkKernel<OWEC_PRECISION_FP64, false>(sc, P, bins, stats, nullptr, nullptr, grid, s);
     else if (mode == OWEC_PRECISION_FP32) walkKernel<OWEC_PRECISION_FP32, false>(sc, P, bins, stats, nullptr, nullptr, grid, s);
     else walkKernel<OWEC_PRECISION_MIXED, false>(sc, P, bins, stats, nullptr, nullptr, grid, s);
+}
+
+void launchResolveWalk(const unsigned long long* bins, size_t n, double scale, double* out, cudaStream_t s) {
+    kResolveWalk<<<unsigned((n + 255) / 256), 256, 0, s>>>(bins, n, scale, out);
 }
 
 void launchWalkAdjoint(int mode, const DeviceScene& sc, const owec_walk_desc& w, const Xform& targetToLocal,
