@@ -507,9 +507,9 @@ typedef struct owec_adjoint_stats {
                            * spheres and meshes, more than 12 heights): left out of the gradient */
     uint64_t faults;      /* bounded loops that ran out */
     double seconds;       /* device time of the call */
-    uint64_t device_bytes;/* device memory the call held beyond what the context held before it: its
-                           * buffers (loss gradient, height gradient, checkpoints, replayed film) and the
-                           * replay kernel's per-thread stacks */
+    uint64_t device_bytes;/* device memory of the call's buffers: loss gradient, height gradient,
+                           * checkpoints, replayed film (the context keeps all but the last for the next
+                           * call) */
     double replay_seconds;/* of seconds, the device time of the derivative replay alone (the rest is the
                            * wavefront phase that runs the paths to their first heightfield crossing) */
 } owec_adjoint_stats;

@@ -5,12 +5,16 @@
 // World::build the kernels need (src/owe/scene/world.cpp:263-350: frames, world boxes, the scene
 // radius and the light table) and converts the geometry to camera-relative FP32. owec_pass runs
 // batches of one-sample sub-passes through the wavefront loop and folds them into the film.
+#include <sys/mman.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "bvh_build.hpp"
@@ -364,6 +368,24 @@ void invertRigid(const double m[12], double out[12]) {
 }  // namespace
 
 // ------------------------------------------------------------------ the context
+// owec_cast_rays: a call of a few chunks goes through the context's own page-locked block (page-locking
+// costs 1 to 3 ms a call here up to 2 MB, whatever the size); a larger one through kCastWorkers host threads
+// with a chunk each, staged in a second block that the first such call page-locks.
+constexpr int kCastWorkers = 4;
+constexpr uint64_t kCastChunk = 16384, kCastSerial = 16;  // up to here one thread costs less than page-locking
+constexpr size_t kCastBytesPerRay = 48 + 16;
+constexpr size_t kHostReports = 4096;  // the context block's first part: what kernels report to the host
+constexpr size_t kHostBlock = kHostReports + kCastChunk * kCastBytesPerRay;
+struct CastWorker {
+    cudaStream_t stream = nullptr;
+    void ensure() {
+        if (!stream) OWEC_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    }
+    ~CastWorker() {
+        if (stream) cudaStreamDestroy(stream);
+    }
+};
+
 struct owec_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -453,12 +475,24 @@ struct owec_ctx {
     double lastPathAdjointSeconds = 0;
     DBuf<uint32_t> dHfTris;
     DBuf<double> dHfVerts, dHfHeights;
+    // the adjoints' workspaces: the loss gradient per bin or film value, the gradient per height, the
+    // counters, and the camera paths' checkpoints
+    DBuf<double> dLossGrad, dHeightGrad;
+    DBuf<unsigned long long> dAdjointStats;
+    DBuf<uint8_t> dCheckpoints;
+    DBuf<uint32_t> dCheckpointCount;
+    DBuf<StatCounters> dAdjointCounters;
     struct MeshCopy {
         std::vector<double> verts;    // shape-frame vertices as uploaded
         std::vector<uint32_t> tris;
     };
     std::vector<MeshCopy> meshes;    // per boundary (empty for analytic ones)
     double lastWalkSeconds = 0, lastAdjointSeconds = 0;
+
+    CastWorker castWorkers[kCastWorkers];
+    DBuf<char> dCast;  // the chunks' rays and hits on the device
+    char* hostBlock = nullptr;    // page-locked, kHostBlock bytes
+    char* castStaging = nullptr;  // page-locked, a chunk per worker
 
     // forward light walks
     owec_walk_desc walk{};
@@ -1386,11 +1420,12 @@ void runParticles(owec_ctx& c, int spp) {
 // each path at its first surface event on the heightfield, leaving its state there (a checkpoint);
 // the derivative replay then resumes only those paths. Paths that never meet the heightfield carry
 // no derivative and so cost one forward pass's work and nothing more.
-// Returns the number of camera paths the first phase generated; freeDuring receives the device's free
-// memory while the phases' buffers are still held.
+// Returns the number of camera paths the first phase generated; heldBytes grows by the checkpoints'
+// device memory. The checkpoints and counters are the context's: allocated and freed in every call, with
+// two questions for the device's free memory, they cost an optimisation step several milliseconds.
 template <int M>
 uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, int spp, const PathAdjointTargets& t,
-                                bool fixedDecisions, size_t& freeDuring, double& replaySeconds) {
+                                bool fixedDecisions, size_t& heldBytes, double& replaySeconds) {
     using R = ModeR<M>;
     const uint32_t nPix = pp.nPixels;
     const uint32_t target = std::max<uint32_t>(nPix, 1u << 21);
@@ -1399,9 +1434,13 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
     Queues q;
     PathBuffers<R> pb = pathState<M>(c, cap, q);
     // every path checkpoints at most once (it ends there)
-    DBuf<uint8_t> ckpt(size_t(cap) * pathCheckpointBytes(M));
-    DBuf<uint32_t> ckptCount(1);
-    DBuf<StatCounters> st(1);  // the phase's own counters: the context's transport statistics stay the forward's
+    DBuf<uint8_t>& ckpt = c.dCheckpoints;
+    DBuf<uint32_t>& ckptCount = c.dCheckpointCount;
+    DBuf<StatCounters>& st = c.dAdjointCounters;  // the phase's own: the transport statistics stay the forward's
+    ckpt.reserve(size_t(cap) * pathCheckpointBytes(M));
+    ckptCount.reserve(1);
+    st.reserve(1);
+    heldBytes += size_t(cap) * pathCheckpointBytes(M);
     OWEC_CUDA(cudaMemsetAsync(st.get(), 0, sizeof(StatCounters), c.stream));
     pp.ckptBoundary = c.hf.boundary;
     pp.ckptCount = ckptCount.get();
@@ -1436,9 +1475,107 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
     StatCounters hs{};
     OWEC_CUDA(cudaMemcpyAsync(&hs, st.get(), sizeof(StatCounters), cudaMemcpyDeviceToHost, c.stream));
     OWEC_CUDA(cudaStreamSynchronize(c.stream));
-    size_t total = 0;
-    OWEC_CUDA(cudaMemGetInfo(&freeDuring, &total));
     return hs.paths;
+}
+
+// m rays packed into `host` (origins, directions; the hits behind them), one copy each way, queued on s.
+template <int M>
+void castChunk(const owec_ctx& c, char* host, char* device, uint64_t m, const double* o, const double* d, cudaStream_t s) {
+    std::memcpy(host, o, 24 * m);
+    std::memcpy(host + 24 * m, d, 24 * m);
+    char* hits = device + 48 * m;
+    OWEC_CUDA(cudaMemcpyAsync(device, host, 48 * m, cudaMemcpyHostToDevice, s));
+    launchCastRays<M>(c.ds, m, reinterpret_cast<double*>(device), reinterpret_cast<double*>(device + 24 * m),
+                      reinterpret_cast<uint32_t*>(hits + 8 * m), reinterpret_cast<uint32_t*>(hits + 12 * m),
+                      reinterpret_cast<double*>(hits), c.numSMs * 8, s);
+    checkLaunch();
+    OWEC_CUDA(cudaMemcpyAsync(host + 48 * m, hits, 16 * m, cudaMemcpyDeviceToHost, s));
+}
+void unpackHits(const char* host, uint64_t m, uint32_t* boundary, uint32_t* prim, double* t) {
+    const char* hits = host + 48 * m;
+    std::memcpy(t, hits, 8 * m);
+    std::memcpy(boundary, hits + 8 * m, 4 * m);
+    std::memcpy(prim, hits + 12 * m, 4 * m);
+}
+
+// Host rays, a few on the context's stream, more in chunks by up to kCastWorkers host threads. Packing and
+// unpacking the 64 bytes of a ray on one core, the driver's own staging of pageable copies, the faults of
+// the results' fresh pages and five allocations a call took ten times the kernel's time (2^20 rays: 10.5 ms
+// around a 0.97 ms kernel; 4.2 ms so; chunks of 4096 rays, two to a thread in turn: 8.9 ms).
+template <int M>
+void castRays(owec_ctx& c, uint64_t n, const double* o, const double* d, uint32_t* boundary, uint32_t* prim, double* t) {
+    const uint64_t chunks = (n + kCastChunk - 1) / kCastChunk;
+    if (chunks <= kCastSerial) {
+        char* staging = c.hostBlock + kHostReports;
+        c.dCast.reserve(std::min(n, kCastChunk) * kCastBytesPerRay);
+        for (uint64_t a = 0; a < n; a += kCastChunk) {
+            const uint64_t m = std::min(kCastChunk, n - a);
+            castChunk<M>(c, staging, c.dCast.get(), m, o + 3 * a, d + 3 * a, c.stream);
+            OWEC_CUDA(cudaStreamSynchronize(c.stream));
+            unpackHits(staging, m, boundary + a, prim + a, t + a);
+        }
+        return;
+    }
+    constexpr int workers = kCastWorkers;
+    constexpr size_t slot = kCastChunk * kCastBytesPerRay;
+    if (!c.castStaging) OWEC_CUDA(cudaMallocHost(&c.castStaging, kCastWorkers * slot));
+    c.dCast.reserve(kCastWorkers * slot);
+    for (int k = 0; k < workers; ++k) c.castWorkers[k].ensure();
+    OWEC_CUDA(cudaStreamSynchronize(c.stream));  // the workers' streams read what it published
+    std::exception_ptr failed[kCastWorkers];
+    auto work = [&](int k) {
+        cudaStream_t s = c.castWorkers[k].stream;
+        char* host = c.castStaging + size_t(k) * slot;
+        try {
+            OWEC_CUDA(cudaSetDevice(c.device));
+            for (uint64_t i = uint64_t(k); i < chunks; i += uint64_t(workers)) {
+                const uint64_t a = i * kCastChunk, m = std::min(kCastChunk, n - a);
+                castChunk<M>(c, host, c.dCast.get() + size_t(k) * slot, m, o + 3 * a, d + 3 * a, s);
+                OWEC_CUDA(cudaStreamSynchronize(s));
+                unpackHits(host, m, boundary + a, prim + a, t + a);
+            }
+        } catch (...) {
+            failed[k] = std::current_exception();
+            cudaStreamSynchronize(s);  // nothing of a failed worker is left in flight
+        }
+    };
+    {
+        struct Joined {
+            std::vector<std::thread> threads;
+            ~Joined() { for (std::thread& th : threads) th.join(); }
+        } joined;
+        for (int k = 1; k < workers; ++k) joined.threads.emplace_back(work, k);
+        work(0);
+    }
+    for (const std::exception_ptr& e : failed)
+        if (e) std::rethrow_exception(e);
+}
+
+// The pages of a large result buffer touched by several threads where most of them are not yet resident: a
+// read-back into fresh memory takes its page faults one by one on the copying thread (8 MB: 3.7 ms,
+// against 0.4 ms resident). The buffer is about to be overwritten whole.
+void touchPages(void* dst, size_t bytes) {
+    constexpr size_t kPage = 4096, kLeast = 1u << 20;
+    if (bytes < kLeast) return;
+    char* first = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(dst) + kPage - 1) & ~uintptr_t(kPage - 1));
+    const size_t pages = size_t(static_cast<char*>(dst) + bytes - first) / kPage;
+    std::vector<unsigned char> resident(pages);
+    if (mincore(first, pages * kPage, resident.data()) != 0) return;
+    size_t missing = 0;
+    for (unsigned char r : resident) missing += !(r & 1);
+    if (missing < pages / 4) return;
+    const size_t workers = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), missing / 64 + 1});
+    auto work = [&](size_t k) {
+        for (size_t p = pages * k / workers; p < pages * (k + 1) / workers; ++p)
+            if (!(resident[p] & 1)) *static_cast<volatile char*>(first + p * kPage) = 0;
+    };
+    std::vector<std::thread> threads;
+    try {
+        for (size_t k = 1; k < workers; ++k) threads.emplace_back(work, k);
+    } catch (...) {  // fewer threads: the copy faults the rest in
+    }
+    work(0);
+    for (std::thread& th : threads) th.join();
 }
 
 }  // namespace
@@ -1492,7 +1629,8 @@ int owec_open(int device, owec_ctx** out) {
         OWEC_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
         OWEC_CUDA(cudaEventCreate(&c->passStart));
         OWEC_CUDA(cudaEventCreate(&c->passStop));
-        OWEC_CUDA(cudaMallocHost(&c->hostCounts, 8 * sizeof(uint32_t)));
+        OWEC_CUDA(cudaMallocHost(&c->hostBlock, kHostBlock));
+        c->hostCounts = reinterpret_cast<uint32_t*>(c->hostBlock);
         c->dCounts.resize(8);
         c->dStats.resize(1);
         c->dScene.resize(1);
@@ -1515,7 +1653,8 @@ int owec_close(owec_ctx* ctx) {
         for (cudaEvent_t e : ctx->travEvents) cudaEventDestroy(e);
         cudaEventDestroy(ctx->passStart);
         cudaEventDestroy(ctx->passStop);
-        cudaFreeHost(ctx->hostCounts);
+        cudaFreeHost(ctx->hostBlock);
+        if (ctx->castStaging) cudaFreeHost(ctx->castStaging);
         cudaStream_t s = ctx->stream;
         delete ctx;  // frees the device buffers
         cudaStreamDestroy(s);
@@ -1618,6 +1757,7 @@ int owec_resolve(owec_ctx* ctx, double* xyz, double* samples) {
                 launchResolveSplats(ctx->dSplat.get(), uint32_t(np), ctx->particles > 0 ? 1.0 / ctx->particles : 0.0,
                                     ctx->dResolved.get(), ctx->stream);
                 checkLaunch();
+                touchPages(xyz, 3 * np * 8);
                 OWEC_CUDA(cudaMemcpyAsync(xyz, ctx->dResolved.get(), 3 * np * 8, cudaMemcpyDeviceToHost, ctx->stream));
                 OWEC_CUDA(cudaStreamSynchronize(ctx->stream));
             }
@@ -1629,6 +1769,7 @@ int owec_resolve(owec_ctx* ctx, double* xyz, double* samples) {
             launchResolve(ctx->dFilm.get(), ctx->dComp.get(), ctx->dSamples.get(), uint32_t(np), ctx->dResolved.get(),
                           ctx->stream);
             checkLaunch();
+            touchPages(xyz, 3 * np * 8);
             OWEC_CUDA(cudaMemcpyAsync(xyz, ctx->dResolved.get(), 3 * np * 8, cudaMemcpyDeviceToHost, ctx->stream));
         }
         if (samples)
@@ -1745,15 +1886,17 @@ int owec_set_pass_index(owec_ctx* ctx, uint64_t pass_index) {
     });
 }
 
+// The film is cleared in place: freeing it here and allocating it again in the next pass cost 2 to 3 ms
+// a frame, and at times ten (cudaFree waits for the device and unmaps).
 int owec_reset_film(owec_ctx* ctx) {
     return guarded([&] {
         require(ctx != nullptr, "owec_reset_film: null context");
+        OWEC_CUDA(cudaSetDevice(ctx->device));
         ctx->passCount = 0;
-        ctx->dFilm.release();
-        ctx->dComp.release();
-        ctx->dSamples.release();
-        ctx->dSplat.release();
         ctx->particles = 0;
+        for (DBuf<double>* b : {&ctx->dFilm, &ctx->dComp, &ctx->dSamples})
+            if (b->size()) OWEC_CUDA(cudaMemsetAsync(b->get(), 0, b->bytes(), ctx->stream));
+        if (ctx->dSplat.size()) OWEC_CUDA(cudaMemsetAsync(ctx->dSplat.get(), 0, ctx->dSplat.bytes(), ctx->stream));
         OWEC_CUDA(cudaMemsetAsync(ctx->dStats.get(), 0, sizeof(StatCounters), ctx->stream));
         OWEC_CUDA(cudaStreamSynchronize(ctx->stream));
     });
@@ -1791,27 +1934,11 @@ int owec_cast_rays(owec_ctx* ctx, uint64_t n, const double* origins, const doubl
         if (n == 0) return;
         OWEC_CUDA(cudaSetDevice(ctx->device));
         ensureReady(*ctx);
-        DBuf<double> o(3 * n), d(3 * n), tt(n);
-        DBuf<uint32_t> b(n), p(n);
-        OWEC_CUDA(cudaMemcpyAsync(o.get(), origins, 24 * n, cudaMemcpyHostToDevice, ctx->stream));
-        OWEC_CUDA(cudaMemcpyAsync(d.get(), directions, 24 * n, cudaMemcpyHostToDevice, ctx->stream));
-        const int grid = ctx->numSMs * 8;
         switch (ctx->settings.precision) {
-            case OWEC_PRECISION_MIXED:
-                launchCastRays<OWEC_PRECISION_MIXED>(ctx->ds, n, o.get(), d.get(), b.get(), p.get(), tt.get(), grid, ctx->stream);
-                break;
-            case OWEC_PRECISION_FP32:
-                launchCastRays<OWEC_PRECISION_FP32>(ctx->ds, n, o.get(), d.get(), b.get(), p.get(), tt.get(), grid, ctx->stream);
-                break;
-            default:
-                launchCastRays<OWEC_PRECISION_FP64>(ctx->ds, n, o.get(), d.get(), b.get(), p.get(), tt.get(), grid, ctx->stream);
-                break;
+            case OWEC_PRECISION_MIXED: castRays<OWEC_PRECISION_MIXED>(*ctx, n, origins, directions, boundary, prim, t); break;
+            case OWEC_PRECISION_FP32: castRays<OWEC_PRECISION_FP32>(*ctx, n, origins, directions, boundary, prim, t); break;
+            default: castRays<OWEC_PRECISION_FP64>(*ctx, n, origins, directions, boundary, prim, t); break;
         }
-        checkLaunch();
-        OWEC_CUDA(cudaMemcpyAsync(boundary, b.get(), 4 * n, cudaMemcpyDeviceToHost, ctx->stream));
-        OWEC_CUDA(cudaMemcpyAsync(prim, p.get(), 4 * n, cudaMemcpyDeviceToHost, ctx->stream));
-        OWEC_CUDA(cudaMemcpyAsync(t, tt.get(), 8 * n, cudaMemcpyDeviceToHost, ctx->stream));
-        OWEC_CUDA(cudaStreamSynchronize(ctx->stream));
     });
 }
 
@@ -1933,8 +2060,9 @@ int owec_walk(owec_ctx* ctx, const owec_walk_desc* w, uint64_t first, uint64_t n
             ctx->walk = *w;
             ctx->hasWalk = true;
             ctx->walks = 0;
-            ctx->dWalkBins.resize(size_t(w->width) * w->height);
-            ctx->dWalkStats.resize(kWalkStatWords);
+            const size_t nb = size_t(w->width) * w->height;
+            if (ctx->dWalkBins.size() != nb) ctx->dWalkBins.resize(nb);
+            ctx->dWalkStats.reserve(kWalkStatWords);
             OWEC_CUDA(cudaMemsetAsync(ctx->dWalkBins.get(), 0, ctx->dWalkBins.bytes(), ctx->stream));
             OWEC_CUDA(cudaMemsetAsync(ctx->dWalkStats.get(), 0, ctx->dWalkStats.bytes(), ctx->stream));
         }
@@ -1958,10 +2086,7 @@ int owec_walk_resolve(owec_ctx* ctx, double* bins, owec_walk_stats* stats) {
         require(ctx->hasWalk, "no walks run", OWEC_E_STATE);
         const owec_walk_desc& w = ctx->walk;
         const size_t nb = size_t(w.width) * w.height;
-        std::vector<unsigned long long> fixed(nb), st(5);
-        OWEC_CUDA(cudaMemcpyAsync(fixed.data(), ctx->dWalkBins.get(), nb * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        OWEC_CUDA(cudaMemcpyAsync(st.data(), ctx->dWalkStats.get(), 5 * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        OWEC_CUDA(cudaStreamSynchronize(ctx->stream));
+        unsigned long long st[kWalkStats];
         if (bins) {
             double measure;
             if (w.source_kind == OWEC_SOURCE_POINT) measure = 2 * kPi * (1 - std::cos(w.extent));
@@ -1969,8 +2094,14 @@ int owec_walk_resolve(owec_ctx* ctx, double* bins, owec_walk_stats* stats) {
             else measure = 4 * w.extent * w.extent;
             const double binArea = (2 * w.half_x / w.width) * (2 * w.half_y / w.height);
             const double scale = ctx->walks ? measure / (double(ctx->walks) * binArea) / 4294967296.0 : 0.0;
-            for (size_t i = 0; i < nb; ++i) bins[i] = double(fixed[i]) * scale;
+            ctx->dResolved.reserve(nb);
+            launchResolveWalk(ctx->dWalkBins.get(), nb, scale, ctx->dResolved.get(), ctx->stream);
+            checkLaunch();
+            touchPages(bins, nb * 8);
+            OWEC_CUDA(cudaMemcpyAsync(bins, ctx->dResolved.get(), nb * 8, cudaMemcpyDeviceToHost, ctx->stream));
         }
+        OWEC_CUDA(cudaMemcpyAsync(st, ctx->dWalkStats.get(), sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
+        OWEC_CUDA(cudaStreamSynchronize(ctx->stream));
         if (stats) {
             stats->walks = st[0];
             stats->binned = st[1];
@@ -2024,8 +2155,11 @@ int owec_walk_adjoint(owec_ctx* ctx, const owec_walk_desc* w, uint64_t first, ui
         OWEC_CUDA(cudaSetDevice(ctx->device));
         ensureReady(*ctx);
         const size_t nb = size_t(w->width) * w->height, nh = ctx->hfVertices;
-        DBuf<double> dG(nb), dDH(nh);
-        DBuf<unsigned long long> st(kWalkStatWords);
+        DBuf<double>&dG = ctx->dLossGrad, &dDH = ctx->dHeightGrad;
+        DBuf<unsigned long long>& st = ctx->dAdjointStats;
+        dG.reserve(nb);
+        dDH.reserve(nh);
+        st.reserve(kWalkStatWords);
         OWEC_CUDA(cudaMemcpyAsync(dG.get(), g, nb * 8, cudaMemcpyHostToDevice, ctx->stream));
         OWEC_CUDA(cudaMemsetAsync(dDH.get(), 0, nh * 8, ctx->stream));
         OWEC_CUDA(cudaMemsetAsync(st.get(), 0, st.bytes(), ctx->stream));
@@ -2112,12 +2246,15 @@ int owec_path_adjoint(owec_ctx* ctx, uint64_t first_pass, int spp, int flags, co
         require(first_pass + uint64_t(spp) <= (1ull << 32), "owec_path_adjoint: the PCG32 stream index is 32 bits");
         OWEC_CUDA(cudaSetDevice(ctx->device));
         ensureReady(*ctx);
-        size_t freeBefore = 0, freeDuring = 0, total = 0;
-        OWEC_CUDA(cudaMemGetInfo(&freeBefore, &total));
         const uint32_t nPix = uint32_t(ctx->ds.det.width) * uint32_t(ctx->ds.det.height);
         const size_t nh = ctx->hfVertices;
-        DBuf<double> dG(3 * size_t(nPix)), dDH(nh), dRep(replay_xyz ? 3 * size_t(nPix) : 0);
-        DBuf<unsigned long long> ctr(4);
+        DBuf<double>&dG = ctx->dLossGrad, &dDH = ctx->dHeightGrad;
+        DBuf<double> dRep(replay_xyz ? 3 * size_t(nPix) : 0);
+        DBuf<unsigned long long>& ctr = ctx->dAdjointStats;
+        dG.reserve(3 * size_t(nPix));
+        dDH.reserve(nh);
+        ctr.reserve(kWalkStatWords);
+        size_t heldBytes = (3 * size_t(nPix) + nh) * 8 + 4 * 8 + dRep.bytes();
         OWEC_CUDA(cudaMemcpyAsync(dG.get(), g, 3 * size_t(nPix) * 8, cudaMemcpyHostToDevice, ctx->stream));
         OWEC_CUDA(cudaMemsetAsync(dDH.get(), 0, nh * 8, ctx->stream));
         OWEC_CUDA(cudaMemsetAsync(ctr.get(), 0, 4 * 8, ctx->stream));
@@ -2151,18 +2288,17 @@ int owec_path_adjoint(owec_ctx* ctx, uint64_t first_pass, int spp, int flags, co
                 done += int(S);
             }
         } else if (ctx->settings.precision == OWEC_PRECISION_FP64) {
-            cameraPaths = runAdjointCheckpointed<OWEC_PRECISION_FP64>(*ctx, pp, first_pass, spp, t, fixed, freeDuring,
+            cameraPaths = runAdjointCheckpointed<OWEC_PRECISION_FP64>(*ctx, pp, first_pass, spp, t, fixed, heldBytes,
                                                                       replaySeconds);
         } else if (ctx->settings.precision == OWEC_PRECISION_FP32) {
-            cameraPaths = runAdjointCheckpointed<OWEC_PRECISION_FP32>(*ctx, pp, first_pass, spp, t, fixed, freeDuring,
+            cameraPaths = runAdjointCheckpointed<OWEC_PRECISION_FP32>(*ctx, pp, first_pass, spp, t, fixed, heldBytes,
                                                                       replaySeconds);
         } else {
-            cameraPaths = runAdjointCheckpointed<OWEC_PRECISION_MIXED>(*ctx, pp, first_pass, spp, t, fixed, freeDuring,
+            cameraPaths = runAdjointCheckpointed<OWEC_PRECISION_MIXED>(*ctx, pp, first_pass, spp, t, fixed, heldBytes,
                                                                       replaySeconds);
         }
         OWEC_CUDA(cudaEventRecord(ctx->passStop, ctx->stream));
         OWEC_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (replay_xyz) OWEC_CUDA(cudaMemGetInfo(&freeDuring, &total));  // the buffers and the kernel's stacks, held
         std::vector<double> h(nh);
         unsigned long long counts[4];
         OWEC_CUDA(cudaMemcpyAsync(h.data(), dDH.get(), nh * 8, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2180,7 +2316,7 @@ int owec_path_adjoint(owec_ctx* ctx, uint64_t first_pass, int spp, int flags, co
             stats->dropped = counts[2];
             stats->faults = counts[3];
             stats->seconds = ms * 1e-3;
-            stats->device_bytes = freeBefore > freeDuring ? uint64_t(freeBefore - freeDuring) : 0;
+            stats->device_bytes = heldBytes;
             stats->replay_seconds = replay_xyz ? ms * 1e-3 : replaySeconds;
         }
     });

@@ -45,7 +45,7 @@ class WalkFilm(torch.autograd.Function):
     def backward(ctx, grad_bins):
         context, boundary, base_z, desc, first, n, h, shape = ctx.args
         _ensure_heights(context, boundary, base_z, h)
-        g = grad_bins.detach().cpu().numpy().astype(np.float64)
+        g = np.asarray(grad_bins.detach().cpu().numpy(), np.float64)
         dh = context.walk_adjoint(desc, first, n, g)
         return torch.from_numpy(dh.reshape(shape)).to(grad_bins.dtype), None, None, None, None, None, None
 
@@ -69,13 +69,13 @@ class CameraFilm(torch.autograd.Function):
         img, _ = context.resolve(samples=False)
         replay = first_pass if adjoint_pass is None else adjoint_pass
         ctx.args = (context, boundary, base_z, replay, spp, fixed_decisions, h, heights.shape)
-        return torch.from_numpy(np.array(img)).to(heights.dtype)
+        return torch.from_numpy(img).to(heights.dtype)  # resolve's own fresh array
 
     @staticmethod
     def backward(ctx, grad_img):
         context, boundary, base_z, first_pass, spp, fixed, h, shape = ctx.args
         _ensure_heights(context, boundary, base_z, h)
-        g = grad_img.detach().cpu().numpy().astype(np.float64)
+        g = np.asarray(grad_img.detach().cpu().numpy(), np.float64)
         dh = context.path_adjoint(first_pass, spp, g, fixed_decisions=fixed)
         return torch.from_numpy(dh.reshape(shape)).to(grad_img.dtype), None, None, None, None, None, None, None
 
