@@ -109,6 +109,7 @@ struct DeviceScene {
     int32_t fullFeatures;     // 1: shapes beyond spheres, conic sags, plain apertures and cylinders, a
                               // planet-sized sphere, contacts or textured materials (the kernels' Full
                               // instantiations)
+    uint32_t opticsUsed;      // kOpticsSimple, kOpticsGeneral: the surface kernels with anything to do
     uint32_t nRegions, nBoundaries, nLights, nMedia;
     const WideNode* nodes;
     const PrimRec* prims;
@@ -138,5 +139,6 @@ struct DeviceScene {
     uint32_t eventLogCap;
 };
 constexpr int kEventRecord = 16;
+constexpr uint32_t kOpticsSimple = 1u, kOpticsGeneral = 2u;
 
 }  // namespace owec

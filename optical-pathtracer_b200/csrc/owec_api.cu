@@ -390,7 +390,9 @@ struct owec_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t passStart = nullptr, passStop = nullptr;
-    std::vector<cudaEvent_t> travEvents;
+    // the shadow kernels' stream, forked from the pass's after a bounce's events and joined before the next's
+    cudaStream_t shadowStream = nullptr;
+    cudaEvent_t eventsDone = nullptr, shadowDone = nullptr;
     int numSMs = 148;
     char name[256] = {0};
 
@@ -467,7 +469,14 @@ struct owec_ctx {
     uint32_t eventLogCap = 0;
     uint32_t capacity = 0;
     double lastPassSeconds = 0, lastIntersectSeconds = 0, lastShadowSeconds = 0, lastIntersectLaunches = 0;
-    uint32_t* hostCounts = nullptr;  // pinned
+    // page-locked: the paths each bounce started with, as the device reports them, and the pass's clock
+    struct HostProgress {
+        unsigned long long bounce[kProgressSlots];
+        BounceClock clock;
+    };
+    HostProgress* progress = nullptr;
+    uint32_t bounces = 0;  // bounces queued so far, over all passes
+    DBuf<BounceClock> dClock;
 
     // the heightfield the adjoint differentiates
     HeightfieldParams hf{kNone, nullptr, {0, 0, 1}};
@@ -1007,6 +1016,12 @@ void uploadScene(owec_ctx& c, const owec_scene_desc& d) {
     ds.boundaries = c.dBoundaries.get();
     ds.lights = c.dLights.get();
     ds.shapeData = c.dShapeData.get();
+    ds.opticsUsed = 0;
+    for (uint32_t i = 0; i < d.n_boundaries; ++i) {
+        const int32_t type = d.optics[d.boundaries[i].optics].type;
+        const bool simple = type == OWEC_SURF_DIFFUSE || type == OWEC_SURF_ABSORBER || type == OWEC_SURF_DETECTOR;
+        ds.opticsUsed |= simple ? kOpticsSimple : kOpticsGeneral;
+    }
     ds.fullFeatures = 0;
     for (uint32_t i = 0; i < d.n_boundaries; ++i) {
         const owec_boundary& b = d.boundaries[i];
@@ -1190,8 +1205,8 @@ PathBuffers<ModeR<M>> pathState(owec_ctx& c, uint32_t cap, Queues& q) {
         c.dQueueShadow.resize(cap);
         c.capacity = cap;
     }
-    q = Queues{{c.dQueue0.get(), c.dQueue1.get()}, c.dQueueSurf.get(), c.dQueueShadow.get(), c.dCounts.get(),
-               c.dQueueSurfSimple.get()};
+    q = Queues{{c.dQueue0.get(), c.dQueue1.get()}, c.dQueueSurf.get(), c.dQueueShadow.get(), nullptr,
+               c.dQueueSurfSimple.get(), nullptr, nullptr, 0};
     return PathBuffers<R>{reinterpret_cast<PathRay<R>*>(c.dPathRay.get()), reinterpret_cast<PathSpec<R>*>(c.dPathSpec.get()),
                           reinterpret_cast<PathAux*>(c.dPathAux.get()), reinterpret_cast<HitRec*>(c.dHit.get()),
                           reinterpret_cast<ShadowRay<R>*>(c.dShadow.get())};
@@ -1202,61 +1217,108 @@ PathBuffers<ModeR<M>> pathState(owec_ctx& c, uint32_t cap, Queues& q) {
 #define OWEC_SHADING_GRID 8
 #endif
 
-// The bounces of one batch of camera paths already generated into pb: intersect, medium, surface
-// and shadow kernels per bounce until the active queue is empty. The kernels read their queue
-// lengths on the device, so the bounces are queued without a look at the host: maxDepth + 1 of
-// them first (a path without null boundaries ends by then), then four at a time until the queue
-// is empty. The host waits once per batch, not once per bounce. With timed, CUDA events around the
-// intersect and shadow launches add their device seconds to travSeconds.
-template <int M>
-void runBounces(owec_ctx& c, const PassParams& pp, PathBuffers<ModeR<M>>& pb, Queues& q, StatCounters* st, int grid,
-                bool timed, double travSeconds[2], int& evUsed, int& intersectLaunches) {
-    cudaStream_t s = c.stream;
-    int cur = 0;
-    int nextCheck = pp.maxDepth + 1;
-    for (int bounce = 0; bounce < 4 * pp.maxDepth + 8; ++bounce) {
-        if (bounce == nextCheck) {
-            OWEC_CUDA(cudaMemcpyAsync(c.hostCounts, c.dCounts.get(), 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            OWEC_CUDA(cudaStreamSynchronize(s));
-            if (c.hostCounts[cur] == 0) break;
-            nextCheck = bounce + 4;
-        }
-        // the next-bounce queue and the per-bounce queues start empty
-        OWEC_CUDA(cudaMemsetAsync(c.dCounts.get() + (cur ^ 1), 0, sizeof(uint32_t), s));
-        OWEC_CUDA(cudaMemsetAsync(c.dCounts.get() + 2, 0, 5 * sizeof(uint32_t), s));  // + fetch counters, simple queue
-        if (timed && size_t(evUsed + 4) > c.travEvents.size())
-            for (int k = 0; k < 4; ++k) {
-                cudaEvent_t e;
-                OWEC_CUDA(cudaEventCreate(&e));
-                c.travEvents.push_back(e);
+// Bounces the host may be ahead of the last one it knows to have started.
+constexpr uint32_t kBouncesAhead = 5;
+constexpr int maxBounces(int maxDepth) { return 4 * maxDepth + 8; }
+static_assert(kBouncesAhead < uint32_t(kProgressSlots), "a bounce's progress word must not be overwritten before it is read");
+
+// A batch's counters, cleared: one set per bounce it may take, one before them for what starts the batch
+// and one behind the last for its survivors.
+void beginBatch(owec_ctx& c, Queues& q, int maxDepth) {
+    const size_t n = size_t(maxBounces(maxDepth) + 2) * kBounceCounters;
+    c.dCounts.reserve(n);
+    OWEC_CUDA(cudaMemsetAsync(c.dCounts.get(), 0, n * sizeof(uint32_t), c.stream));
+    q.counts = c.dCounts.get();
+}
+
+// The bounces of one batch of nPaths paths already started: bounce(q, grid) queues the kernels of
+// one. The kernels read their queue lengths on the device, and the closest-hit kernel reports to
+// page-locked memory how many paths its bounce started with: the host queues up to kBouncesAhead bounces
+// beyond the last report it has read, gives the grids the blocks that report's paths can fill, and stops
+// at a bounce that started with none. (Queueing maxDepth + 1 bounces of full grids blindly, with three
+// clears and four events each, took three quarters of a small frame at the default depth: 480 x 270,
+// depth 64, 65 bounces where 20 have paths.)
+template <class Bounce>
+void runBounces(owec_ctx& c, Queues q, int maxDepth, uint32_t nPaths, int& bounces, const Bounce& bounce) {
+    uint32_t known = nPaths;
+    const uint32_t first = c.bounces;
+    uint32_t read = 0;  // reports read so far
+    for (uint32_t k = 0; k < uint32_t(maxBounces(maxDepth)); ++k) {
+        while (read < k) {
+            const volatile unsigned long long* word = c.progress->bounce + (first + read) % kProgressSlots;
+            unsigned long long v = *word;
+            if (uint32_t(v >> 32) != first + read + 1) {
+                if (k - read < kBouncesAhead) break;
+                // wait for it; a stream that has failed or finished without it ends the wait
+                for (int spin = 0; uint32_t((v = *word) >> 32) != first + read + 1;) {
+                    if (++spin < 2048) continue;
+                    spin = 0;
+                    const cudaError_t e = cudaStreamQuery(c.stream);
+                    if (e == cudaErrorNotReady) continue;
+                    OWEC_CUDA(e);
+                    v = *word;
+                    if (uint32_t(v >> 32) != first + read + 1) throw Error(OWEC_E_CUDA, "a bounce ended without its report");
+                    break;
+                }
             }
-        if (timed) OWEC_CUDA(cudaEventRecord(c.travEvents[evUsed], s));
-        launchIntersect<M>(c.ds, pb, q, cur, st, c.dCounts.get() + 4, grid, s);
-        ++intersectLaunches;
-        if (c.ds.travCounters && c.launchQueryCount < owec_ctx::kLaunchLog)
-            OWEC_CUDA(cudaMemcpyAsync(c.dLaunchQueries.get() + c.launchQueryCount++, c.ds.travCounters,
-                                      sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s));
-        if (timed) OWEC_CUDA(cudaEventRecord(c.travEvents[evUsed + 1], s));
-        checkLaunch();
-        launchMedium<M>(c.ds, pp, pb, q, cur, st, c.numSMs * OWEC_SHADING_GRID, s);
-        launchSurface<M>(c.ds, pp, pb, q, cur, st, c.numSMs * OWEC_SHADING_GRID, s);
-        if (timed) OWEC_CUDA(cudaEventRecord(c.travEvents[evUsed + 2], s));
-        launchShadow<M>(c.ds, pp, pb, q, st, c.dCounts.get() + 5, c.dShadowVis.get(), grid, s);
-        if (timed) OWEC_CUDA(cudaEventRecord(c.travEvents[evUsed + 3], s));
-        checkLaunch();
-        if (timed) evUsed += 4;
-        OWEC_CUDA(cudaMemsetAsync(c.dCounts.get() + cur, 0, sizeof(uint32_t), s));
-        cur ^= 1;
-        if (timed && evUsed >= 256) {  // fold the timings in before reusing the events
-            OWEC_CUDA(cudaStreamSynchronize(s));
-            for (int e = 0; e < evUsed; e += 2) {
-                float ms = 0;
-                OWEC_CUDA(cudaEventElapsedTime(&ms, c.travEvents[e], c.travEvents[e + 1]));
-                travSeconds[(e >> 1) & 1] += ms * 1e-3;
-            }
-            evUsed = 0;
+            known = uint32_t(v);
+            ++read;
+            if (known == 0) return;
         }
+        q.progress = c.progress->bounce + c.bounces % kProgressSlots;
+        q.bounce = ++c.bounces;
+        const int grid = int(std::min<uint32_t>(uint32_t(c.numSMs) * OWEC_SHADING_GRID, (known + 127) / 128));
+        bounce(q, std::max(1, grid));
+        ++bounces;
+        checkLaunch();
+        q.counts += kBounceCounters;
+        std::swap(q.active[0], q.active[1]);
     }
+}
+
+// The shadow kernels of a bounce run beside the next bounce's closest-hit kernel: neither reads what the
+// other writes (radiance and connections; hits), and each leaves the GPU to its last long rays for a
+// quarter of its time (kIntersect's SMs were active for 73 % of it). shadowsBegin: on the shadow stream
+// from here, after the events queued so far; shadowsEnd: the pass's stream waits for them.
+template <class Launch>
+void queueShadows(owec_ctx& c, const Launch& launch) {
+    OWEC_CUDA(cudaEventRecord(c.eventsDone, c.stream));
+    OWEC_CUDA(cudaStreamWaitEvent(c.shadowStream, c.eventsDone, 0));
+    launch(c.shadowStream);
+    OWEC_CUDA(cudaEventRecord(c.shadowDone, c.shadowStream));
+}
+void joinShadows(owec_ctx& c) { OWEC_CUDA(cudaStreamWaitEvent(c.stream, c.shadowDone, 0)); }
+
+// A bounce of the camera paths.
+template <int M>
+void queueBounce(owec_ctx& c, const PassParams& pp, const PathBuffers<ModeR<M>>& pb, const Queues& q, int grid, StatCounters* st) {
+    cudaStream_t s = c.stream;
+    launchIntersect<M>(c.ds, pb, q, st, grid, s);
+    if (c.ds.travCounters && c.launchQueryCount < owec_ctx::kLaunchLog)
+        OWEC_CUDA(cudaMemcpyAsync(c.dLaunchQueries.get() + c.launchQueryCount++, c.ds.travCounters,
+                                  sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s));
+    joinShadows(c);  // the last bounce's: the events below read and write the radiance they add to
+    launchMedium<M>(c.ds, pp, pb, q, st, grid, s);
+    launchSurface<M>(c.ds, pp, pb, q, st, grid, s);
+    queueShadows(c, [&](cudaStream_t ss) { launchShadow<M>(c.ds, pp, pb, q, st, c.dShadowVis.get(), grid, ss); });
+}
+
+// Around a pass: its clock, and its times once it is done (owec_last_pass_timing).
+void beginPass(owec_ctx& c, Queues& q) {
+    q.clock = c.dClock.get();
+    OWEC_CUDA(cudaMemsetAsync(q.clock, 0, sizeof(BounceClock), c.stream));
+    OWEC_CUDA(cudaEventRecord(c.passStart, c.stream));
+}
+void endPass(owec_ctx& c, int bounces) {
+    OWEC_CUDA(cudaEventRecord(c.passStop, c.stream));
+    OWEC_CUDA(cudaMemcpyAsync(&c.progress->clock, c.dClock.get(), sizeof(BounceClock), cudaMemcpyDeviceToHost, c.stream));
+    OWEC_CUDA(cudaStreamSynchronize(c.stream));
+    float ms = 0;
+    OWEC_CUDA(cudaEventElapsedTime(&ms, c.passStart, c.passStop));
+    c.lastPassSeconds = ms * 1e-3;
+    c.lastIntersectSeconds = double(c.progress->clock.intersect) * 1e-9;
+    c.lastShadowSeconds = double(c.progress->clock.shadow) * 1e-9;
+    c.lastIntersectLaunches = bounces;
 }
 
 template <int M>
@@ -1279,37 +1341,24 @@ void runPass(owec_ctx& c, int spp) {
     pp.fresnelFloor = float(std::min(0.49, std::max(0.0, c.settings.fresnel_floor)));
     pp.nPixels = nPix;
     pp.anyHitShadows = c.hasNull ? 0 : 1;
-    const int grid = c.numSMs * 8;
     cudaStream_t s = c.stream;
-    double travSeconds[2] = {0, 0};
-    int intersectLaunches = 0;
-    OWEC_CUDA(cudaEventRecord(c.passStart, s));
-    int evUsed = 0;
+    int bounces = 0;
+    beginPass(c, q);
     for (int done = 0; done < spp;) {
         const uint32_t S = std::min<uint32_t>(perBatch, uint32_t(spp - done));
         pp.nPaths = S * nPix;
         pp.streamBase = uint32_t(c.passCount + done);
-        OWEC_CUDA(cudaMemsetAsync(c.dCounts.get(), 0, 8 * sizeof(uint32_t), s));
+        beginBatch(c, q, pp.maxDepth);
         launchGenerate<M>(c.ds, pp, pb, q, c.dStats.get(), s);
         checkLaunch();
-        runBounces<M>(c, pp, pb, q, c.dStats.get(), grid, true, travSeconds, evUsed, intersectLaunches);
+        runBounces(c, q, pp.maxDepth, pp.nPaths, bounces,
+                   [&](const Queues& bq, int grid) { queueBounce<M>(c, pp, pb, bq, grid, c.dStats.get()); });
+        joinShadows(c);
         launchFilm<M>(c.ds, pp, pb, c.dFilm.get(), c.dComp.get(), c.dSamples.get(), S, s);
         checkLaunch();
         done += int(S);
     }
-    OWEC_CUDA(cudaEventRecord(c.passStop, s));
-    OWEC_CUDA(cudaEventSynchronize(c.passStop));
-    for (int e = 0; e < evUsed; e += 2) {
-        float ms = 0;
-        OWEC_CUDA(cudaEventElapsedTime(&ms, c.travEvents[e], c.travEvents[e + 1]));
-        travSeconds[(e >> 1) & 1] += ms * 1e-3;  // pairs alternate: intersect, shadow
-    }
-    float passMs = 0;
-    OWEC_CUDA(cudaEventElapsedTime(&passMs, c.passStart, c.passStop));
-    c.lastPassSeconds = passMs * 1e-3;
-    c.lastIntersectSeconds = travSeconds[0];
-    c.lastShadowSeconds = travSeconds[1];
-    c.lastIntersectLaunches = intersectLaunches;
+    endPass(c, bounces);
     c.passCount += uint64_t(spp);
 }
 
@@ -1342,76 +1391,37 @@ void runParticles(owec_ctx& c, int spp) {
                                                      : (2 * det.halfX / det.width) * (2 * det.halfY / det.height);
     PassParams pp{};
     pp.anyHitShadows = c.hasNull ? 0 : 1;
-    const int grid = c.numSMs * 8;
     cudaStream_t s = c.stream;
-    uint32_t* counts = c.dCounts.get();
-    double travSeconds[2] = {0, 0};
-    int intersectLaunches = 0, evUsed = 0;
-    OWEC_CUDA(cudaEventRecord(c.passStart, s));
+    int bounces = 0;
+    beginPass(c, q);
     // nothing emits: the estimate is zero, but the particles still count
     const bool emits = c.pSky > 0 || !c.lights.empty();
     for (uint64_t first = 0; emits && first < total; first += cap) {
         const uint32_t n = uint32_t(std::min<uint64_t>(cap, total - first));
         P.first = first;
-        OWEC_CUDA(cudaMemsetAsync(counts, 0, 8 * sizeof(uint32_t), s));
+        beginBatch(c, q, P.maxDepth);
         launchEmit<M>(c.ds, P, pb, q, c.dStats.get(), film, n, s);
-        launchConnect<M>(c.ds, pp, pb, q, c.dStats.get(), counts + 5, c.dShadowVis.get(), film, grid, s);
+        // the emitters' own connections; the particles they start are the first bounce's
+        const int grid = int(std::min<uint32_t>(uint32_t(c.numSMs) * OWEC_SHADING_GRID, (n + 127) / 128));
+        queueShadows(c, [&](cudaStream_t ss) {
+            launchConnect<M>(c.ds, pp, pb, q, c.dStats.get(), c.dShadowVis.get(), film, grid, ss);
+        });
         checkLaunch();
-        int cur = 0;
-        // as the camera paths: bounces queued without a host wait, the queue looked at once the
-        // depth cap is reached and every four bounces after it
-        int nextCheck = P.maxDepth + 1;
-        for (int bounce = 0; bounce < 4 * P.maxDepth + 8; ++bounce) {
-            if (bounce == nextCheck) {
-                OWEC_CUDA(cudaMemcpyAsync(c.hostCounts, counts, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-                OWEC_CUDA(cudaStreamSynchronize(s));
-                if (c.hostCounts[cur] == 0) break;
-                nextCheck = bounce + 4;
-            }
-            OWEC_CUDA(cudaMemsetAsync(counts + (cur ^ 1), 0, sizeof(uint32_t), s));
-            OWEC_CUDA(cudaMemsetAsync(counts + 2, 0, 5 * sizeof(uint32_t), s));  // shadow queue, fetch counters
-            if (size_t(evUsed + 4) > c.travEvents.size())
-                for (int k = 0; k < 4; ++k) {
-                    cudaEvent_t e;
-                    OWEC_CUDA(cudaEventCreate(&e));
-                    c.travEvents.push_back(e);
-                }
-            OWEC_CUDA(cudaEventRecord(c.travEvents[evUsed], s));
-            launchIntersect<M>(c.ds, pb, q, cur, c.dStats.get(), counts + 4, grid, s);
-            ++intersectLaunches;
-            OWEC_CUDA(cudaEventRecord(c.travEvents[evUsed + 1], s));
-            launchParticleEvent<M>(c.ds, P, pb, q, cur, c.dStats.get(), film, grid, s);
-            OWEC_CUDA(cudaEventRecord(c.travEvents[evUsed + 2], s));
-            launchConnect<M>(c.ds, pp, pb, q, c.dStats.get(), counts + 5, c.dShadowVis.get(), film, grid, s);
-            OWEC_CUDA(cudaEventRecord(c.travEvents[evUsed + 3], s));
-            checkLaunch();
-            evUsed += 4;
-            OWEC_CUDA(cudaMemsetAsync(counts + cur, 0, sizeof(uint32_t), s));
-            cur ^= 1;
-            if (evUsed >= 256) {  // fold the timings in before reusing the events
-                OWEC_CUDA(cudaStreamSynchronize(s));
-                for (int e = 0; e < evUsed; e += 2) {
-                    float ms = 0;
-                    OWEC_CUDA(cudaEventElapsedTime(&ms, c.travEvents[e], c.travEvents[e + 1]));
-                    travSeconds[(e >> 1) & 1] += ms * 1e-3;
-                }
-                evUsed = 0;
-            }
-        }
+        Queues bounceQueues = q;
+        bounceQueues.counts += kBounceCounters;
+        std::swap(bounceQueues.active[0], bounceQueues.active[1]);
+        runBounces(c, bounceQueues, P.maxDepth, n, bounces, [&](const Queues& bq, int g) {
+            launchIntersect<M>(c.ds, pb, bq, c.dStats.get(), g, s);
+            joinShadows(c);
+            launchParticleEvent<M>(c.ds, P, pb, bq, c.dStats.get(), film, g, s);
+            queueShadows(c, [&](cudaStream_t ss) {
+                launchConnect<M>(c.ds, pp, pb, bq, c.dStats.get(), c.dShadowVis.get(), film, g, ss);
+            });
+        });
+        joinShadows(c);
+        checkLaunch();
     }
-    OWEC_CUDA(cudaEventRecord(c.passStop, s));
-    OWEC_CUDA(cudaEventSynchronize(c.passStop));
-    for (int e = 0; e < evUsed; e += 2) {
-        float ms = 0;
-        OWEC_CUDA(cudaEventElapsedTime(&ms, c.travEvents[e], c.travEvents[e + 1]));
-        travSeconds[(e >> 1) & 1] += ms * 1e-3;  // pairs alternate: intersect, connections
-    }
-    float ms = 0;
-    OWEC_CUDA(cudaEventElapsedTime(&ms, c.passStart, c.passStop));
-    c.lastPassSeconds = ms * 1e-3;
-    c.lastIntersectSeconds = travSeconds[0];
-    c.lastShadowSeconds = travSeconds[1];
-    c.lastIntersectLaunches = intersectLaunches;
+    endPass(c, bounces);
     c.particles += double(total);
     c.passCount += uint64_t(spp);
 }
@@ -1446,8 +1456,7 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
     pp.ckptCount = ckptCount.get();
     pp.ckpt = ckpt.get();
     const int grid = c.numSMs * 8;
-    double unusedSeconds[2] = {0, 0};
-    int unusedEvents = 0, unusedLaunches = 0;
+    int unusedBounces = 0;
     cudaEvent_t replayStart, replayStop;
     OWEC_CUDA(cudaEventCreate(&replayStart));
     OWEC_CUDA(cudaEventCreate(&replayStop));
@@ -1455,11 +1464,13 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
         const uint32_t S = std::min<uint32_t>(perBatch, uint32_t(spp - done));
         pp.nPaths = S * nPix;
         pp.streamBase = uint32_t(firstPass + uint64_t(done));
-        OWEC_CUDA(cudaMemsetAsync(c.dCounts.get(), 0, 8 * sizeof(uint32_t), c.stream));
+        beginBatch(c, q, pp.maxDepth);
         OWEC_CUDA(cudaMemsetAsync(ckptCount.get(), 0, sizeof(uint32_t), c.stream));
         launchGenerate<M>(c.ds, pp, pb, q, st.get(), c.stream);
         checkLaunch();
-        runBounces<M>(c, pp, pb, q, st.get(), grid, false, unusedSeconds, unusedEvents, unusedLaunches);
+        runBounces(c, q, pp.maxDepth, pp.nPaths, unusedBounces,
+                   [&](const Queues& bq, int g) { queueBounce<M>(c, pp, pb, bq, g, st.get()); });
+        joinShadows(c);
         OWEC_CUDA(cudaEventRecord(replayStart, c.stream));
         launchPathAdjoint(M, c.ds, pp, c.hf, t, fixedDecisions, ckpt.get(), ckptCount.get(), grid, c.stream);
         checkLaunch();
@@ -1627,11 +1638,16 @@ int owec_open(int device, owec_ctx** out) {
         c->numSMs = prop.multiProcessorCount;
         std::snprintf(c->name, sizeof(c->name), "%s", prop.name);
         OWEC_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+        OWEC_CUDA(cudaStreamCreateWithFlags(&c->shadowStream, cudaStreamNonBlocking));
+        OWEC_CUDA(cudaEventCreateWithFlags(&c->eventsDone, cudaEventDisableTiming));
+        OWEC_CUDA(cudaEventCreateWithFlags(&c->shadowDone, cudaEventDisableTiming));
         OWEC_CUDA(cudaEventCreate(&c->passStart));
         OWEC_CUDA(cudaEventCreate(&c->passStop));
         OWEC_CUDA(cudaMallocHost(&c->hostBlock, kHostBlock));
-        c->hostCounts = reinterpret_cast<uint32_t*>(c->hostBlock);
-        c->dCounts.resize(8);
+        c->progress = reinterpret_cast<owec_ctx::HostProgress*>(c->hostBlock);
+        static_assert(sizeof(owec_ctx::HostProgress) <= kHostReports, "the reports fit their part of the block");
+        std::memset(c->progress, 0, sizeof(owec_ctx::HostProgress));
+        c->dClock.resize(1);
         c->dStats.resize(1);
         c->dScene.resize(1);
         OWEC_CUDA(cudaMemsetAsync(c->dStats.get(), 0, sizeof(StatCounters), c->stream));
@@ -1650,7 +1666,10 @@ int owec_close(owec_ctx* ctx) {
             for (int k = 0; k < 2; ++k) cudaEventDestroy(ctx->resolvedEv[k]);
             cudaStreamDestroy(ctx->copyStream);
         }
-        for (cudaEvent_t e : ctx->travEvents) cudaEventDestroy(e);
+        cudaStreamSynchronize(ctx->shadowStream);
+        cudaEventDestroy(ctx->eventsDone);
+        cudaEventDestroy(ctx->shadowDone);
+        cudaStreamDestroy(ctx->shadowStream);
         cudaEventDestroy(ctx->passStart);
         cudaEventDestroy(ctx->passStop);
         cudaFreeHost(ctx->hostBlock);

@@ -122,7 +122,7 @@ __device__ void queueConnection(const DeviceScene& sc, PathBuffers<RT<M>>& pb, Q
     if (mask == 0) return;
     const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
     uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(&q.counts[3], uint32_t(__popc(mask)));
+    if (lane == leader) base = atomicAdd(&q.counts[kCountShadow], uint32_t(__popc(mask)));
     base = __shfl_sync(active, base, leader);
     if (!push) return;
     const uint32_t slot = base + __popc(mask & ((1u << lane) - 1u));
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(128) kEmit(DeviceScene sc, ParticleParams P, P
     pb.aux[i] = aux;
     queueConnection<M>(sc, pb, q, film, i, sp.pdf, value, k, cp, cRegion, cB, 0u, cErr, connect);
     warpCount(&st->paths, true);
-    warpPush(q.active[0], &q.counts[0], live, i);
+    warpPush(q.active[1], &q.counts[kCountNext], live, i);
 }
 
 // ------------------------------------------------------------------ one event of every particle
@@ -323,16 +323,15 @@ __global__ void __launch_bounds__(128) kEmit(DeviceScene sc, ParticleParams P, P
 // the other lobes fold away, and with them the registers they hold.
 template <int M, bool Full, bool Lean>
 __global__ void __launch_bounds__(128, Lean ? 4 : 3) kParticleEvent(DeviceScene sc, ParticleParams P, PathBuffers<RT<M>> pb,
-                                                                   Queues q, int cur, StatCounters* st, SplatTarget film) {
+                                                                   Queues q, StatCounters* st, SplatTarget film) {
     using R = RT<M>;
     using Ro = typename Mode<M>::Ro;
     using Rr = typename Mode<M>::Rr;
-    const int nxt = cur ^ 1;
-    const uint32_t n = q.counts[cur];
+    const uint32_t n = q.counts[kCountActive];
     const DDetector& det = sc.det;
     const bool observer = det.kind == OWEC_DETECTOR_OBSERVER;
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const uint32_t i = q.active[cur][e];
+        const uint32_t i = q.active[0][e];
         const HitRec h = loadStream(pb.hit + i);
         PathRay<R> ray = loadStream(pb.ray + i);
         PathSpec<R> sp = loadStream(pb.spec + i);
@@ -525,7 +524,7 @@ __global__ void __launch_bounds__(128, Lean ? 4 : 3) kParticleEvent(DeviceScene 
         warpCount(&st->leaks, leak);
         warpCount(&st->inconsistencies, inconsistent);
         warpCount(&st->faults, lost);
-        warpPush(q.active[nxt], &q.counts[nxt], cont, i);
+        warpPush(q.active[1], &q.counts[kCountNext], cont, i);
     }
 }
 
@@ -549,10 +548,10 @@ void launchEmit(const DeviceScene& sc, const ParticleParams& P, const PathBuffer
 }
 template <int M>
 void launchParticleEvent(const DeviceScene& sc, const ParticleParams& P, const PathBuffers<ModeR<M>>& pb,
-                         const Queues& q, int cur, StatCounters* st, const SplatTarget& film, int grid, cudaStream_t s) {
-    if (sc.fullFeatures) kParticleEvent<M, true, false><<<grid, 128, 0, s>>>(sc, P, pb, q, cur, st, film);
-    else if (sc.simpleOptics) kParticleEvent<M, false, true><<<grid, 128, 0, s>>>(sc, P, pb, q, cur, st, film);
-    else kParticleEvent<M, false, false><<<grid, 128, 0, s>>>(sc, P, pb, q, cur, st, film);
+                         const Queues& q, StatCounters* st, const SplatTarget& film, int grid, cudaStream_t s) {
+    if (sc.fullFeatures) kParticleEvent<M, true, false><<<grid, 128, 0, s>>>(sc, P, pb, q, st, film);
+    else if (sc.simpleOptics) kParticleEvent<M, false, true><<<grid, 128, 0, s>>>(sc, P, pb, q, st, film);
+    else kParticleEvent<M, false, false><<<grid, 128, 0, s>>>(sc, P, pb, q, st, film);
 }
 void launchResolveSplats(const unsigned long long* splat, uint32_t nPixels, double scale, double* xyz, cudaStream_t s) {
     kResolveSplats<<<(3 * nPixels + 255) / 256, 256, 0, s>>>(splat, nPixels, scale, xyz);
@@ -562,7 +561,7 @@ void launchResolveSplats(const unsigned long long* splat, uint32_t nPixels, doub
     template void launchEmit<M>(const DeviceScene&, const ParticleParams&, const PathBuffers<ModeR<M>>&,          \
                                 const Queues&, StatCounters*, const SplatTarget&, uint32_t, cudaStream_t);         \
     template void launchParticleEvent<M>(const DeviceScene&, const ParticleParams&, const PathBuffers<ModeR<M>>&, \
-                                         const Queues&, int, StatCounters*, const SplatTarget&, int, cudaStream_t);
+                                         const Queues&, StatCounters*, const SplatTarget&, int, cudaStream_t);
 
 OWEC_INSTANTIATE_PARTICLES(0)
 OWEC_INSTANTIATE_PARTICLES(1)

@@ -25,16 +25,16 @@ struct ParticleParams {
                             // sensor: a pixel's area on the sensor
 };
 
-// Starts n particles (P.first onward) in path slots 0..n-1: active queue 0, and the emitters' own
-// connections in the shadow queue.
+// Starts n particles (P.first onward) in path slots 0..n-1: in the next bounce's queue, and the emitters'
+// own connections in the shadow queue.
 template <int M>
 void launchEmit(const DeviceScene&, const ParticleParams&, const PathBuffers<ModeR<M>>&, const Queues&, StatCounters*,
                 const SplatTarget&, uint32_t n, cudaStream_t);
-// One event of every particle in active queue `cur` (after its closest-hit query): survivors go to
-// the other active queue, connections to the shadow queue, sensor records to the film.
+// One event of every particle in this bounce's active queue (after its closest-hit query): survivors go to
+// the next bounce's queue, connections to the shadow queue, sensor records to the film.
 template <int M>
 void launchParticleEvent(const DeviceScene&, const ParticleParams&, const PathBuffers<ModeR<M>>&, const Queues&,
-                         int cur, StatCounters*, const SplatTarget&, int grid, cudaStream_t);
+                         StatCounters*, const SplatTarget&, int grid, cudaStream_t);
 
 // XYZ per pixel from the splat sums: sum * 2^kSplatExp0 * scale.
 void launchResolveSplats(const unsigned long long* splat, uint32_t nPixels, double scale, double* xyz, cudaStream_t s);

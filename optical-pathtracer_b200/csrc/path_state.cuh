@@ -125,14 +125,53 @@ struct alignas(16) ShadowRay {
 };
 static_assert(sizeof(ShadowRay<float>) == 96, "a mixed-precision shadow record stays six 16-byte words");
 
+// Device time of a pass's closest-hit and shadow kernels (owec_last_pass_timing), in nanoseconds of the
+// global timer, from a kernel's first thread to its last warp. The two kinds overlap: a bounce's shadow
+// kernels run beside the next bounce's closest-hit kernel.
+struct BounceClock {
+    unsigned long long intersectStart, intersect, shadowStart, shadow;
+};
+
+// Counters of one bounce; every bounce of a batch has its own set, all cleared at once before it.
+constexpr int kCountActive = 0, kWarpsIntersect = 1, kCountSurface = 2, kCountShadow = 3, kFetchIntersect = 4, kFetchShadow = 5,
+              kCountSimple = 6, kWarpsShadow = 7, kBounceCounters = 8, kCountNext = kBounceCounters + kCountActive;
+// The paths a bounce started with, as the closest-hit kernel reports them to the host (Queues::progress):
+// the bounce's number in the upper half, so that a stale word is never taken for it.
+constexpr int kProgressSlots = 64;
+
 struct Queues {
-    uint32_t* active[2];
+    uint32_t* active[2];      // this bounce's paths and the next one's
     uint32_t* surface;        // surface events with any optics
     uint32_t* shadow;
-    uint32_t* counts;         // [0], [1] active ping-pong, [2] surface, [3] shadow, [4], [5] fetch
-                              // counters of the persistent kernels, [6] simple surface
+    uint32_t* counts;         // this bounce's counters, the next bounce's behind them
     uint32_t* surfaceSimple;  // surface events on Lambertian, absorbing and detecting boundaries
+    BounceClock* clock;       // null: not timed
+    unsigned long long* progress;  // this bounce's word in page-locked host memory
+    uint32_t bounce;          // this bounce's number, counted on from pass to pass
 };
+
+#if defined(__CUDACC__)
+__device__ __forceinline__ unsigned long long globalTimer() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// The first thread of a bounce's closest-hit kernel, and of its first shadow kernel.
+__device__ __forceinline__ void stampIntersect(const Queues& q) {
+    *reinterpret_cast<volatile unsigned long long*>(q.progress) = (uint64_t(q.bounce) << 32) | q.counts[kCountActive];
+    if (q.clock) q.clock->intersectStart = globalTimer();
+}
+__device__ __forceinline__ void stampShadow(const Queues& q) {
+    if (q.clock) q.clock->shadowStart = globalTimer();
+}
+// One lane of each warp of a kernel at its end, counted in warps: the last one adds the time since start.
+__device__ __forceinline__ void stampEnd(uint32_t* warps, const unsigned long long& start, unsigned long long& sum) {
+    if (atomicAdd(warps, 1u) + 1 != gridDim.x * (blockDim.x >> 5)) return;
+    __threadfence();
+    sum += globalTimer() - *const_cast<const volatile unsigned long long*>(&start);
+}
+__device__ __forceinline__ bool firstThread() { return blockIdx.x == 0 && threadIdx.x == 0; }
+#endif
 
 struct StatCounters {
     unsigned long long paths, segments, inconsistencies, leaks, shadowRays, faults;

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(256) kGenerate(DeviceScene sc, PassParams pp, 
     pb.spec[i] = sp;
     pb.aux[i] = aux;
     warpCount(&st->paths, live);
-    warpPush(q.active[0], &q.counts[0], live, i);
+    warpPush(q.active[0], &q.counts[kCountActive], live, i);
 }
 
 // ------------------------------------------------------------------ intersect
@@ -110,20 +110,21 @@ __device__ __forceinline__ void warpFlush(unsigned long long* counter, uint32_t 
 // visits at a time and, when it ends, takes the next query of the queue, so that lanes whose rays
 // finish early do not idle until the warp's longest ray is done.
 template <int M, bool Count, bool Full>
-__global__ void OWEC_TRAVERSAL_BOUNDS kIntersect(DeviceScene sc, PathBuffers<RT<M>> pb, Queues q, int cur,
+__global__ void OWEC_TRAVERSAL_BOUNDS kIntersect(DeviceScene sc, PathBuffers<RT<M>> pb, Queues q,
                                                   StatCounters* st, uint32_t* fetch) {
     using R = RT<M>;
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
     ColdRay<R>* cold = coldRay<R>(stackMem);
-    const uint32_t n = q.counts[cur];
+    if (firstThread()) stampIntersect(q);
+    const uint32_t n = q.counts[kCountActive];
     Traversal<R, typename Mode<M>::Ro, typename Mode<M>::Rr, false, SharedStack, Count, Full> tr;
     uint32_t path = 0, segments = 0, faults = 0;
     bool alive = false, exhausted = false;
     for (;;) {
         const uint32_t k = refillLanes(!alive, fetch, n, exhausted);
         if (!alive && k < n) {
-            path = q.active[cur][k];
+            path = q.active[0][k];
             const PathRay<R> ray = loadStream(pb.ray + path);
             RayQuery<R> rq;
             rq.od = rayOrigin(ray.o);
@@ -164,6 +165,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kIntersect(DeviceScene sc, PathBuffers<RT<
     }
     warpFlush(&st->segments, segments);
     warpFlush(&st->faults, faults);
+    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kWarpsIntersect, q.clock->intersectStart, q.clock->intersect);
 }
 
 // ------------------------------------------------------------------ next-event estimation
@@ -195,7 +197,7 @@ __device__ void queueNee(const DeviceScene& sc, PathBuffers<RT<M>>& pb, Queues& 
     if (mask == 0) return;
     const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
     uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(&q.counts[3], uint32_t(__popc(mask)));
+    if (lane == leader) base = atomicAdd(&q.counts[kCountShadow], uint32_t(__popc(mask)));
     base = __shfl_sync(active, base, leader);
     if (!push) return;
     const uint32_t slot = base + __popc(mask & ((1u << lane) - 1u));
@@ -227,13 +229,11 @@ __device__ __forceinline__ void checkpointPath(const PassParams& pp, const PathR
 }
 
 template <int M>
-__global__ void __launch_bounds__(128, OWEC_SHADING_MIN_BLOCKS) kMedium(DeviceScene sc, PassParams pp, PathBuffers<RT<M>> pb, Queues q,
-                                               int cur, StatCounters* st) {
+__global__ void __launch_bounds__(128, OWEC_SHADING_MIN_BLOCKS) kMedium(DeviceScene sc, PassParams pp, PathBuffers<RT<M>> pb, Queues q, StatCounters* st) {
     using R = RT<M>;
-    const int nxt = cur ^ 1;
-    const uint32_t n = q.counts[cur];
+    const uint32_t n = q.counts[kCountActive];
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t i = q.active[cur][k];
+        const uint32_t i = q.active[0][k];
         const HitRec h = loadStream(pb.hit + i);
         {
             // A segment through a region without absorption or scattering that met a boundary has
@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(128, OWEC_SHADING_MIN_BLOCKS) kMedium(DeviceSc
                 }
                 const int32_t ot = sc.optics[sc.boundaries[h.boundary].optics].type;
                 const bool simple = ot == OWEC_SURF_DIFFUSE || ot == OWEC_SURF_ABSORBER || ot == OWEC_SURF_DETECTOR;
-                warpPush(q.surface, &q.counts[2], !simple, i);
-                warpPush(q.surfaceSimple, &q.counts[6], simple, i);
+                warpPush(q.surface, &q.counts[kCountSurface], !simple, i);
+                warpPush(q.surfaceSimple, &q.counts[kCountSimple], simple, i);
                 continue;
             }
         }
@@ -366,9 +366,9 @@ __global__ void __launch_bounds__(128, OWEC_SHADING_MIN_BLOCKS) kMedium(DeviceSc
             const int32_t ot = sc.optics[sc.boundaries[h.boundary].optics].type;
             simple = ot == OWEC_SURF_DIFFUSE || ot == OWEC_SURF_ABSORBER || ot == OWEC_SURF_DETECTOR;
         }
-        warpPush(q.surface, &q.counts[2], toSurface && !simple, i);
-        warpPush(q.surfaceSimple, &q.counts[6], toSurface && simple, i);
-        warpPush(q.active[nxt], &q.counts[nxt], cont, i);
+        warpPush(q.surface, &q.counts[kCountSurface], toSurface && !simple, i);
+        warpPush(q.surfaceSimple, &q.counts[kCountSimple], toSurface && simple, i);
+        warpPush(q.active[1], &q.counts[kCountNext], cont, i);
     }
 }
 
@@ -394,13 +394,11 @@ __device__ __noinline__ void logInconsistency(const DeviceScene& sc, const PathR
 }
 
 template <int M, bool Simple, bool Full>
-__global__ void __launch_bounds__(128, Simple ? OWEC_SIMPLE_MIN_BLOCKS : OWEC_SHADING_MIN_BLOCKS) kSurface(DeviceScene sc, PassParams pp, PathBuffers<RT<M>> pb, Queues q,
-                                                int cur, StatCounters* st) {
+__global__ void __launch_bounds__(128, Simple ? OWEC_SIMPLE_MIN_BLOCKS : OWEC_SHADING_MIN_BLOCKS) kSurface(DeviceScene sc, PassParams pp, PathBuffers<RT<M>> pb, Queues q, StatCounters* st) {
     using R = RT<M>;
     using Ro = typename Mode<M>::Ro;
     using Rr = typename Mode<M>::Rr;
-    const int nxt = cur ^ 1;
-    const uint32_t n = Simple ? q.counts[6] : q.counts[2];
+    const uint32_t n = Simple ? q.counts[kCountSimple] : q.counts[kCountSurface];
     const uint32_t* queue = Simple ? q.surfaceSimple : q.surface;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const uint32_t i = queue[k];
@@ -544,7 +542,7 @@ __global__ void __launch_bounds__(128, Simple ? OWEC_SIMPLE_MIN_BLOCKS : OWEC_SH
         storeStream(pb.aux + i, aux);
         queueNee<M>(sc, pb, q, i, sp, betaNee, ls, fN, pdfS, cosF, g.p, neeRegion, h.boundary, h.prim, errN, neeValid);
         warpCount(&st->inconsistencies, inconsistent);
-        warpPush(q.active[nxt], &q.counts[nxt], cont, i);
+        warpPush(q.active[1], &q.counts[kCountNext], cont, i);
     }
 }
 
@@ -575,7 +573,8 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadow(DeviceScene sc, PassParams pp, Pat
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
     ColdRay<R>* cold = coldRay<R>(stackMem);
-    const uint32_t n = q.counts[3];
+    if (firstThread()) stampShadow(q);
+    const uint32_t n = q.counts[kCountShadow];
     Traversal<R, Ro, Rr, AnyHit, SharedStack, Count, Full> tr;
     // the light point's identity decides (the Full instantiation's next-event rays)
     constexpr bool kEndpoint = Full && !Splat && !AnyHit;
@@ -715,6 +714,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadow(DeviceScene sc, PassParams pp, Pat
     }
     warpFlush(&st->shadowRays, rays);
     warpFlush(&st->faults, faults);
+    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kWarpsShadow, q.clock->shadowStart, q.clock->shadow);
 }
 
 // Without null boundaries a shadow ray is one any-hit query, and its bookkeeping (the medium's
@@ -731,7 +731,8 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadowVis(DeviceScene sc, PathBuffers<RT<
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
     ColdRay<R>* cold = coldRay<R>(stackMem);
-    const uint32_t n = q.counts[3];
+    if (firstThread()) stampShadow(q);
+    const uint32_t n = q.counts[kCountShadow];
     Traversal<R, Ro, Rr, true, SharedStack, Count, Full> tr;
     uint32_t job = 0;
     bool alive = false, exhausted = false;
@@ -783,7 +784,7 @@ template <int M, bool Splat = false>
 __global__ void __launch_bounds__(256) kShadowApply(DeviceScene sc, PathBuffers<RT<M>> pb, Queues q, const uint8_t* vis,
                                                     StatCounters* st, SplatTarget film) {
     using R = RT<M>;
-    const uint32_t n = q.counts[3];
+    const uint32_t n = q.counts[kCountShadow];
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         uint8_t v = vis[k];
         bool clear = v == 1;
@@ -817,6 +818,7 @@ __global__ void __launch_bounds__(256) kShadowApply(DeviceScene sc, PathBuffers<
         warpCount(&st->shadowRays, true);
         warpCount(&st->faults, v == 2);
     }
+    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kWarpsShadow, q.clock->shadowStart, q.clock->shadow);
 }
 
 // ------------------------------------------------------------------ film
@@ -1017,31 +1019,34 @@ void launchGenerate(const DeviceScene& sc, const PassParams& pp, const PathBuffe
     kGenerate<M><<<(pp.nPaths + 255) / 256, 256, 0, s>>>(sc, pp, pb, q, st);
 }
 template <int M>
-void launchIntersect(const DeviceScene& sc, const PathBuffers<RT<M>>& pb, const Queues& q, int cur, StatCounters* st,
-                     uint32_t* fetch, int grid, cudaStream_t s) {
+void launchIntersect(const DeviceScene& sc, const PathBuffers<RT<M>>& pb, const Queues& q, StatCounters* st,
+                     int grid, cudaStream_t s) {
+    uint32_t* fetch = q.counts + kFetchIntersect;
     const size_t smem = persistentSharedBytes<M>(128);
     if (sc.fullFeatures) {
-        if (sc.travCounters) kIntersect<M, true, true><<<grid, 128, smem, s>>>(sc, pb, q, cur, st, fetch);
-        else kIntersect<M, false, true><<<grid, 128, smem, s>>>(sc, pb, q, cur, st, fetch);
+        if (sc.travCounters) kIntersect<M, true, true><<<grid, 128, smem, s>>>(sc, pb, q, st, fetch);
+        else kIntersect<M, false, true><<<grid, 128, smem, s>>>(sc, pb, q, st, fetch);
     } else {
-        if (sc.travCounters) kIntersect<M, true, false><<<grid, 128, smem, s>>>(sc, pb, q, cur, st, fetch);
-        else kIntersect<M, false, false><<<grid, 128, smem, s>>>(sc, pb, q, cur, st, fetch);
+        if (sc.travCounters) kIntersect<M, true, false><<<grid, 128, smem, s>>>(sc, pb, q, st, fetch);
+        else kIntersect<M, false, false><<<grid, 128, smem, s>>>(sc, pb, q, st, fetch);
     }
 }
 template <int M>
-void launchMedium(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q, int cur,
+void launchMedium(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
                   StatCounters* st, int grid, cudaStream_t s) {
-    kMedium<M><<<grid, 128, 0, s>>>(sc, pp, pb, q, cur, st);
+    kMedium<M><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
 }
 template <int M>
-void launchSurface(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q, int cur,
+void launchSurface(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
                    StatCounters* st, int grid, cudaStream_t s) {
+    // a scene whose boundaries are all Lambertian, absorbing or detecting (or none of them) fills one of
+    // the two surface queues only
     if (sc.fullFeatures) {
-        kSurface<M, true, true><<<grid, 128, 0, s>>>(sc, pp, pb, q, cur, st);
-        kSurface<M, false, true><<<grid, 128, 0, s>>>(sc, pp, pb, q, cur, st);
+        if (sc.opticsUsed & kOpticsSimple) kSurface<M, true, true><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
+        if (sc.opticsUsed & kOpticsGeneral) kSurface<M, false, true><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
     } else {
-        kSurface<M, true, false><<<grid, 128, 0, s>>>(sc, pp, pb, q, cur, st);
-        kSurface<M, false, false><<<grid, 128, 0, s>>>(sc, pp, pb, q, cur, st);
+        if (sc.opticsUsed & kOpticsSimple) kSurface<M, true, false><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
+        if (sc.opticsUsed & kOpticsGeneral) kSurface<M, false, false><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
     }
 }
 // The shadow-ray kernels of a bounce: visibility then contributions without null boundaries, the
@@ -1073,13 +1078,13 @@ void shadowKernels(const DeviceScene& sc, const PassParams& pp, const PathBuffer
 
 template <int M>
 void launchShadow(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
-                  StatCounters* st, uint32_t* fetch, uint8_t* vis, int grid, cudaStream_t s) {
-    shadowKernels<M, false>(sc, pp, pb, q, st, fetch, vis, SplatTarget{}, grid, s);
+                  StatCounters* st, uint8_t* vis, int grid, cudaStream_t s) {
+    shadowKernels<M, false>(sc, pp, pb, q, st, q.counts + kFetchShadow, vis, SplatTarget{}, grid, s);
 }
 template <int M>
 void launchConnect(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
-                   StatCounters* st, uint32_t* fetch, uint8_t* vis, const SplatTarget& film, int grid, cudaStream_t s) {
-    shadowKernels<M, true>(sc, pp, pb, q, st, fetch, vis, film, grid, s);
+                   StatCounters* st, uint8_t* vis, const SplatTarget& film, int grid, cudaStream_t s) {
+    shadowKernels<M, true>(sc, pp, pb, q, st, q.counts + kFetchShadow, vis, film, grid, s);
 }
 void launchFoldFilm(const double* film, const double* comp, double* out, size_t n, cudaStream_t s) {
     kFoldFilm<<<int(std::min<size_t>((n + 255) / 256, 4096)), 256, 0, s>>>(film, comp, out, n);
@@ -1117,16 +1122,16 @@ void launchMaterialize(const uint32_t* leafOrder, uint32_t n, const float4* tri,
 #define OWEC_INSTANTIATE(M)                                                                                         \
     template void launchGenerate<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&, \
                                     StatCounters*, cudaStream_t);                                                   \
-    template void launchIntersect<M>(const DeviceScene&, const PathBuffers<RT<M>>&, const Queues&, int,             \
-                                     StatCounters*, uint32_t*, int, cudaStream_t);                                             \
+    template void launchIntersect<M>(const DeviceScene&, const PathBuffers<RT<M>>&, const Queues&,                  \
+                                     StatCounters*, int, cudaStream_t);                                             \
     template void launchMedium<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&,   \
-                                  int, StatCounters*, int, cudaStream_t);                                           \
+                                  StatCounters*, int, cudaStream_t);                                                \
     template void launchSurface<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&,  \
-                                   int, StatCounters*, int, cudaStream_t);                                          \
+                                   StatCounters*, int, cudaStream_t);                                               \
     template void launchShadow<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&,   \
-                                  StatCounters*, uint32_t*, uint8_t*, int, cudaStream_t);                                                \
+                                  StatCounters*, uint8_t*, int, cudaStream_t);                                      \
     template void launchConnect<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&,  \
-                                   StatCounters*, uint32_t*, uint8_t*, const SplatTarget&, int, cudaStream_t);      \
+                                   StatCounters*, uint8_t*, const SplatTarget&, int, cudaStream_t);                 \
     template void launchFilm<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, double*, double*,  \
                                 double*, uint32_t, cudaStream_t);                                                   \
     template void launchCastRays<M>(const DeviceScene&, uint64_t, const double*, const double*, uint32_t*,          \

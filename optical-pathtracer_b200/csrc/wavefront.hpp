@@ -17,21 +17,21 @@ template <int M>
 void launchGenerate(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&, StatCounters*,
                     cudaStream_t);
 template <int M>
-void launchIntersect(const DeviceScene&, const PathBuffers<ModeR<M>>&, const Queues&, int cur, StatCounters*,
-                     uint32_t* fetch, int grid, cudaStream_t);
+void launchIntersect(const DeviceScene&, const PathBuffers<ModeR<M>>&, const Queues&, StatCounters*, int grid,
+                     cudaStream_t);
 template <int M>
-void launchMedium(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&, int cur,
+void launchMedium(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&,
                   StatCounters*, int grid, cudaStream_t);
 template <int M>
-void launchSurface(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&, int cur,
+void launchSurface(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&,
                    StatCounters*, int grid, cudaStream_t);
 template <int M>
 void launchShadow(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&, StatCounters*,
-                  uint32_t* fetch, uint8_t* vis, int grid, cudaStream_t);
+                  uint8_t* vis, int grid, cudaStream_t);
 // The light integrator's connections to the eye: their visibility, transmittance and splats.
 template <int M>
 void launchConnect(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&, StatCounters*,
-                   uint32_t* fetch, uint8_t* vis, const SplatTarget& film, int grid, cudaStream_t);
+                   uint8_t* vis, const SplatTarget& film, int grid, cudaStream_t);
 void launchResolve(const double* film, const double* comp, const double* samples, uint32_t nPixels, double* xyz,
                    cudaStream_t);
 // out[i] = film[i] - comp[i] (the compensated sums as plain sums), n values, on stream s.
