@@ -109,6 +109,7 @@ struct DeviceScene {
     int32_t fullFeatures;     // 1: shapes beyond spheres, conic sags, plain apertures and cylinders, a
                               // planet-sized sphere, contacts or textured materials (the kernels' Full
                               // instantiations)
+    int32_t anyMedium;        // 1: some region's medium absorbs or scatters
     uint32_t opticsUsed;      // kOpticsSimple, kOpticsGeneral: the surface kernels with anything to do
     uint32_t nRegions, nBoundaries, nLights, nMedia;
     const WideNode* nodes;

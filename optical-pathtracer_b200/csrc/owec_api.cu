@@ -1016,6 +1016,12 @@ void uploadScene(owec_ctx& c, const owec_scene_desc& d) {
     ds.boundaries = c.dBoundaries.get();
     ds.lights = c.dLights.get();
     ds.shapeData = c.dShapeData.get();
+    ds.anyMedium = 0;
+    for (uint32_t i = 0; i < d.n_regions; ++i) {
+        const owec_medium& m = d.media[d.region_medium[i]];
+        for (int32_t sp : {m.absorption, m.scattering})
+            if (sp >= 0 && !(d.spectra[sp].kind == OWEC_SPEC_CONSTANT && d.spectra[sp].a == 0.0)) ds.anyMedium = 1;
+    }
     ds.opticsUsed = 0;
     for (uint32_t i = 0; i < d.n_boundaries; ++i) {
         const int32_t type = d.optics[d.boundaries[i].optics].type;

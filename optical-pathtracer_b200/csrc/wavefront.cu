@@ -372,6 +372,59 @@ __global__ void __launch_bounds__(128, OWEC_SHADING_MIN_BLOCKS) kMedium(DeviceSc
     }
 }
 
+// kMedium for a scene without any absorbing or scattering medium: a segment that met a boundary goes to
+// its surface queue on the hit record alone, and one that met none gathers the sky. 64 registers instead
+// of kMedium's 164: it waits on scattered loads, which twice the resident warps hide. With the surface
+// kernels' next index loaded ahead, the 256 x 256 glass film at 64 spp: 5.45 -> 5.09 ms a pass, the
+// 1920 x 1080 room 14.35 -> 13.91 ms (prefetching the next records as well gained nothing).
+template <int M>
+__global__ void __launch_bounds__(256) kRoute(DeviceScene sc, PassParams pp, PathBuffers<RT<M>> pb, Queues q, StatCounters* st) {
+    using R = RT<M>;
+    const uint32_t n = q.counts[kCountActive];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const uint32_t i = q.active[0][k];
+        const HitRec h = loadStream(pb.hit + i);
+        bool simple = false, general = false, leak = false;
+        if (h.boundary < kNone - 1u) {
+            if (h.boundary == pp.ckptBoundary) {
+                checkpointPath<M>(pp, loadStream(pb.ray + i), loadStream(pb.spec + i), loadStream(pb.aux + i), h);
+            } else {
+                const int32_t ot = sc.optics[sc.boundaries[h.boundary].optics].type;
+                simple = ot == OWEC_SURF_DIFFUSE || ot == OWEC_SURF_ABSORBER || ot == OWEC_SURF_DETECTOR;
+                general = !simple;
+            }
+        } else {
+            PathAux& aux = pb.aux[i];
+            const uint32_t flags = aux.flags;
+            if (h.boundary == kNone) {
+                const PathRay<R> ray = loadStream(pb.ray + i);
+                if (ray.region == 0) {
+                    // skyMet (transport.cpp:401-417)
+                    const V3<R> d = rayDir(ray);
+                    PathSpec<R>& sp = pb.spec[i];
+                    const bool spec = flags & kFlagSpecular;
+                    const V3<double> dd(d);
+                    const bool inSun = sc.hasSun && dot(dd, V3<double>(sc.sunDir[0], sc.sunDir[1], sc.sunDir[2])) >= sc.sunCosMax;
+                    R w = R(1);
+                    if (!spec && inSun) w = powerHeuristic(R(aux.prevPdf), R(sc.sunSelectPdf / sc.sunSolidAngle));
+                    for (int j = 0; j < NW; ++j) {
+                        const R lam = R(sp.lambda[j]);
+                        const R sky = skyRadiance(sc, dd, lam);
+                        const R sun = inSun ? evalSpectrum(sc, sc.sunSpectrum, lam) : R(0);
+                        sp.L[j] += float(sp.beta[j] * (sky + sun * w));
+                    }
+                } else {
+                    leak = true;
+                }
+            }
+            aux.flags = flags & ~kFlagAlive;
+        }
+        warpCount(&st->leaks, leak);
+        warpPush(q.surface, &q.counts[kCountSurface], general, i);
+        warpPush(q.surfaceSimple, &q.counts[kCountSimple], simple, i);
+    }
+}
+
 // ------------------------------------------------------------------ surface
 // Simple: the lean instantiation for the simple surface queue (Lambertian, absorbing and detecting
 // boundaries): the other lobes, dispersion and the index models compile out, and with them most of
@@ -400,8 +453,12 @@ __global__ void __launch_bounds__(128, Simple ? OWEC_SIMPLE_MIN_BLOCKS : OWEC_SH
     using Rr = typename Mode<M>::Rr;
     const uint32_t n = Simple ? q.counts[kCountSimple] : q.counts[kCountSurface];
     const uint32_t* queue = Simple ? q.surfaceSimple : q.surface;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t i = queue[k];
+    // the next path's index is loaded an iteration ahead: its records' loads then do not wait for it
+    const uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    uint32_t iNext = k0 < n ? queue[k0] : 0u;
+    for (uint32_t k = k0; k < n; k += stride) {
+        const uint32_t i = iNext;
+        if (k + stride < n) iNext = queue[k + stride];
         PathRay<R> ray = loadStream(pb.ray + i);
         PathSpec<R> sp = loadStream(pb.spec + i);
         PathAux aux = loadStream(pb.aux + i);
@@ -1034,7 +1091,8 @@ void launchIntersect(const DeviceScene& sc, const PathBuffers<RT<M>>& pb, const 
 template <int M>
 void launchMedium(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
                   StatCounters* st, int grid, cudaStream_t s) {
-    kMedium<M><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
+    if (sc.anyMedium) kMedium<M><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
+    else kRoute<M><<<grid, 256, 0, s>>>(sc, pp, pb, q, st);
 }
 template <int M>
 void launchSurface(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
