@@ -77,6 +77,7 @@ __device__ __forceinline__ bool survivesQ(PathSpec<R>& sp, Pcg32& rng, double& q
 // carries derivatives, so the maximum is the hero's).
 __device__ __forceinline__ void rouletteTangents(double* dB, int n, double q, double b0, bool fixedDecisions) {
     const bool moves = fixedDecisions && q < 1 && b0 > 0;
+#pragma unroll 1
     for (int k = 0; k < n; ++k) dB[k] = moves ? dB[k] / q - b0 * dB[k] / (q * q) : dB[k] / q;
 }
 
@@ -99,7 +100,7 @@ __device__ V3<double> hgDirectionTangent(const V3<double>& wo, const V3<double>&
 // Lambertian f = albedo / pi with pdf |cos| / pi about the fixed normal n. Medium vertices: the
 // Henyey-Greenstein phase of -d . wi as f and pdf, cosF = 1.
 template <int N>
-__device__ Dual<N> neeToArea(const DV3<N>& x, const DV3<N>* d, double g, const V3<double>& n, double albedoOverPi,
+__device__ __noinline__ Dual<N> neeToArea(const DV3<N>& x, const DV3<N>* d, double g, const V3<double>& n, double albedoOverPi,
                              const V3<double>& y, const V3<double>& nL, double area, double sel, double Le,
                              double sigmaT) {
     const DV3<N> v = y - x;
@@ -136,6 +137,7 @@ struct AdjointParams {
 template <int N>
 __device__ __forceinline__ void gather(PathTangents& tg, double beta, const Dual<N>& cb, const double (*pos)[3],
                                        bool useDir, bool usePdf) {
+#pragma unroll 1
     for (int k = 0; k < tg.n; ++k) {
         double s = 0;
         if (pos) s += cb.d[0] * pos[k][0] + cb.d[1] * pos[k][1] + cb.d[2] * pos[k][2];
@@ -147,6 +149,41 @@ __device__ __forceinline__ void gather(PathTangents& tg, double beta, const Dual
         }
         tg.acc[k] += cb.v * tg.dB[k] + beta * s;
     }
+}
+
+// The large pieces of a bounce that run at two or three of its places, out of line (with neeToArea, and
+// the loops over wavelengths and slots kept rolled): inlined everywhere, the replay was 632 KB of code, and
+// a warp spent 27 of 33.9 cycles per instruction waiting for the next one to be fetched. At 493 KB the
+// replay of 31,785 paths of the fog room takes 4.9 ms instead of 8.3 (10.4 before the lazy roots and the
+// out-of-line spectra). Arguments and results go by value, so that the caller's state stays in registers.
+// What feeds the forward pass's decisions in FP32 (interfaces, lobes) stays inline: a call boundary there
+// changed a rounding, and with it paths.
+template <class R>
+struct LightDraw {
+    LightSampleD ls;
+    uint64_t rngState;
+    int li;
+    bool ok;
+};
+template <class R>
+__device__ __noinline__ LightDraw<R> drawLight(const DeviceScene* sc, V3<double> ref, Pcg32 rng) {
+    LightDraw<R> r;
+    r.ok = sampleLight<R>(*sc, ref, rng, r.ls, r.li);
+    r.rngState = rng.state;
+    return r;
+}
+struct TraceResult {
+    HitRec hit;
+    int status;
+};
+template <int M, bool AnyHit, bool Full>
+__device__ __noinline__ TraceResult traceQuery(const DeviceScene* sc, RayQuery<typename Mode<M>::R> q, StackEntry* stack, int stride) {
+    TraceResult r;
+    r.hit.boundary = kNone;
+    r.hit.t = INFINITY;
+    r.hit.flags = 0;
+    r.status = traceRay<typename Mode<M>::R, typename Mode<M>::Ro, typename Mode<M>::Rr, AnyHit, Full>(*sc, q, stack, stride, r.hit);
+    return r;
 }
 
 // The visibility and transmittance of a next-event sample (kShadowVis and kShadowApply: any-hit
@@ -178,12 +215,10 @@ __device__ bool neeClear(const DeviceScene& sc, const LightSampleD& ls, const V3
         sq.errN = R(errN);
         sq.tmax = R(tq);
         sq.region = region;
-        HitRec sh;
-        sh.boundary = kNone;
-        sh.t = INFINITY;
-        sh.flags = 0;
         if (kEndpoint && finite) {
-            const int vs = traceRay<R, Ro, Rr, false, Full>(sc, sq, stack, stride, sh);
+            const TraceResult tr = traceQuery<M, false, Full>(sc.self, sq, stack, stride);
+            const HitRec& sh = tr.hit;
+            const int vs = tr.status;
             if (vs == kTraceOverflow) {
                 fault = true;
                 return false;
@@ -191,7 +226,7 @@ __device__ bool neeClear(const DeviceScene& sc, const LightSampleD& ls, const V3
             clear = vs != kTraceHit || sh.t > ls.dist ||
                     (sh.boundary == ls.boundary && !(sh.flags & kHitAmbiguous) && fabs(sh.t - ls.dist) <= w);
         } else {
-            const int vs = traceRay<R, Ro, Rr, true, Full>(sc, sq, stack, stride, sh);
+            const int vs = traceQuery<M, true, Full>(sc.self, sq, stack, stride).status;
             if (vs == kTraceOverflow) {
                 fault = true;
                 return false;
@@ -267,10 +302,9 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
             rq.depP = ray.depP;
             rq.region = ray.region;
             rq.errN = R(ray.errN);
-            h.boundary = kNone;
-            h.t = INFINITY;
-            h.flags = 0;
-            const int s = traceRay<R, Ro, Rr, false, Full>(sc, rq, stack, stride, h);
+            const TraceResult tr = traceQuery<M, false, Full>(sc.self, rq, stack, stride);
+            h = tr.hit;
+            const int s = tr.status;
             if (s != kTraceHit) { h.boundary = kNone; h.t = INFINITY; }
             if (s == kTraceOverflow) { fault = true; break; }
             found = h.boundary < kNone - 1u;
@@ -289,6 +323,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                             sp.beta[j] *= evalSpectrum(sc, med.scattering, R(sp.lambda[j])) * exp(-sT[j] * R(tS)) / pdf0;
                         // the hero's weight sigma_s / sigma_t does not move with the heights
                         const double w0 = b0 != R(0) ? double(sp.beta[0]) / double(b0) : 0.0;
+#pragma unroll 1
                         for (int k = 0; k < tg.n; ++k) tg.dB[k] *= w0;
                         event = 1;
                     } else if (isinf(seg)) {
@@ -312,13 +347,18 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
         if (event == 1) {
             // ------------------------------------------------------------ scatterInMedium
             const V3<double> sp3 = rayOrigin(ray.o) + dd * tS;
+#pragma unroll 1
             for (int k = 0; k < tg.n; ++k)
                 for (int a = 0; a < 3; ++a) tg.dO[k][a] += tS * tg.dD[k][a];
             if (int(aux.depth) >= pp.maxDepth) break;
             R betaNee[NW];
             for (int j = 0; j < NW; ++j) betaNee[j] = sp.beta[j];
             int li;
-            if (sampleLight<R>(sc, sp3, rng, ls, li)) {
+            const LightDraw<R> draw = drawLight<R>(sc.self, sp3, rng);
+            rng.state = draw.rngState;
+            ls = draw.ls;
+            li = draw.li;
+            if (draw.ok) {
                 bool leZero = true;
                 for (int j = 0; j < NW; ++j)
                     if (lightSampleLe<R>(sc, ls, R(sp.lambda[j])) != R(0)) leZero = false;
@@ -357,6 +397,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
             if (tg.n > 0 && P.fixedDecisions) {
                 // the drawn angles stay: the direction turns with the incident one, weight 1
                 const V3<double> wo = -dd, w(wi);
+#pragma unroll 1
                 for (int k = 0; k < tg.n; ++k) {
                     st3(tg.dD[k], hgDirectionTangent(wo, w, -ld3(tg.dD[k])));
                     tg.dPdf[k] = 0;
@@ -368,6 +409,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                 const double denom = 1 + g * g + 2 * g * c;
                 const double ph = (1 - g * g) / (4 * kPi * denom * sqrt(denom));
                 const double dphdc = ph * (-1.5) * (2 * g) / denom;
+#pragma unroll 1
                 for (int k = 0; k < tg.n; ++k) {
                     const double dc = -(tg.dD[k][0] * w.x + tg.dD[k][1] * w.y + tg.dD[k][2] * w.z);
                     tg.dB[k] += double(sp.beta[0]) * dphdc * dc / ph;
@@ -454,6 +496,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                         for (int a = 0; a < 3; ++a) vid[a] = int(P.hf.tris[3 * size_t(h.prim) + a]);
                         for (int a = 0; a < 3 && tg.valid; ++a) {
                             bool present = false;
+#pragma unroll 1
                             for (int k = 0; k < tg.n; ++k) present = present || tg.vert[k] == vid[a];
                             if (present) continue;
                             if (tg.n == kSlots) { tg.valid = false; break; }
@@ -473,6 +516,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                     const double t = dot(gp.p - rayOrigin(ray.o), dd);  // the refined distance
                     V3<double> center;
                     if (bd.shape == OWEC_SHAPE_SPHERE) center = bd.toWorld.point(V3<double>(0, 0, 0));
+#pragma unroll 1
                     for (int k = 0; k < tg.n; ++k) {
                         V3<double> dv0, dv1, dv2, dnuk;
                         if (hfHit) {
@@ -532,6 +576,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                             const Dual<7> cosL = dabs(ddot(v, n)) / dsqrt(d2);
                             const Dual<7> plD = sc.lights[bd.light].pdf * d2 / (cosL * bd.area);
                             const Dual<7> cb = Le * dpowerHeuristic(Dual<7>::var(double(aux.prevPdf), 6), plD);
+#pragma unroll 1
                             for (int k = 0; k < tg.n; ++k) {
                                 double dc = cb.v * tg.dB[k];
                                 double s3 = 0;
@@ -555,6 +600,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                 ray.errN = errN;
                 cont = int(aux.depth) < 4 * pp.maxDepth;
                 if (tg.valid)
+#pragma unroll 1
                     for (int k = 0; k < tg.n; ++k)
                         for (int c = 0; c < 3; ++c) tg.dO[k][c] = dP[k][c];
             } else if (o.type != OWEC_SURF_ABSORBER && o.type != OWEC_SURF_DETECTOR && int(aux.depth) < pp.maxDepth) {
@@ -567,6 +613,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                     bool alive2 = false;
                     for (int j = 1; j < NW; ++j) alive2 = alive2 || sp.pdf[j] != 0.f;
                     if (alive2) {
+#pragma unroll 1
                         for (int j = 1; j < NW; ++j) {
                             if (sp.pdf[j] == 0.f) continue;
                             const Interface<R> it2 = makeInterface(sc, bd, gp.n, R(sp.lambda[j]), R(pp.fresnelFloor), tex);
@@ -591,7 +638,11 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                 for (int j = 0; j < NW; ++j) betaNee[j] = sp.beta[j];
                 if (!isDeltaOptics<R>(o)) {
                     int li;
-                    if (sampleLight<R>(sc, gp.p, rng, ls, li)) {
+                    const LightDraw<R> draw = drawLight<R>(sc.self, gp.p, rng);
+                    rng.state = draw.rngState;
+                    ls = draw.ls;
+                    li = draw.li;
+                    if (draw.ok) {
                         bool leZero = true;
                         for (int j = 0; j < NW; ++j)
                             if (lightSampleLe<R>(sc, ls, R(sp.lambda[j])) != R(0)) leZero = false;
@@ -600,6 +651,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                             bool fZero = true;
                             R fN[NW] = {R(0), R(0), R(0), R(0)};
                             R pdfS = R(0);
+#pragma unroll 1
                             for (int j = 0; j < NW; ++j) {
                                 if (sp.pdf[j] == 0.f) continue;
                                 R pdf;
@@ -674,6 +726,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                             const bool fr = dot(dd, n) < 0;
                             const double ni = fr ? double(it.nFront) : double(it.nBack);
                             const double nt = fr ? double(it.nBack) : double(it.nFront);
+#pragma unroll 1
                             for (int k = 0; k < tg.n; ++k) {
                                 const V3<double> dnk = ld3(dN[k]), dDk = ld3(tg.dD[k]);
                                 const double dc = -(dot(dDk, n) + dot(dd, dnk));  // d cos(incidence) against n
@@ -691,6 +744,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                                 tg.dPdf[k] = 0;
                             }
                         } else if (o.type == OWEC_SURF_MIRROR) {
+#pragma unroll 1
                             for (int k = 0; k < tg.n; ++k) {
                                 tg.dB[k] *= double(ss.weight);
                                 st3(tg.dD[k], reflectTangent(dd, n, ld3(tg.dD[k]), ld3(dN[k])));
@@ -699,17 +753,20 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                         } else {
                             // Lambertian: the direction drawn about the fixed normal stays; its
                             // weight (the albedo) and pdf do not move
+#pragma unroll 1
                             for (int k = 0; k < tg.n; ++k) {
                                 tg.dB[k] *= double(ss.weight);
                                 tg.dD[k][0] = tg.dD[k][1] = tg.dD[k][2] = 0;
                                 tg.dPdf[k] = 0;
                             }
                         }
+#pragma unroll 1
                         for (int k = 0; k < tg.n; ++k)
                             for (int c = 0; c < 3; ++c) tg.dO[k][c] = dP[k][c];
                     }
                     // weighScatter (transport.cpp:227-233)
                     sp.beta[0] *= ss.weight;
+#pragma unroll 1
                     for (int j = 1; j < NW; ++j) {
                         if (sp.pdf[j] == 0.f) continue;
                         const Interface<R> itj = makeInterface<R, false>(sc, bd, gp.n, R(sp.lambda[j]), R(pp.fresnelFloor), tex);
@@ -767,6 +824,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
     const double gam = double(aux.weight) * inv / double(sp.pdf[0]) * (g[0] * cieX(l0) + g[1] * cieY(l0) + g[2] * cieZ(l0)) *
                        P.t.invSamples;
     if (gam == 0) return;
+#pragma unroll 1
     for (int k = 0; k < tg.n; ++k)
         if (tg.acc[k] != 0) atomicAdd(P.t.dH + tg.vert[k], tg.acc[k] * gam);
 }
