@@ -1461,7 +1461,6 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
     pp.ckptBoundary = c.hf.boundary;
     pp.ckptCount = ckptCount.get();
     pp.ckpt = ckpt.get();
-    const int grid = c.numSMs * 8;
     int unusedBounces = 0;
     cudaEvent_t replayStart, replayStop;
     OWEC_CUDA(cudaEventCreate(&replayStart));
@@ -1478,7 +1477,7 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
                    [&](const Queues& bq, int g) { queueBounce<M>(c, pp, pb, bq, g, st.get()); });
         joinShadows(c);
         OWEC_CUDA(cudaEventRecord(replayStart, c.stream));
-        launchPathAdjoint(M, c.ds, pp, c.hf, t, fixedDecisions, ckpt.get(), ckptCount.get(), grid, c.stream);
+        launchPathAdjoint(M, c.ds, pp, c.hf, t, fixedDecisions, ckpt.get(), ckptCount.get(), c.numSMs, c.stream);
         checkLaunch();
         OWEC_CUDA(cudaEventRecord(replayStop, c.stream));
         OWEC_CUDA(cudaEventSynchronize(replayStop));
@@ -2094,7 +2093,7 @@ int owec_walk(owec_ctx* ctx, const owec_walk_desc* w, uint64_t first, uint64_t n
         if (n == 0) return;
         OWEC_CUDA(cudaEventRecord(ctx->passStart, ctx->stream));
         launchWalk(ctx->settings.precision, ctx->ds, *w, ctx->boundaries[w->target].toLocal, first, n,
-                   ctx->dWalkBins.get(), ctx->dWalkStats.get(), ctx->numSMs * 8, ctx->stream);
+                   ctx->dWalkBins.get(), ctx->dWalkStats.get(), ctx->numSMs, ctx->stream);
         checkLaunch();
         OWEC_CUDA(cudaEventRecord(ctx->passStop, ctx->stream));
         OWEC_CUDA(cudaEventSynchronize(ctx->passStop));
@@ -2195,7 +2194,7 @@ int owec_walk_adjoint(owec_ctx* ctx, const owec_walk_desc* w, uint64_t first, ui
         const double binArea = (2 * w->half_x / w->width) * (2 * w->half_y / w->height);
         OWEC_CUDA(cudaEventRecord(ctx->passStart, ctx->stream));
         launchWalkAdjoint(ctx->settings.precision, ctx->ds, *w, ctx->boundaries[w->target].toLocal, ctx->hf, first, n,
-                          measure / (double(n) * binArea), dG.get(), dDH.get(), st.get(), ctx->numSMs * 8, ctx->stream);
+                          measure / (double(n) * binArea), dG.get(), dDH.get(), st.get(), ctx->numSMs, ctx->stream);
         checkLaunch();
         OWEC_CUDA(cudaEventRecord(ctx->passStop, ctx->stream));
         std::vector<double> h(nh);
@@ -2245,7 +2244,7 @@ int owec_walk_adjoint_noalloc(owec_ctx* ctx, const owec_walk_desc* w, uint64_t f
         publishScene(*ctx);  // a copy into the context's own scene buffer: no allocation
         OWEC_CUDA(cudaEventRecord(ctx->passStart, ctx->stream));
         launchWalkAdjoint(ctx->settings.precision, ctx->ds, *w, ctx->boundaries[w->target].toLocal, ctx->hf, first, n,
-                          measure / (double(n) * binArea), dG, dDH, st, ctx->numSMs * 8, ctx->stream);
+                          measure / (double(n) * binArea), dG, dDH, st, ctx->numSMs, ctx->stream);
         checkLaunch();
         OWEC_CUDA(cudaEventRecord(ctx->passStop, ctx->stream));
         OWEC_CUDA(cudaMemcpyAsync(dheights, dDH, nh * 8, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2307,8 +2306,8 @@ int owec_path_adjoint(owec_ctx* ctx, uint64_t first_pass, int spp, int flags, co
                 const uint32_t S = std::min<uint32_t>(perBatch, uint32_t(spp - done));
                 pp.nPaths = S * nPix;
                 pp.streamBase = uint32_t(first_pass + uint64_t(done));
-                launchPathAdjoint(ctx->settings.precision, ctx->ds, pp, ctx->hf, t, fixed, nullptr, nullptr,
-                                  ctx->numSMs * 8, ctx->stream);
+                launchPathAdjoint(ctx->settings.precision, ctx->ds, pp, ctx->hf, t, fixed, nullptr, nullptr, ctx->numSMs,
+                                  ctx->stream);
                 checkLaunch();
                 done += int(S);
             }

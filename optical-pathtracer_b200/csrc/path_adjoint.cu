@@ -249,23 +249,33 @@ __device__ bool neeClear(const DeviceScene& sc, const LightSampleD& ls, const V3
     return clear;
 }
 
-// One camera path from `ray`, `sp`, `aux`, `rng` on: from its camera ray (resume null), or from a
-// checkpoint at its first heightfield surface event (resume: that event's hit, whose segment's free
-// flight the forward pass has already taken).
+// A camera path in replay: from its camera ray, or from a checkpoint at its first heightfield surface event
+// (resume: that event's hit, whose segment's free flight the forward pass has already taken).
+template <class R>
+struct AdjointPath {
+    PathRay<R> ray;
+    PathSpec<R> sp;
+    PathAux aux;
+    Pcg32 rng;
+    HitRec resumed;
+    bool resume, metHeightfield, fault;
+};
+
+// One bounce of the path; false when the path ends with it.
 template <int M, bool Full>
-__device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathRay<typename Mode<M>::R> ray,
-                            PathSpec<typename Mode<M>::R> sp, PathAux aux, Pcg32 rng, const HitRec* resume,
-                            StackEntry* stack, int stride) {
+__device__ __forceinline__ bool adjointBounce(const DeviceScene& sc, const AdjointParams& P,
+                                              AdjointPath<typename Mode<M>::R>& ps, PathTangents& tg, StackEntry* stack,
+                                              int stride) {
     using R = typename Mode<M>::R;
     using Ro = typename Mode<M>::Ro;
     using Rr = typename Mode<M>::Rr;
     const PassParams& pp = P.pp;
-    unsigned long long* ctr = P.t.counters;
-    PathTangents tg;
-    tg.n = 0;
-    tg.valid = true;
-    bool metHeightfield = false, fault = false;
-    for (;;) {
+    PathRay<R>& ray = ps.ray;
+    PathSpec<R>& sp = ps.sp;
+    PathAux& aux = ps.aux;
+    Pcg32& rng = ps.rng;
+    bool &metHeightfield = ps.metHeightfield, &fault = ps.fault;
+    {
         const V3<R> d = rayDir(ray);
         const V3<double> dd(d);
         const owec_medium med = sc.media[sc.regionMedium[ray.region]];
@@ -281,10 +291,10 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
         LightSampleD ls;
         R contrib[NW] = {R(0), R(0), R(0), R(0)};
         R Tr[NW];
-        if (resume) {
+        if (ps.resume) {
             // the checkpointed surface event: its segment's Beer-Lambert factor is already applied
-            h = *resume;
-            resume = nullptr;
+            h = ps.resumed;
+            ps.resume = false;
             found = true;
             if (absorbs && !scatters) {
                 sigmaA0 = evalSpectrum(sc, med.absorption, R(sp.lambda[0]));
@@ -306,7 +316,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
             h = tr.hit;
             const int s = tr.status;
             if (s != kTraceHit) { h.boundary = kNone; h.t = INFINITY; }
-            if (s == kTraceOverflow) { fault = true; break; }
+            if (s == kTraceOverflow) { fault = true; return false; }
             found = h.boundary < kNone - 1u;
             // ------------------------------------------------------------ free flight (kMedium)
             if (!(found && !absorbs && !scatters)) {
@@ -350,7 +360,7 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
 #pragma unroll 1
             for (int k = 0; k < tg.n; ++k)
                 for (int a = 0; a < 3; ++a) tg.dO[k][a] += tS * tg.dD[k][a];
-            if (int(aux.depth) >= pp.maxDepth) break;
+            if (int(aux.depth) >= pp.maxDepth) return false;
             R betaNee[NW];
             for (int j = 0; j < NW; ++j) betaNee[j] = sp.beta[j];
             int li;
@@ -460,9 +470,9 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
                     }
                 }
             }
-            break;
+            return false;
         } else if (event == 2) {
-            break;
+            return false;
         } else {
             // ------------------------------------------------------------ the boundary met (kSurface)
             const DBoundary& bd = sc.boundaries[h.boundary];
@@ -794,9 +804,19 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
             }
             (void)scattered;
         }
-        if (!cont) break;
-        aux.depth += 1;
+        if (cont) aux.depth += 1;
+        return cont;
     }
+}
+
+// The end of a path: its derivative weighted as the film weighs its radiance, added to the vertices'.
+template <int M>
+__device__ __forceinline__ void adjointEnd(const DeviceScene& sc, const AdjointParams& P,
+                                           const AdjointPath<typename Mode<M>::R>& ps, const PathTangents& tg) {
+    const PathSpec<typename Mode<M>::R>& sp = ps.sp;
+    const PathAux& aux = ps.aux;
+    const bool metHeightfield = ps.metHeightfield, fault = ps.fault;
+    unsigned long long* ctr = P.t.counters;
     // ---------------------------------------------------------------- the film's weighting (kFilm)
     const uint32_t pixel = aux.pixel;
     const double inv = 1.0 / (NW * sc.cieYIntegral);
@@ -829,33 +849,64 @@ __device__ void adjointPath(const DeviceScene& sc, const AdjointParams& P, PathR
         if (tg.acc[k] != 0) atomicAdd(P.t.dH + tg.vert[k], tg.acc[k] * gam);
 }
 
+// Both replays run one block of kAdjointBlock threads per SM, whose warps take their bounces in step: out of
+// step, each of them dragged its own part of the kernel's code through the instruction cache. A lane whose
+// path ends takes its next one. Paths are dealt to the blocks in turn, so that a launch of fewer paths than
+// lanes still fills every SM. The fog room's 31,785 paths: 4.9 -> 3.86 ms.
+constexpr int kAdjointBlock = 256;
+
 // Full replay: every camera path of the batch from its camera ray.
 template <int M, bool Full>
-__global__ void __launch_bounds__(128) kPathAdjoint(DeviceScene sc, AdjointParams P) {
+__global__ void __launch_bounds__(kAdjointBlock) kPathAdjoint(DeviceScene sc, AdjointParams P) {
     extern __shared__ StackEntry stackMem[];
-    StackEntry* stack = stackMem + threadIdx.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.pp.nPaths; i += gridDim.x * blockDim.x) {
-        PathRay<typename Mode<M>::R> ray;
-        PathSpec<typename Mode<M>::R> sp;
-        PathAux aux;
-        Pcg32 rng;
-        if (generateCameraPath<M>(sc, P.pp, i, ray, sp, aux, rng))
-            adjointPath<M, Full>(sc, P, ray, sp, aux, rng, nullptr, stack, blockDim.x);
+    AdjointPath<typename Mode<M>::R> ps;
+    PathTangents tg;
+    bool alive = false;
+    for (uint64_t i = blockIdx.x + uint64_t(gridDim.x) * threadIdx.x;;) {
+        for (; !alive && i < P.pp.nPaths; i += uint64_t(gridDim.x) * blockDim.x) {
+            alive = generateCameraPath<M>(sc, P.pp, uint32_t(i), ps.ray, ps.sp, ps.aux, ps.rng);
+            ps.resume = ps.metHeightfield = ps.fault = false;
+            tg.n = 0;
+            tg.valid = true;
+        }
+        if (!__syncthreads_or(alive)) break;
+        if (alive && !adjointBounce<M, Full>(sc, P, ps, tg, stackMem + threadIdx.x, blockDim.x)) {
+            adjointEnd<M>(sc, P, ps, tg);
+            alive = false;
+        }
     }
 }
 
 // From the checkpoints the wavefront left at the paths' first heightfield surface events.
 template <int M, bool Full>
-__global__ void __launch_bounds__(128) kPathAdjointResume(DeviceScene sc, AdjointParams P,
-                                                          const PathCheckpoint<typename Mode<M>::R>* ckpt,
-                                                          const uint32_t* count) {
+__global__ void __launch_bounds__(kAdjointBlock) kPathAdjointResume(DeviceScene sc, AdjointParams P,
+                                                                    const PathCheckpoint<typename Mode<M>::R>* ckpt,
+                                                                    const uint32_t* count) {
     extern __shared__ StackEntry stackMem[];
-    StackEntry* stack = stackMem + threadIdx.x;
     const uint32_t n = *count;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const PathCheckpoint<typename Mode<M>::R> c = loadStream(ckpt + i);
-        const Pcg32 rng{c.aux.rngState, (uint64_t(c.aux.stream) << 1u) | 1u};
-        adjointPath<M, Full>(sc, P, c.ray, c.spec, c.aux, rng, &c.hit, stack, blockDim.x);
+    AdjointPath<typename Mode<M>::R> ps;
+    PathTangents tg;
+    bool alive = false;
+    for (uint64_t i = blockIdx.x + uint64_t(gridDim.x) * threadIdx.x;;) {
+        if (!alive && i < n) {
+            const PathCheckpoint<typename Mode<M>::R> c = loadStream(ckpt + i);
+            i += uint64_t(gridDim.x) * blockDim.x;
+            ps.ray = c.ray;
+            ps.sp = c.spec;
+            ps.aux = c.aux;
+            ps.rng = Pcg32{c.aux.rngState, (uint64_t(c.aux.stream) << 1u) | 1u};
+            ps.resumed = c.hit;
+            ps.resume = true;
+            ps.metHeightfield = ps.fault = false;
+            tg.n = 0;
+            tg.valid = true;
+            alive = true;
+        }
+        if (!__syncthreads_or(alive)) break;
+        if (alive && !adjointBounce<M, Full>(sc, P, ps, tg, stackMem + threadIdx.x, blockDim.x)) {
+            adjointEnd<M>(sc, P, ps, tg);
+            alive = false;
+        }
     }
 }
 
@@ -863,13 +914,13 @@ template <int M>
 void launchMode(const DeviceScene& sc, const AdjointParams& P, const void* ckpt, const uint32_t* count, int grid,
                 cudaStream_t s) {
     using C = PathCheckpoint<typename Mode<M>::R>;
-    const size_t smem = traversalSharedBytes(128);
+    const size_t smem = traversalSharedBytes(kAdjointBlock);
     if (ckpt) {
-        if (sc.fullFeatures) kPathAdjointResume<M, true><<<grid, 128, smem, s>>>(sc, P, static_cast<const C*>(ckpt), count);
-        else kPathAdjointResume<M, false><<<grid, 128, smem, s>>>(sc, P, static_cast<const C*>(ckpt), count);
+        if (sc.fullFeatures) kPathAdjointResume<M, true><<<grid, kAdjointBlock, smem, s>>>(sc, P, static_cast<const C*>(ckpt), count);
+        else kPathAdjointResume<M, false><<<grid, kAdjointBlock, smem, s>>>(sc, P, static_cast<const C*>(ckpt), count);
     } else {
-        if (sc.fullFeatures) kPathAdjoint<M, true><<<grid, 128, smem, s>>>(sc, P);
-        else kPathAdjoint<M, false><<<grid, 128, smem, s>>>(sc, P);
+        if (sc.fullFeatures) kPathAdjoint<M, true><<<grid, kAdjointBlock, smem, s>>>(sc, P);
+        else kPathAdjoint<M, false><<<grid, kAdjointBlock, smem, s>>>(sc, P);
     }
 }
 

@@ -362,13 +362,10 @@ __device__ __forceinline__ WalkEnd walkEvent(const DeviceScene& sc, const WalkPa
     }
 }
 
-// Resident blocks per SM the lean kernels are compiled for: 128 registers with a little spilling
-// against 166 without (three blocks): 9.3 against 10.3 ms for 4.2 M lens walks, 4.4 either way for the
-// caustic slab's, 6.75 against 6.86 ms for their adjoint; two blocks 14.0, 5.6 and 7.9 ms. The Full
-// kernels spill far more and take what registers they need.
-#ifndef OWEC_WALK_MIN_BLOCKS
-#define OWEC_WALK_MIN_BLOCKS 4
-#endif
+// Threads of a block: one block fills an SM's registers (128 each with a little spilling in the lean
+// kernels, 255 in the Full ones, which spill far more below that).
+template <bool Full>
+constexpr int kWalkBlock = Full ? 256 : 512;
 
 // Adds a per-lane count to a counter, one atomic per warp (all lanes of the warp present).
 __device__ __forceinline__ void flushCount(unsigned long long* counter, uint32_t v) {
@@ -379,14 +376,17 @@ __device__ __forceinline__ void flushCount(unsigned long long* counter, uint32_t
 // Persistent: a lane whose walk ends takes the next one before its warp's next event, so that a warp
 // does not run its longest walk (a ghost's many reflections) with the others' lanes idle, and the
 // counters are summed per lane and added once per warp at the end instead of with four atomics on one
-// line per walk. The kernel is bound by FP64 arithmetic of few lanes and by instruction fetch (its code
-// exceeds the instruction cache). 4.2 M walks: the cemented achromat 24.1 -> 9.3 ms with the analytic
-// roots taken lazily (classicRoots), the caustic slab 4.73 -> 4.40 ms, its adjoint 7.49 -> 6.75 ms;
-// refilling only when 8 or 32 lanes are idle: 22 and 25 ms for the lens.
+// line per walk. The kernel is bound by FP64 arithmetic and by instruction fetch (its 228 KB of code exceed
+// the instruction cache), so the warps of an SM take their events in step, one block to an SM: out of step
+// each of them drags its own part of the code through the cache.
+// 4.2 M walks, before / refilled, with the analytic roots taken lazily (classicRoots) / in step as well:
+// the cemented achromat 24.1 / 9.2 / 7.6 ms, the caustic slab 4.73 / 4.38 / 4.21, its adjoint 7.49 / 6.63 /
+// 5.30. Two blocks of 256 in step 9.0, 4.19 and 5.56 ms, four of 128 9.9, 4.25 and 6.12; refilling only when 8
+// lanes are idle 22 ms for the lens.
 template <int M, bool ADJ, bool Full>
-__global__ void __launch_bounds__(128, Full ? 1 : OWEC_WALK_MIN_BLOCKS) kWalk(DeviceScene sc, WalkParams P, unsigned long long* bins,
-                                                                   unsigned long long* stats, const double* g, double* dH,
-                                                                   unsigned long long* fetch) {
+__global__ void __launch_bounds__(kWalkBlock<Full>) kWalk(DeviceScene sc, WalkParams P, unsigned long long* bins,
+                                                          unsigned long long* stats, const double* g, double* dH,
+                                                          unsigned long long* fetch) {
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(128, Full ? 1 : OWEC_WALK_MIN_BLOCKS) kWalk(De
                 alive = true;
             }
         }
-        if (__ballot_sync(0xFFFFFFFFu, alive) == 0) break;
+        if (!__syncthreads_or(alive)) break;
         if (alive) {
             const WalkEnd e = walkEvent<M, ADJ, Full>(sc, P, ws, tg, stack, blockDim.x, bins, g, dH);
             if (e != kWalkGoes) {
@@ -436,17 +436,26 @@ __global__ void __launch_bounds__(128, Full ? 1 : OWEC_WALK_MIN_BLOCKS) kWalk(De
     flush();
 }
 
+template <int M, bool ADJ, bool Full>
+void walkKernelOf(const DeviceScene& sc, const WalkParams& P, unsigned long long* bins, unsigned long long* stats,
+                  const double* g, double* dH, int numSMs, cudaStream_t s) {
+    constexpr int block = kWalkBlock<Full>;
+    const size_t smem = traversalSharedBytes(block);
+    OWEC_CUDA(cudaFuncSetAttribute(kWalk<M, ADJ, Full>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    unsigned long long* fetch = stats + kWalkFetchWord;
+    OWEC_CUDA(cudaMemsetAsync(fetch, 0, sizeof(*fetch), s));
+    // few walks: a warp or two on every SM rather than full blocks on some
+    const uint64_t threads = std::min<uint64_t>(block, std::max<uint64_t>(32, (P.n / numSMs + 31) / 32 * 32));
+    const int grid = int(std::min<uint64_t>(uint64_t(numSMs), (P.n + threads - 1) / threads));
+    if (grid == 0) return;
+    kWalk<M, ADJ, Full><<<grid, int(threads), smem, s>>>(sc, P, bins, stats, g, dH, fetch);
+}
 // kWalk for the scene's shapes (the lean traversal unless the scene needs the full set).
 template <int M, bool ADJ>
 void walkKernel(const DeviceScene& sc, const WalkParams& P, unsigned long long* bins, unsigned long long* stats,
-                const double* g, double* dH, int grid, cudaStream_t s) {
-    const size_t smem = traversalSharedBytes(128);
-    unsigned long long* fetch = stats + kWalkFetchWord;
-    OWEC_CUDA(cudaMemsetAsync(fetch, 0, sizeof(*fetch), s));
-    grid = int(std::min<uint64_t>(uint64_t(grid), (P.n + 127) / 128));
-    if (grid == 0) return;
-    if (sc.fullFeatures) kWalk<M, ADJ, true><<<grid, 128, smem, s>>>(sc, P, bins, stats, g, dH, fetch);
-    else kWalk<M, ADJ, false><<<grid, 128, smem, s>>>(sc, P, bins, stats, g, dH, fetch);
+                const double* g, double* dH, int numSMs, cudaStream_t s) {
+    if (sc.fullFeatures) walkKernelOf<M, ADJ, true>(sc, P, bins, stats, g, dH, numSMs, s);
+    else walkKernelOf<M, ADJ, false>(sc, P, bins, stats, g, dH, numSMs, s);
 }
 
 __global__ void __launch_bounds__(256) kResolveWalk(const unsigned long long* bins, size_t n, double scale, double* out) {
@@ -476,13 +485,13 @@ WalkParams makeParams(const owec_walk_desc& w, const Xform& targetToLocal, uint6
 }  // namespace
 
 void launchWalk(int mode, const DeviceScene& sc, const owec_walk_desc& w, const Xform& targetToLocal, uint64_t first,
-                uint64_t n, unsigned long long* bins, unsigned long long* stats, int grid, cudaStream_t s) {
+                uint64_t n, unsigned long long* bins, unsigned long long* stats, int numSMs, cudaStream_t s) {
     HeightfieldParams hf{};
     hf.boundary = kNone;
     const WalkParams P = makeParams(w, targetToLocal, first, n, 1.0, hf);
-    if (mode == OWEC_PRECISION_FP64) walkKernel<OWEC_PRECISION_FP64, false>(sc, P, bins, stats, nullptr, nullptr, grid, s);
-    else if (mode == OWEC_PRECISION_FP32) walkKernel<OWEC_PRECISION_FP32, false>(sc, P, bins, stats, nullptr, nullptr, grid, s);
-    else walkKernel<OWEC_PRECISION_MIXED, false>(sc, P, bins, stats, nullptr, nullptr, grid, s);
+    if (mode == OWEC_PRECISION_FP64) walkKernel<OWEC_PRECISION_FP64, false>(sc, P, bins, stats, nullptr, nullptr, numSMs, s);
+    else if (mode == OWEC_PRECISION_FP32) walkKernel<OWEC_PRECISION_FP32, false>(sc, P, bins, stats, nullptr, nullptr, numSMs, s);
+    else walkKernel<OWEC_PRECISION_MIXED, false>(sc, P, bins, stats, nullptr, nullptr, numSMs, s);
 }
 
 void launchResolveWalk(const unsigned long long* bins, size_t n, double scale, double* out, cudaStream_t s) {
@@ -491,11 +500,11 @@ void launchResolveWalk(const unsigned long long* bins, size_t n, double scale, d
 
 void launchWalkAdjoint(int mode, const DeviceScene& sc, const owec_walk_desc& w, const Xform& targetToLocal,
                        const HeightfieldParams& hf, uint64_t first, uint64_t n, double scale, const double* g,
-                       double* dH, unsigned long long* stats, int grid, cudaStream_t s) {
+                       double* dH, unsigned long long* stats, int numSMs, cudaStream_t s) {
     const WalkParams P = makeParams(w, targetToLocal, first, n, scale, hf);
-    if (mode == OWEC_PRECISION_FP64) walkKernel<OWEC_PRECISION_FP64, true>(sc, P, nullptr, stats, g, dH, grid, s);
-    else if (mode == OWEC_PRECISION_FP32) walkKernel<OWEC_PRECISION_FP32, true>(sc, P, nullptr, stats, g, dH, grid, s);
-    else walkKernel<OWEC_PRECISION_MIXED, true>(sc, P, nullptr, stats, g, dH, grid, s);
+    if (mode == OWEC_PRECISION_FP64) walkKernel<OWEC_PRECISION_FP64, true>(sc, P, nullptr, stats, g, dH, numSMs, s);
+    else if (mode == OWEC_PRECISION_FP32) walkKernel<OWEC_PRECISION_FP32, true>(sc, P, nullptr, stats, g, dH, numSMs, s);
+    else walkKernel<OWEC_PRECISION_MIXED, true>(sc, P, nullptr, stats, g, dH, numSMs, s);
 }
 
 }  // namespace owec

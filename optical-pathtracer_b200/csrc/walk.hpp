@@ -22,7 +22,7 @@ constexpr int kWalkStats = 5, kWalkFetchWord = 5, kWalkStatWords = 6;
 // n walks starting at walk index `first`, binned into `bins` (width * height 64-bit fixed-point
 // sums, 2^-32 per unit throughput); stats: kWalkStatWords words.
 void launchWalk(int mode, const DeviceScene& sc, const owec_walk_desc& w, const Xform& targetToLocal, uint64_t first,
-                uint64_t n, unsigned long long* bins, unsigned long long* stats, int grid, cudaStream_t s);
+                uint64_t n, unsigned long long* bins, unsigned long long* stats, int numSMs, cudaStream_t s);
 
 // The irradiance per bin: out[i] = bins[i] * scale.
 void launchResolveWalk(const unsigned long long* bins, size_t n, double scale, double* out, cudaStream_t s);
@@ -31,6 +31,6 @@ void launchResolveWalk(const unsigned long long* bins, size_t n, double scale, d
 // whose derivative could not be followed are counted in stats[4].
 void launchWalkAdjoint(int mode, const DeviceScene& sc, const owec_walk_desc& w, const Xform& targetToLocal,
                        const HeightfieldParams& hf, uint64_t first, uint64_t n, double scale, const double* g,
-                       double* dH, unsigned long long* stats, int grid, cudaStream_t s);
+                       double* dH, unsigned long long* stats, int numSMs, cudaStream_t s);
 
 }  // namespace owec
