@@ -1096,15 +1096,13 @@ void launchMedium(const DeviceScene& sc, const PassParams& pp, const PathBuffers
 }
 template <int M>
 void launchSurface(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
-                   StatCounters* st, int grid, cudaStream_t s) {
-    // a scene whose boundaries are all Lambertian, absorbing or detecting (or none of them) fills one of
-    // the two surface queues only
+                   StatCounters* st, uint32_t optics, int grid, cudaStream_t s) {
     if (sc.fullFeatures) {
-        if (sc.opticsUsed & kOpticsSimple) kSurface<M, true, true><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
-        if (sc.opticsUsed & kOpticsGeneral) kSurface<M, false, true><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
+        if (optics == kOpticsSimple) kSurface<M, true, true><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
+        if (optics == kOpticsGeneral) kSurface<M, false, true><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
     } else {
-        if (sc.opticsUsed & kOpticsSimple) kSurface<M, true, false><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
-        if (sc.opticsUsed & kOpticsGeneral) kSurface<M, false, false><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
+        if (optics == kOpticsSimple) kSurface<M, true, false><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
+        if (optics == kOpticsGeneral) kSurface<M, false, false><<<grid, 128, 0, s>>>(sc, pp, pb, q, st);
     }
 }
 // The shadow-ray kernels of a bounce: visibility then contributions without null boundaries, the
@@ -1185,7 +1183,7 @@ void launchMaterialize(const uint32_t* leafOrder, uint32_t n, const float4* tri,
     template void launchMedium<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&,   \
                                   StatCounters*, int, cudaStream_t);                                                \
     template void launchSurface<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&,  \
-                                   StatCounters*, int, cudaStream_t);                                               \
+                                   StatCounters*, uint32_t, int, cudaStream_t);                                               \
     template void launchShadow<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&,   \
                                   StatCounters*, uint8_t*, int, cudaStream_t);                                      \
     template void launchConnect<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, const Queues&,  \

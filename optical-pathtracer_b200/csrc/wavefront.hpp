@@ -22,9 +22,10 @@ void launchIntersect(const DeviceScene&, const PathBuffers<ModeR<M>>&, const Que
 template <int M>
 void launchMedium(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&,
                   StatCounters*, int grid, cudaStream_t);
+// optics: kOpticsSimple or kOpticsGeneral, one surface queue's kernel.
 template <int M>
 void launchSurface(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&,
-                   StatCounters*, int grid, cudaStream_t);
+                   StatCounters*, uint32_t optics, int grid, cudaStream_t);
 template <int M>
 void launchShadow(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&, StatCounters*,
                   uint8_t* vis, int grid, cudaStream_t);
