@@ -134,9 +134,7 @@ __device__ __forceinline__ bool acceptCrossing(const DeviceScene& sc, const V3<T
 }
 
 // Relative widening of far planes against the rounding of the slab distances (a few ulps).
-template <class T> __device__ __forceinline__ T farWiden();
-template <> __device__ __forceinline__ float farWiden<float>() { return 4e-7f; }
-template <> __device__ __forceinline__ double farWiden<double>() { return 4e-16; }
+constexpr float kFarWiden = 4e-7f;
 
 // The analytic boundary b's first acceptable crossing in (0, best); FP64 refinement when Rr = double.
 template <class R, class Rr, class T, bool Full, bool Rolled>
@@ -293,9 +291,15 @@ __device__ __forceinline__ void loadNode(const WideNode* nodes, uint32_t i, Node
 }
 
 
-// Decoded child boxes of a node, slab-tested against the ray. Returns the hit mask (slot order).
-template <class T>
-__device__ __forceinline__ uint32_t intersectChildren(const NodeWords& nd, const V3<T>& inv, const V3<T>& oinv, T tmin, T tmax) {
+// Decoded child boxes of a node, slab-tested against the ray. Returns the hit mask (slot order). The test is
+// in FP32 in every mode: it only has to be conservative. FromDouble: the ray is an FP64 one, whose origin's
+// and direction's rounding the slabs are widened by (a couple of ulps of each plane's and the origin's
+// distances along the ray), where the FP32 modes' boxes are padded for their rays. 641 x 359 room in FP64 at
+// 3 spp: 8.21 -> 6.74 ms a pass, kIntersect 5.35 -> 4.10 ms, films the same to the bit.
+template <bool FromDouble>
+__device__ __forceinline__ uint32_t intersectChildren(const NodeWords& nd, const V3<float>& inv, const V3<float>& oinv, float tmin,
+                                                      float tmax) {
+    using T = float;
     const T sx = T(__uint_as_float((nd.a.w & 0xFFu) << 23));
     const T sy = T(__uint_as_float(((nd.a.w >> 8) & 0xFFu) << 23));
     const T sz = T(__uint_as_float(((nd.a.w >> 16) & 0xFFu) << 23));
@@ -311,13 +315,18 @@ __device__ __forceinline__ uint32_t intersectChildren(const NodeWords& nd, const
     const T b0y = T(__uint_as_float(nd.a.y)) * inv.y - oinv.y;
     const T b0z = T(__uint_as_float(nd.a.z)) * inv.z - oinv.z;
     const T bx = b0x - T(32768) * ax, by = b0y - T(32768) * ay, bz = b0z - T(32768) * az;
-    const T mx = T(0.00390625) * fabs(ax) + T(2.4e-7) * fabs(bx);
-    const T my = T(0.00390625) * fabs(ay) + T(2.4e-7) * fabs(by);
-    const T mz = T(0.00390625) * fabs(az) + T(2.4e-7) * fabs(bz);
+    T mx = T(0.00390625) * fabs(ax) + T(2.4e-7) * fabs(bx);
+    T my = T(0.00390625) * fabs(ay) + T(2.4e-7) * fabs(by);
+    T mz = T(0.00390625) * fabs(az) + T(2.4e-7) * fabs(bz);
+    if (FromDouble) {
+        mx += T(3e-7) * (fabs(oinv.x) + fabs(b0x));
+        my += T(3e-7) * (fabs(oinv.y) + fabs(b0y));
+        mz += T(3e-7) * (fabs(oinv.z) + fabs(b0z));
+    }
     const T nbx = bx - mx, nby = by - my, nbz = bz - mz;
-    const T fbx = bx + mx + (fabs(b0x) + T(255) * fabs(ax)) * farWiden<T>();
-    const T fby = by + my + (fabs(b0y) + T(255) * fabs(ay)) * farWiden<T>();
-    const T fbz = bz + mz + (fabs(b0z) + T(255) * fabs(az)) * farWiden<T>();
+    const T fbx = bx + mx + (fabs(b0x) + T(255) * fabs(ax)) * kFarWiden;
+    const T fby = by + my + (fabs(b0y) + T(255) * fabs(ay)) * kFarWiden;
+    const T fbz = bz + mz + (fabs(b0z) + T(255) * fabs(az)) * kFarWiden;
     const bool nx = inv.x < T(0), ny = inv.y < T(0), nz = inv.z < T(0);
     // near and far planes per axis, chosen by the ray's direction on whole words
     const uint32_t nxl0 = nx ? nd.d.z : nd.c.x, nxl1 = nx ? nd.d.w : nd.c.y;
@@ -419,7 +428,7 @@ __device__ __forceinline__ uint32_t permuteSlots(uint32_t m, uint32_t x) {
 template <class T, class R, class Rr, bool AnyHit, class Stack = SharedStack, bool Count = true, bool Full = false>
 struct Traversal {
     V3<T> o, d;           // the ray, camera-relative
-    V3<T> inv, oinv;
+    V3<float> inv, oinv;  // for the slab tests
     T best;
     T bestCos;            // contact-resolving instantiation: |cos| of the closest crossing's incidence
     double bestD;         // and its distance in the refinement's precision
@@ -447,8 +456,8 @@ struct Traversal {
         c->region = q.region;
         o = q.o;
         d = q.d;
-        inv = V3<T>(safeInverse(d.x), safeInverse(d.y), safeInverse(d.z));
-        oinv = V3<T>(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+        inv = V3<float>(safeInverse(float(d.x)), safeInverse(float(d.y)), safeInverse(float(d.z)));
+        oinv = V3<float>(float(o.x) * inv.x, float(o.y) * inv.y, float(o.z) * inv.z);
         best = q.tmax;
         bestCos = T(1);
         bestD = double(q.tmax);
@@ -508,7 +517,7 @@ struct Traversal {
                 NodeWords nd;
                 loadNode(sc.nodes, node, nd);
                 if (Count) ++nodeVisits;
-                const uint32_t mask = intersectChildren(nd, inv, oinv, T(0), (Full && !AnyHit) ? tieLimit() : best);
+                const uint32_t mask = intersectChildren<sizeof(T) == sizeof(double)>(nd, inv, oinv, 0.f, slabLimit((Full && !AnyHit) ? tieLimit() : best));
                 const uint32_t inner = nd.a.w >> 24;
                 nodeBase = nd.b.x;
                 nodeBits = permuteSlots(mask & inner, first) | (inner << 8);
@@ -530,6 +539,12 @@ struct Traversal {
             }
         }
         return kTraceRunning;
+    }
+
+    // A distance as the slab tests' FP32 limit, rounded up.
+    __device__ __forceinline__ static float slabLimit(T t) {
+        if constexpr (sizeof(T) == sizeof(float)) return t;
+        else return float(t) + 3e-7f * fabsf(float(t));
     }
 
     // Contact decisions compare FP64 distances where the instantiation has them: the FP64 one, and
