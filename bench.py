@@ -702,11 +702,12 @@ def run_cuda(args):
             line["adjoint_study"] = adjoint_study(local)
             line["configs_study"] = configs_study(local)
             line["light_study"] = light_study(local)
-        # our own kernel launches in the timed region: intersect, medium, two surface kernels, the
-        # shadow visibility and its contributions per bounce, and generate + film per step; for
+        # our own kernel launches in the timed region: intersect, route, the lean surface kernel (the
+        # room's boundaries are all Lambertian or absorbing, its region holds no medium), the shadow
+        # visibility and its contributions per bounce, and generate + film per step; for
         # particles intersect, event, visibility and splats per bounce, and emit with the emitters'
         # own connections (visibility and splats) per step
-        line["gpu_launches"] = int(4 * launches + 3 * args.steps) if light else int(6 * launches + 2 * args.steps)
+        line["gpu_launches"] = int(4 * launches + 3 * args.steps) if light else int(5 * launches + 2 * args.steps)
         print(json.dumps(line))
     renderer.close()
     if world > 1:

@@ -368,14 +368,14 @@ void invertRigid(const double m[12], double out[12]) {
 }  // namespace
 
 // ------------------------------------------------------------------ the context
-// owec_cast_rays: a call of a few chunks goes through the context's own page-locked block (page-locking
-// costs 1 to 3 ms a call here up to 2 MB, whatever the size); a larger one through kCastWorkers host threads
-// with a chunk each, staged in a second block that the first such call page-locks.
+// owec_cast_rays: a small call goes through the context's own page-locked block, which is small enough to
+// share the runtime's 2 MB page-locked granules with other contexts' (a granule costs 1 to 3 ms); a larger
+// one through kCastWorkers host threads with a chunk each, staged in a block that the first such call makes.
 constexpr int kCastWorkers = 4;
-constexpr uint64_t kCastChunk = 16384, kCastSerial = 16;  // up to here one thread costs less than page-locking
+constexpr uint64_t kCastPiece = 4096, kCastSerial = 16 * kCastPiece, kCastChunk = 16384;
 constexpr size_t kCastBytesPerRay = 48 + 16;
 constexpr size_t kHostReports = 4096;  // the context block's first part: what kernels report to the host
-constexpr size_t kHostBlock = kHostReports + kCastChunk * kCastBytesPerRay;
+constexpr size_t kHostBlock = kHostReports + 2 * kCastPiece * kCastBytesPerRay;
 struct CastWorker {
     cudaStream_t stream = nullptr;
     void ensure() {
@@ -414,6 +414,8 @@ struct owec_ctx {
     uint32_t nTriangles = 0, nPrims = 0;
     bool hasNull = false;
     DeviceScene ds{};
+    DeviceScene published{};  // what dScene holds, once scenePublished
+    bool scenePublished = false;
     DBuf<DeviceScene> dScene;  // ds's copy on the device (DeviceScene::self), allocated when the context opens
     bool contacts = false;  // touching bodies or plates thinner than the FP32 anchor error
     // particles: the sky's share of the emitted power and the disc distant light leaves from
@@ -499,6 +501,7 @@ struct owec_ctx {
     double lastWalkSeconds = 0, lastAdjointSeconds = 0;
 
     CastWorker castWorkers[kCastWorkers];
+    cudaEvent_t castDone[2] = {nullptr, nullptr};
     DBuf<char> dCast;  // the chunks' rays and hits on the device
     char* hostBlock = nullptr;    // page-locked, kHostBlock bytes
     char* castStaging = nullptr;  // page-locked, a chunk per worker
@@ -1162,7 +1165,11 @@ void ensurePrims64(owec_ctx& c) {
 // as this returns.
 void publishScene(owec_ctx& c) {
     c.ds.self = c.dScene.get();
+    if (c.scenePublished && std::memcmp(&c.published, &c.ds, sizeof(DeviceScene)) == 0) return;  // nothing changed
+    c.scenePublished = false;
     OWEC_CUDA(cudaMemcpyAsync(c.dScene.get(), &c.ds, sizeof(DeviceScene), cudaMemcpyHostToDevice, c.stream));
+    std::memcpy(&c.published, &c.ds, sizeof(DeviceScene));
+    c.scenePublished = true;
 }
 
 void ensureReady(owec_ctx& c) {
@@ -1527,24 +1534,78 @@ void unpackHits(const char* host, uint64_t m, uint32_t* boundary, uint32_t* prim
     std::memcpy(prim, hits + 12 * m, 4 * m);
 }
 
+// Up to kCastSerial rays on the context's stream: packed into the two halves of its block in turn while the
+// other half is copied, traced by one launch, and unpacked the same way.
+template <int M>
+void castSerial(owec_ctx& c, uint64_t n, const double* o, const double* d, uint32_t* boundary, uint32_t* prim, double* t) {
+    constexpr size_t half = kCastPiece * kCastBytesPerRay;
+    constexpr uint64_t outPiece = half / 16;
+    char* staging = c.hostBlock + kHostReports;
+    c.dCast.reserve(n * kCastBytesPerRay);
+    char* dev = c.dCast.get();
+    char* hits = dev + 48 * n;  // n distances, n boundaries, n primitives
+    cudaStream_t s = c.stream;
+    auto upload = [&](size_t at, const char* host, size_t bytes) {
+        OWEC_CUDA(cudaMemcpyAsync(dev + at, host, bytes, cudaMemcpyHostToDevice, s));
+    };
+    for (uint64_t i = 0; i * kCastPiece < n; ++i) {
+        const uint64_t a = i * kCastPiece, m = std::min(kCastPiece, n - a);
+        char* host = staging + (i & 1) * half;
+        if (i >= 2) OWEC_CUDA(cudaEventSynchronize(c.castDone[i & 1]));
+        std::memcpy(host, o + 3 * a, 24 * m);
+        std::memcpy(host + 24 * m, d + 3 * a, 24 * m);
+        if (m == n) {
+            upload(0, host, 48 * n);
+        } else {
+            upload(24 * a, host, 24 * m);
+            upload(24 * (n + a), host + 24 * m, 24 * m);
+        }
+        OWEC_CUDA(cudaEventRecord(c.castDone[i & 1], s));
+    }
+    launchCastRays<M>(c.ds, n, reinterpret_cast<double*>(dev), reinterpret_cast<double*>(dev + 24 * n),
+                      reinterpret_cast<uint32_t*>(hits + 8 * n), reinterpret_cast<uint32_t*>(hits + 12 * n),
+                      reinterpret_cast<double*>(hits), c.numSMs * 8, s);
+    checkLaunch();
+    auto download = [&](char* host, size_t at, size_t bytes) {
+        OWEC_CUDA(cudaMemcpyAsync(host, hits + at, bytes, cudaMemcpyDeviceToHost, s));
+    };
+    const uint64_t pieces = (n + outPiece - 1) / outPiece;
+    auto unpack = [&](uint64_t i) {
+        const uint64_t a = i * outPiece, m = std::min(outPiece, n - a);
+        const char* host = staging + (i & 1) * half;
+        OWEC_CUDA(cudaEventSynchronize(c.castDone[i & 1]));
+        std::memcpy(t + a, host, 8 * m);
+        std::memcpy(boundary + a, host + 8 * m, 4 * m);
+        std::memcpy(prim + a, host + 12 * m, 4 * m);
+    };
+    for (uint64_t i = 0; i < pieces; ++i) {
+        const uint64_t a = i * outPiece, m = std::min(outPiece, n - a);
+        char* host = staging + (i & 1) * half;
+        if (i >= 2) unpack(i - 2);
+        if (m == n) {
+            download(host, 0, 16 * n);
+        } else {
+            download(host, 8 * a, 8 * m);
+            download(host + 8 * m, 8 * n + 4 * a, 4 * m);
+            download(host + 12 * m, 12 * n + 4 * a, 4 * m);
+        }
+        OWEC_CUDA(cudaEventRecord(c.castDone[i & 1], s));
+    }
+    if (pieces >= 2) unpack(pieces - 2);
+    unpack(pieces - 1);
+}
+
 // Host rays, a few on the context's stream, more in chunks by up to kCastWorkers host threads. Packing and
 // unpacking the 64 bytes of a ray on one core, the driver's own staging of pageable copies, the faults of
 // the results' fresh pages and five allocations a call took ten times the kernel's time (2^20 rays: 10.5 ms
-// around a 0.97 ms kernel; 4.2 ms so; chunks of 4096 rays, two to a thread in turn: 8.9 ms).
+// around a 0.97 ms kernel; 4.9 ms so; chunks of 4096 rays, two to a thread in turn: 8.9 ms).
 template <int M>
 void castRays(owec_ctx& c, uint64_t n, const double* o, const double* d, uint32_t* boundary, uint32_t* prim, double* t) {
-    const uint64_t chunks = (n + kCastChunk - 1) / kCastChunk;
-    if (chunks <= kCastSerial) {
-        char* staging = c.hostBlock + kHostReports;
-        c.dCast.reserve(std::min(n, kCastChunk) * kCastBytesPerRay);
-        for (uint64_t a = 0; a < n; a += kCastChunk) {
-            const uint64_t m = std::min(kCastChunk, n - a);
-            castChunk<M>(c, staging, c.dCast.get(), m, o + 3 * a, d + 3 * a, c.stream);
-            OWEC_CUDA(cudaStreamSynchronize(c.stream));
-            unpackHits(staging, m, boundary + a, prim + a, t + a);
-        }
+    if (n <= kCastSerial) {
+        castSerial<M>(c, n, o, d, boundary, prim, t);
         return;
     }
+    const uint64_t chunks = (n + kCastChunk - 1) / kCastChunk;
     constexpr int workers = kCastWorkers;
     constexpr size_t slot = kCastChunk * kCastBytesPerRay;
     if (!c.castStaging) OWEC_CUDA(cudaMallocHost(&c.castStaging, kCastWorkers * slot));
@@ -1651,15 +1712,13 @@ int owec_open(int device, owec_ctx** out) {
         OWEC_CUDA(cudaSetDevice(device));
         auto c = std::make_unique<owec_ctx>();
         c->device = device;
-        cudaDeviceProp prop;
-        OWEC_CUDA(cudaGetDeviceProperties(&prop, device));
-        c->numSMs = prop.multiProcessorCount;
-        std::snprintf(c->name, sizeof(c->name), "%s", prop.name);
+        OWEC_CUDA(cudaDeviceGetAttribute(&c->numSMs, cudaDevAttrMultiProcessorCount, device));
         OWEC_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
         OWEC_CUDA(cudaStreamCreateWithFlags(&c->shadowStream, cudaStreamNonBlocking));
         OWEC_CUDA(cudaEventCreateWithFlags(&c->eventsDone, cudaEventDisableTiming));
         OWEC_CUDA(cudaEventCreateWithFlags(&c->shadowDone, cudaEventDisableTiming));
         OWEC_CUDA(cudaEventCreateWithFlags(&c->generalDone, cudaEventDisableTiming));
+        for (cudaEvent_t& e : c->castDone) OWEC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         OWEC_CUDA(cudaEventCreate(&c->passStart));
         OWEC_CUDA(cudaEventCreate(&c->passStop));
         OWEC_CUDA(cudaMallocHost(&c->hostBlock, kHostBlock));
@@ -1689,6 +1748,7 @@ int owec_close(owec_ctx* ctx) {
         cudaEventDestroy(ctx->eventsDone);
         cudaEventDestroy(ctx->shadowDone);
         cudaEventDestroy(ctx->generalDone);
+        for (cudaEvent_t e : ctx->castDone) cudaEventDestroy(e);
         cudaStreamDestroy(ctx->shadowStream);
         cudaEventDestroy(ctx->passStart);
         cudaEventDestroy(ctx->passStop);
@@ -1703,6 +1763,11 @@ int owec_close(owec_ctx* ctx) {
 int owec_device_name(owec_ctx* ctx, char* buf, size_t len) {
     return guarded([&] {
         require(ctx && buf && len > 0, "owec_device_name: bad arguments");
+        if (!ctx->name[0]) {  // asked for here: the device's properties take 2.4 ms, most of opening a context
+            cudaDeviceProp prop;
+            OWEC_CUDA(cudaGetDeviceProperties(&prop, ctx->device));
+            std::snprintf(ctx->name, sizeof(ctx->name), "%s", prop.name);
+        }
         std::snprintf(buf, len, "%s", ctx->name);
     });
 }
@@ -1937,7 +2002,6 @@ int owec_reset_film(owec_ctx* ctx) {
             if (b->size()) OWEC_CUDA(cudaMemsetAsync(b->get(), 0, b->bytes(), ctx->stream));
         if (ctx->dSplat.size()) OWEC_CUDA(cudaMemsetAsync(ctx->dSplat.get(), 0, ctx->dSplat.bytes(), ctx->stream));
         OWEC_CUDA(cudaMemsetAsync(ctx->dStats.get(), 0, sizeof(StatCounters), ctx->stream));
-        OWEC_CUDA(cudaStreamSynchronize(ctx->stream));
     });
 }
 

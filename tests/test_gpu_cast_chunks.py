@@ -10,7 +10,7 @@ import scenes
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 255, 16384, 16385, 16 * 16384, 16 * 16384 + 1, 300001])
+@pytest.mark.parametrize("n", [1, 255, 4096, 4097, 8193, 16385, 40000, 16 * 4096, 16 * 4096 + 1, 5 * 16384, 300001])
 def test_batches_match_their_rays_in_small_calls(n):
     desc = scenes.bvh_stress_room(16, 16, 64, 32).desc()
     o, d = scenes.random_rays(n, 5, (-2.5, -2.5, 0.3), (2.5, 2.5, 3.7), (-1.2, -1.2, 0.1), (1.2, 1.2, 2.4))
