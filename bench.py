@@ -214,7 +214,9 @@ def precision_study(device, ref_rows=16, ref_spp=1024, spp=16, bias_spp=256):
     transport statistics. speedup_at_equal_relmse: FP64's seconds to that relMSE over the mode's."""
     import owe_cuda
     sys.path.insert(0, os.path.join(ROOT, "tests"))
-    from oracle_ref import ReferenceEngine  # the FP64 oracle image, not a timed leg
+    from oracle_ref import REF_LIB, ReferenceEngine  # the FP64 oracle image, not a timed leg
+    if not os.path.exists(REF_LIB):
+        return {"unavailable": "the reference engine is not built"}
     desc = scenes.bvh_stress_room(WIDTH, HEIGHT).desc()
     r0 = HEIGHT // 2 - ref_rows // 2
     t0 = time.perf_counter()
