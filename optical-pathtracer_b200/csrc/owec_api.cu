@@ -2192,6 +2192,7 @@ int owec_walk_resolve(owec_ctx* ctx, double* bins, owec_walk_stats* stats) {
     return guarded([&] {
         require(ctx != nullptr, "owec_walk_resolve: null context");
         require(ctx->hasWalk, "no walks run", OWEC_E_STATE);
+        OWEC_CUDA(cudaSetDevice(ctx->device));
         const owec_walk_desc& w = ctx->walk;
         const size_t nb = size_t(w.width) * w.height;
         unsigned long long st[kWalkStats];
