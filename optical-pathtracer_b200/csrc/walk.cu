@@ -362,10 +362,16 @@ __device__ __forceinline__ WalkEnd walkEvent(const DeviceScene& sc, const WalkPa
     }
 }
 
-// Threads of a block: one block fills an SM's registers (128 each with a little spilling in the lean
-// kernels, 255 in the Full ones, which spill far more below that).
+// Threads of a block, one block to an SM: 512 of 128 registers for the lean kernels, which spill a little, and
+// 384 of 168 for the Full ones, whose numeric roots need more. 2.1 M walks through the achromat with a cone in
+// its scene (Full), mixed / FP32 / FP64: 256 threads 6.75 / 6.31 / 7.93 ms (bounded by threads alone the
+// compiler stops at 128 registers in FP32; told that one block is resident, 255: 6.56 / 5.88 / 7.96), 320 6.39 /
+// 5.68 / 7.66, 384 5.35 / 4.75 / 6.58, 512 5.18 / 4.04 / 6.97. The slab with the cone, 1 M walks, forward 2.68 /
+// 2.95 / 2.94 at 256, 2.33 / 1.90 / 2.75 at 384, 2.64 / 1.86 / 2.87 at 512, adjoint 3.03 / 3.46 / 3.57, 2.91 /
+// 2.25 / 3.18 and 3.26 / 2.22 / 3.42: 384 is the only one that loses nowhere to the unrefilled kernel's
+// 128-thread blocks (slab in FP32 2.20).
 template <bool Full>
-constexpr int kWalkBlock = Full ? 256 : 512;
+constexpr int kWalkBlock = Full ? 384 : 512;
 
 // Adds a per-lane count to a counter, one atomic per warp (all lanes of the warp present).
 __device__ __forceinline__ void flushCount(unsigned long long* counter, uint32_t v) {
@@ -384,7 +390,7 @@ __device__ __forceinline__ void flushCount(unsigned long long* counter, uint32_t
 // 5.30. Two blocks of 256 in step 9.0, 4.19 and 5.56 ms, four of 128 9.9, 4.25 and 6.12; refilling only when 8
 // lanes are idle 22 ms for the lens.
 template <int M, bool ADJ, bool Full>
-__global__ void __launch_bounds__(kWalkBlock<Full>) kWalk(DeviceScene sc, WalkParams P, unsigned long long* bins,
+__global__ void __launch_bounds__(kWalkBlock<Full>, 1) kWalk(DeviceScene sc, WalkParams P, unsigned long long* bins,
                                                           unsigned long long* stats, const double* g, double* dH,
                                                           unsigned long long* fetch) {
     extern __shared__ StackEntry stackMem[];
