@@ -8,6 +8,7 @@
 #include <sys/mman.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <exception>
@@ -23,6 +24,7 @@
 #include "spectral.cuh"
 #include "path_adjoint.hpp"
 #include "peaks.hpp"
+#include "phased_workers.hpp"
 #include "walk.hpp"
 #include "wavefront.hpp"
 
@@ -368,23 +370,20 @@ void invertRigid(const double m[12], double out[12]) {
 }  // namespace
 
 // ------------------------------------------------------------------ the context
-// owec_cast_rays: a small call goes through the context's own page-locked block, which is small enough to
-// share the runtime's 2 MB page-locked granules with other contexts' (a granule costs 1 to 3 ms); a larger
-// one through kCastWorkers host threads with a chunk each, staged in a block that the first such call makes.
+// owec_cast_rays: rays travel in pieces through page-locked slots, up to kCastSerial of them by the calling
+// thread, more by up to kCastWorkers host threads with a slot each. The calling thread's slot lies in the
+// context's own block; the others' are made by the first such call. Together they fit a 2 MB granule of the
+// runtime's page-locked memory, which takes 2 to 4 ms to make (4 MB of staging made the first call of 70,000
+// rays 6.3 ms, against 2.6 without any).
 constexpr int kCastWorkers = 4;
-constexpr uint64_t kCastPiece = 4096, kCastSerial = 16 * kCastPiece, kCastChunk = 16384;
-constexpr size_t kCastBytesPerRay = 48 + 16;
+constexpr int kCastPieceShift = 13, kCastSerialPieceShift = 12;  // rays of a piece, as powers of two
+constexpr uint64_t kCastSerial = 65536;
+constexpr uint64_t kCastKept = 1ull << 21, kCastBatch = 1ull << 24;  // see castRays
+constexpr size_t kCastSlot = (size_t(1) << kCastPieceShift) * 48;
+constexpr int kCastGroups = 4;  // launches of a batch at most, of at least kCastGroupPieces pieces each
+constexpr uint64_t kCastGroupPieces = 8;
 constexpr size_t kHostReports = 4096;  // the context block's first part: what kernels report to the host
-constexpr size_t kHostBlock = kHostReports + 2 * kCastPiece * kCastBytesPerRay;
-struct CastWorker {
-    cudaStream_t stream = nullptr;
-    void ensure() {
-        if (!stream) OWEC_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    }
-    ~CastWorker() {
-        if (stream) cudaStreamDestroy(stream);
-    }
-};
+constexpr size_t kHostBlock = kHostReports + kCastSlot;
 
 struct owec_ctx {
     int device = 0;
@@ -500,11 +499,12 @@ struct owec_ctx {
     std::vector<MeshCopy> meshes;    // per boundary (empty for analytic ones)
     double lastWalkSeconds = 0, lastAdjointSeconds = 0;
 
-    CastWorker castWorkers[kCastWorkers];
-    cudaEvent_t castDone[2] = {nullptr, nullptr};
-    DBuf<char> dCast;  // the chunks' rays and hits on the device
+    cudaEvent_t castDone[kCastWorkers][2] = {};  // the copies of the two halves of a worker's slot
+    cudaEvent_t castUp[kCastGroups] = {}, castTraced[kCastGroups] = {};  // a group's rays there, its hits there
+    cudaStream_t castStreams[kCastGroups - 1] = {};  // trace the groups but the first, the shadow stream that one
+    DBuf<char> dCast;             // rays and hits on the device, up to kCastKept of them
     char* hostBlock = nullptr;    // page-locked, kHostBlock bytes
-    char* castStaging = nullptr;  // page-locked, a chunk per worker
+    char* castStaging = nullptr;  // page-locked, a slot per worker but the first
 
     // forward light walks
     owec_walk_desc walk{};
@@ -1519,131 +1519,178 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
     return hs.paths;
 }
 
-// m rays packed into `host` (origins, directions; the hits behind them), one copy each way, queued on s.
-template <int M>
-void castChunk(const owec_ctx& c, char* host, char* device, uint64_t m, const double* o, const double* d, cudaStream_t s) {
-    std::memcpy(host, o, 24 * m);
-    std::memcpy(host + 24 * m, d, 24 * m);
-    char* hits = device + 48 * m;
-    OWEC_CUDA(cudaMemcpyAsync(device, host, 48 * m, cudaMemcpyHostToDevice, s));
-    launchCastRays<M>(c.ds, m, reinterpret_cast<double*>(device), reinterpret_cast<double*>(device + 24 * m),
-                      reinterpret_cast<uint32_t*>(hits + 8 * m), reinterpret_cast<uint32_t*>(hits + 12 * m),
-                      reinterpret_cast<double*>(hits), c.numSMs * 8, s);
-    checkLaunch();
-    OWEC_CUDA(cudaMemcpyAsync(host + 48 * m, hits, 16 * m, cudaMemcpyDeviceToHost, s));
-}
-void unpackHits(const char* host, uint64_t m, uint32_t* boundary, uint32_t* prim, double* t) {
-    const char* hits = host + 48 * m;
-    std::memcpy(t, hits, 8 * m);
-    std::memcpy(boundary, hits + 8 * m, 4 * m);
-    std::memcpy(prim, hits + 12 * m, 4 * m);
+// Share k of n of a result buffer's whole pages, faulted in while the rays are traced (a kernel without the advice
+// faults them in under the workers' copies). What the pages hold stays: a worker done with its share may already be
+// writing hits into another's.
+void populateShare(void* dst, size_t bytes, size_t k, size_t n) {
+    constexpr size_t kPage = 4096;
+    char* first = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(dst) + kPage - 1) & ~uintptr_t(kPage - 1));
+    char* end = static_cast<char*>(dst) + bytes;
+    if (end <= first) return;
+    const size_t pages = size_t(end - first) / kPage, from = pages * k / n, to = pages * (k + 1) / n;
+    if (from < to) (void)madvise(first + from * kPage, (to - from) * kPage, MADV_POPULATE_WRITE);
 }
 
-// Up to kCastSerial rays on the context's stream: packed into the two halves of its block in turn while the
-// other half is copied, traced by one launch, and unpacked the same way.
-template <int M>
-void castSerial(owec_ctx& c, uint64_t n, const double* o, const double* d, uint32_t* boundary, uint32_t* prim, double* t) {
-    constexpr size_t half = kCastPiece * kCastBytesPerRay;
-    constexpr uint64_t outPiece = half / 16;
-    char* staging = c.hostBlock + kHostReports;
-    c.dCast.reserve(n * kCastBytesPerRay);
-    char* dev = c.dCast.get();
-    char* hits = dev + 48 * n;  // n distances, n boundaries, n primitives
-    cudaStream_t s = c.stream;
-    auto upload = [&](size_t at, const char* host, size_t bytes) {
-        OWEC_CUDA(cudaMemcpyAsync(dev + at, host, bytes, cudaMemcpyHostToDevice, s));
-    };
-    for (uint64_t i = 0; i * kCastPiece < n; ++i) {
-        const uint64_t a = i * kCastPiece, m = std::min(kCastPiece, n - a);
-        char* host = staging + (i & 1) * half;
-        if (i >= 2) OWEC_CUDA(cudaEventSynchronize(c.castDone[i & 1]));
-        std::memcpy(host, o + 3 * a, 24 * m);
-        std::memcpy(host + 24 * m, d + 3 * a, 24 * m);
-        if (m == n) {
-            upload(0, host, 48 * n);
-        } else {
-            upload(24 * a, host, 24 * m);
-            upload(24 * (n + a), host + 24 * m, 24 * m);
-        }
-        OWEC_CUDA(cudaEventRecord(c.castDone[i & 1], s));
-    }
-    launchCastRays<M>(c.ds, n, reinterpret_cast<double*>(dev), reinterpret_cast<double*>(dev + 24 * n),
-                      reinterpret_cast<uint32_t*>(hits + 8 * n), reinterpret_cast<uint32_t*>(hits + 12 * n),
-                      reinterpret_cast<double*>(hits), c.numSMs * 8, s);
-    checkLaunch();
-    auto download = [&](char* host, size_t at, size_t bytes) {
-        OWEC_CUDA(cudaMemcpyAsync(host, hits + at, bytes, cudaMemcpyDeviceToHost, s));
-    };
-    const uint64_t pieces = (n + outPiece - 1) / outPiece;
-    auto unpack = [&](uint64_t i) {
-        const uint64_t a = i * outPiece, m = std::min(outPiece, n - a);
-        const char* host = staging + (i & 1) * half;
-        OWEC_CUDA(cudaEventSynchronize(c.castDone[i & 1]));
-        std::memcpy(t + a, host, 8 * m);
-        std::memcpy(boundary + a, host + 8 * m, 4 * m);
-        std::memcpy(prim + a, host + 12 * m, 4 * m);
-    };
-    for (uint64_t i = 0; i < pieces; ++i) {
-        const uint64_t a = i * outPiece, m = std::min(outPiece, n - a);
-        char* host = staging + (i & 1) * half;
-        if (i >= 2) unpack(i - 2);
-        if (m == n) {
-            download(host, 0, 16 * n);
-        } else {
-            download(host, 8 * a, 8 * m);
-            download(host + 8 * m, 8 * n + 4 * a, 4 * m);
-            download(host + 12 * m, 12 * n + 4 * a, 4 * m);
-        }
-        OWEC_CUDA(cudaEventRecord(c.castDone[i & 1], s));
-    }
-    if (pieces >= 2) unpack(pieces - 2);
-    unpack(pieces - 1);
-}
+// One batch of host rays: pieces of 2^shift rays, dealt to the workers as they come for them and traced by the
+// group. A piece travels to the device as its origins and then its directions, its hits come back as distances,
+// boundaries, primitives (CastPieces, the layout launchCastRays reads and writes).
+struct CastBatch {
+    uint64_t n;
+    const double *o, *d;
+    uint32_t *boundary, *prim;
+    double* t;
+    char* device;
+    int shift;
+    uint64_t groupPieces;
+    std::atomic<uint64_t> up{0}, down{0}, queued[kCastGroups]{};
+    uint64_t pieces() const { return (n + (1ull << shift) - 1) >> shift; }
+    uint64_t groups() const { return (pieces() + groupPieces - 1) / groupPieces; }
+    char* hits() const { return device + 48 * n; }
+};
 
-// Host rays, a few on the context's stream, more in chunks by up to kCastWorkers host threads. Packing and
-// unpacking the 64 bytes of a ray on one core, the driver's own staging of pageable copies, the faults of
-// the results' fresh pages and five allocations a call took ten times the kernel's time (2^20 rays: 10.5 ms
-// around a 0.97 ms kernel; 4.9 ms so; chunks of 4096 rays, two to a thread in turn: 8.9 ms).
+// Group g's rays are all queued: its trace.
 template <int M>
-void castRays(owec_ctx& c, uint64_t n, const double* o, const double* d, uint32_t* boundary, uint32_t* prim, double* t) {
-    if (n <= kCastSerial) {
-        castSerial<M>(c, n, o, d, boundary, prim, t);
+void traceGroup(owec_ctx& c, CastBatch& b, uint64_t g) {
+    const uint64_t first = g * b.groupPieces << b.shift, n = std::min(b.groupPieces << b.shift, b.n - first);
+    const CastPieces pieces{n, b.device + 48 * first, b.hits() + 16 * first, b.shift};
+    if (b.groups() == 1) {
+        launchCastRays<M>(c.ds, pieces, c.numSMs * 8, c.stream);
+        checkLaunch();
         return;
     }
-    const uint64_t chunks = (n + kCastChunk - 1) / kCastChunk;
-    constexpr int workers = kCastWorkers;
-    constexpr size_t slot = kCastChunk * kCastBytesPerRay;
-    if (!c.castStaging) OWEC_CUDA(cudaMallocHost(&c.castStaging, kCastWorkers * slot));
-    c.dCast.reserve(kCastWorkers * slot);
-    for (int k = 0; k < workers; ++k) c.castWorkers[k].ensure();
-    OWEC_CUDA(cudaStreamSynchronize(c.stream));  // the workers' streams read what it published
-    std::exception_ptr failed[kCastWorkers];
-    auto work = [&](int k) {
-        cudaStream_t s = c.castWorkers[k].stream;
-        char* host = c.castStaging + size_t(k) * slot;
-        try {
-            OWEC_CUDA(cudaSetDevice(c.device));
-            for (uint64_t i = uint64_t(k); i < chunks; i += uint64_t(workers)) {
-                const uint64_t a = i * kCastChunk, m = std::min(kCastChunk, n - a);
-                castChunk<M>(c, host, c.dCast.get() + size_t(k) * slot, m, o + 3 * a, d + 3 * a, s);
-                OWEC_CUDA(cudaStreamSynchronize(s));
-                unpackHits(host, m, boundary + a, prim + a, t + a);
-            }
-        } catch (...) {
-            failed[k] = std::current_exception();
-            cudaStreamSynchronize(s);  // nothing of a failed worker is left in flight
-        }
-    };
-    {
-        struct Joined {
-            std::vector<std::thread> threads;
-            ~Joined() { for (std::thread& th : threads) th.join(); }
-        } joined;
-        for (int k = 1; k < workers; ++k) joined.threads.emplace_back(work, k);
-        work(0);
+    const cudaStream_t s = g ? c.castStreams[g - 1] : c.shadowStream;
+    OWEC_CUDA(cudaEventRecord(c.castUp[g], c.stream));
+    OWEC_CUDA(cudaStreamWaitEvent(s, c.castUp[g], 0));
+    launchCastRays<M>(c.ds, pieces, c.numSMs * 4, s);
+    checkLaunch();
+    OWEC_CUDA(cudaEventRecord(c.castTraced[g], s));
+}
+
+template <int M>
+void uploadPieces(owec_ctx& c, CastBatch& b, int worker, char* slot) {
+    const uint64_t piece = 1ull << b.shift, pieces = b.pieces();
+    const int slots = int(kCastSlot / (48 * piece));  // one or two
+    uint64_t k = 0;
+    for (uint64_t i; (i = b.up.fetch_add(1)) < pieces; ++k) {
+        const uint64_t a = i << b.shift, m = std::min(piece, b.n - a), g = i / b.groupPieces;
+        const int j = int(k % uint64_t(slots));
+        char* host = slot + size_t(j) * 48 * piece;
+        if (k >= uint64_t(slots)) OWEC_CUDA(cudaEventSynchronize(c.castDone[worker][j]));
+        std::memcpy(host, b.o + 3 * a, 24 * m);
+        std::memcpy(host + 24 * m, b.d + 3 * a, 24 * m);
+        OWEC_CUDA(cudaMemcpyAsync(b.device + 48 * a, host, 48 * m, cudaMemcpyHostToDevice, c.stream));
+        OWEC_CUDA(cudaEventRecord(c.castDone[worker][j], c.stream));
+        // the worker that queues a group's last piece has it traced
+        if (b.queued[g].fetch_add(1) + 1 == std::min(b.groupPieces, pieces - g * b.groupPieces)) traceGroup<M>(c, b, g);
     }
-    for (const std::exception_ptr& e : failed)
-        if (e) std::rethrow_exception(e);
+}
+
+// The hits, as many pieces at a time as half a slot holds, one half unpacked while the other is copied.
+void downloadPieces(owec_ctx& c, CastBatch& b, int worker, char* slot) {
+    const uint64_t piece = 1ull << b.shift, run = kCastSlot / 2 / (16 * piece);
+    uint64_t held = 0, traced = ~0ull;
+    bool any = false;
+    for (uint64_t k = 0;; ++k) {
+        const uint64_t i = b.down.fetch_add(run), a = i << b.shift;
+        const bool more = a < b.n;
+        if (more) {
+            const uint64_t g = i / b.groupPieces;
+            if (b.groups() > 1 && g != traced) OWEC_CUDA(cudaStreamWaitEvent(c.stream, c.castTraced[g], 0));
+            traced = g;
+            OWEC_CUDA(cudaMemcpyAsync(slot + (k & 1) * (kCastSlot / 2), b.hits() + 16 * a,
+                                      16 * std::min(run << b.shift, b.n - a), cudaMemcpyDeviceToHost, c.stream));
+            OWEC_CUDA(cudaEventRecord(c.castDone[worker][k & 1], c.stream));
+        }
+        if (any) {
+            OWEC_CUDA(cudaEventSynchronize(c.castDone[worker][(k - 1) & 1]));
+            const char* host = slot + ((k - 1) & 1) * (kCastSlot / 2);
+            for (uint64_t p = held; p < std::min(held + (run << b.shift), b.n); p += piece) {
+                const uint64_t m = std::min(piece, b.n - p);
+                std::memcpy(b.t + p, host, 8 * m);
+                std::memcpy(b.boundary + p, host + 8 * m, 4 * m);
+                std::memcpy(b.prim + p, host + 12 * m, 4 * m);
+                host += 16 * m;
+            }
+        }
+        if (!more) return;
+        held = a;
+        any = true;
+    }
+}
+
+template <int M>
+void castBatch(owec_ctx& c, CastBatch& b, int workers) {
+    char* const own = c.hostBlock + kHostReports;
+    if (workers == 1) {
+        uploadPieces<M>(c, b, 0, own);
+        downloadPieces(c, b, 0, own);
+        return;
+    }
+    // hits are unpacked once all rays are packed: a program may have them overwrite its rays
+    PhasedWorkers gang(workers);
+    gang.run(
+        [&](int k) {
+            if (k) OWEC_CUDA(cudaSetDevice(c.device));
+            uploadPieces<M>(c, b, k, k ? c.castStaging + size_t(k - 1) * kCastSlot : own);
+        },
+        [&](int k, int n) {
+            populateShare(b.t, 8 * b.n, size_t(k), size_t(n));
+            populateShare(b.boundary, 4 * b.n, size_t(k), size_t(n));
+            populateShare(b.prim, 4 * b.n, size_t(k), size_t(n));
+            downloadPieces(c, b, k, k ? c.castStaging + size_t(k - 1) * kCastSlot : own);
+        });
+}
+
+// The slots, events and stream that a call with several workers needs besides; false where they cannot be had.
+bool castStagingReady(owec_ctx& c) {
+    if (c.castStaging) return true;
+    auto event = [](cudaEvent_t& e) {
+        if (!e) OWEC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    };
+    for (int k = 1; k < kCastWorkers; ++k)
+        for (cudaEvent_t& e : c.castDone[k]) event(e);
+    for (int g = 0; g < kCastGroups; ++g) {
+        event(c.castUp[g]);
+        event(c.castTraced[g]);
+    }
+    for (cudaStream_t& s : c.castStreams)
+        if (!s) OWEC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    if (cudaMallocHost(&c.castStaging, size_t(kCastWorkers - 1) * kCastSlot) == cudaSuccess) return true;
+    cudaGetLastError();
+    c.castStaging = nullptr;
+    return false;
+}
+
+// Host rays: packed and copied by the workers, traced by the group, copied back and unpacked. One core's packing
+// of a ray's 64 bytes, the driver's own staging of pageable copies, the faults of the results' fresh pages and
+// five allocations a call took ten times the kernel's time (2^20 rays into the room of 2^18 triangles: 10.5 ms
+// around a 0.97 ms kernel). The groups' launches, each on its own stream, overlap the copies and each other's
+// last rays, and each has the rays to fill the GPU: launches of 16,384 rays, one after another on four streams,
+// left most of it idle where the tracing is the longer part (2^20 rays into the FP32 wave pool: 50.3 ms, against
+// 23.6 in one launch). Device memory for
+// up to kCastKept rays (128 MB) stays with the context; larger calls allocate theirs, for kCastBatch rays
+// (1 GB) at a time.
+template <int M>
+void castRays(owec_ctx& c, uint64_t n, const double* o, const double* d, uint32_t* boundary, uint32_t* prim, double* t) {
+    const uint64_t batch = std::min(n, kCastBatch);
+    DBuf<char> large;
+    DBuf<char>& buf = batch <= kCastKept ? c.dCast : large;
+    buf.reserve(64 * batch);
+    const int workers = batch > kCastSerial && castStagingReady(c) ? kCastWorkers : 1;
+    const int shift = workers == 1 ? kCastSerialPieceShift : kCastPieceShift;
+    for (uint64_t a = 0; a < n; a += batch) {
+        CastBatch b{std::min(batch, n - a), o + 3 * a, d + 3 * a, boundary + a, prim + a, t + a, buf.get(), shift, 0};
+        const uint64_t groups = workers == 1 ? 1 : std::max<uint64_t>(1, std::min<uint64_t>(kCastGroups, b.pieces() / kCastGroupPieces));
+        b.groupPieces = (b.pieces() + groups - 1) / groups;
+        try {
+            castBatch<M>(c, b, workers);
+        } catch (...) {  // nothing of a failed call is left in flight
+            for (cudaStream_t s : {c.stream, c.shadowStream}) cudaStreamSynchronize(s);
+            for (cudaStream_t s : c.castStreams)
+                if (s) cudaStreamSynchronize(s);
+            throw;
+        }
+    }
 }
 
 // The pages of a large result buffer touched by several threads where most of them are not yet resident: a
@@ -1723,7 +1770,7 @@ int owec_open(int device, owec_ctx** out) {
         OWEC_CUDA(cudaEventCreateWithFlags(&c->eventsDone, cudaEventDisableTiming));
         OWEC_CUDA(cudaEventCreateWithFlags(&c->shadowDone, cudaEventDisableTiming));
         OWEC_CUDA(cudaEventCreateWithFlags(&c->generalDone, cudaEventDisableTiming));
-        for (cudaEvent_t& e : c->castDone) OWEC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        for (cudaEvent_t& e : c->castDone[0]) OWEC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         OWEC_CUDA(cudaEventCreate(&c->passStart));
         OWEC_CUDA(cudaEventCreate(&c->passStop));
         OWEC_CUDA(cudaMallocHost(&c->hostBlock, kHostBlock));
@@ -1753,7 +1800,14 @@ int owec_close(owec_ctx* ctx) {
         cudaEventDestroy(ctx->eventsDone);
         cudaEventDestroy(ctx->shadowDone);
         cudaEventDestroy(ctx->generalDone);
-        for (cudaEvent_t e : ctx->castDone) cudaEventDestroy(e);
+        for (auto& pair : ctx->castDone)
+            for (cudaEvent_t e : pair)
+                if (e) cudaEventDestroy(e);
+        for (int g = 0; g < kCastGroups; ++g)
+            for (cudaEvent_t e : {ctx->castUp[g], ctx->castTraced[g]})
+                if (e) cudaEventDestroy(e);
+        for (cudaStream_t s : ctx->castStreams)
+            if (s) cudaStreamDestroy(s);
         cudaStreamDestroy(ctx->shadowStream);
         cudaEventDestroy(ctx->passStart);
         cudaEventDestroy(ctx->passStop);

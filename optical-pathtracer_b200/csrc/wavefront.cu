@@ -1022,20 +1022,25 @@ __device__ __forceinline__ void castQueries(const DeviceScene& sc, uint64_t n, c
 }
 
 template <int M, bool Full>
-__global__ void OWEC_TRAVERSAL_BOUNDS kCastRays(DeviceScene sc, uint64_t n, const double* o, const double* d, uint32_t* boundary,
-                                                uint32_t* prim, double* t) {
+__global__ void OWEC_TRAVERSAL_BOUNDS kCastRays(DeviceScene sc, CastPieces b) {
     using R = RT<M>;
-    auto origin = [&](uint64_t i) {
-        const V3<double> od(o[3 * i] - sc.origin[0], o[3 * i + 1] - sc.origin[1], o[3 * i + 2] - sc.origin[2]);
-        return Mode<M>::plainOrigin ? V3<double>(V3<float>(od)) : od;
+    // ray i's origin and direction, in its piece of the batch
+    auto ray = [&](uint64_t i, V3<double>& od, V3<double>& d) {
+        const uint64_t first = i >> b.shift << b.shift, left = b.n - first, piece = 1ull << b.shift;
+        const double* o = reinterpret_cast<const double*>(b.rays + 48 * first) + 3 * (i - first);
+        const double* v = o + 3 * (left < piece ? left : piece);
+        od = V3<double>(o[0] - sc.origin[0], o[1] - sc.origin[1], o[2] - sc.origin[2]);
+        if (Mode<M>::plainOrigin) od = V3<double>(V3<float>(od));
+        d = V3<double>(v[0], v[1], v[2]);
     };
     castQueries<R, typename Mode<M>::Ro, typename Mode<M>::Rr, Full>(
-        sc, n,
+        sc, b.n,
         [&](uint64_t i) {
             RayQuery<R> rq;
-            rq.od = origin(i);
+            V3<double> d;
+            ray(i, rq.od, d);
             rq.o = V3<R>(rq.od);
-            rq.d = V3<R>(R(d[3 * i]), R(d[3 * i + 1]), R(d[3 * i + 2]));
+            rq.d = V3<R>(d);
             rq.tmax = R(INFINITY);
             rq.depB = rq.depP = kNone;
             rq.region = kNone;
@@ -1043,16 +1048,19 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kCastRays(DeviceScene sc, uint64_t n, cons
             return rq;
         },
         [&](uint64_t i, int s, const HitRec& h) {
-            if (s == kTraceHit) {
-                boundary[i] = h.boundary;
-                prim[i] = h.prim;
-                const bool refine = sizeof(typename Mode<M>::Rr) == sizeof(double) && sc.boundaries[h.boundary].shape == OWEC_SHAPE_MESH;
-                t[i] = refine ? refineTriangleT(sc, h.slot, origin(i), V3<double>(d[3 * i], d[3 * i + 1], d[3 * i + 2]), h.t) : h.t;
-            } else {
-                boundary[i] = s == kTraceOverflow ? kNone - 1u : kNone;
-                prim[i] = 0;
-                t[i] = INFINITY;
+            const bool hit = s == kTraceHit;
+            double t = hit ? h.t : INFINITY;
+            if (hit && sizeof(typename Mode<M>::Rr) == sizeof(double) && sc.boundaries[h.boundary].shape == OWEC_SHAPE_MESH) {
+                V3<double> od, d;
+                ray(i, od, d);
+                t = refineTriangleT(sc, h.slot, od, d, h.t);
             }
+            const uint64_t first = i >> b.shift << b.shift, left = b.n - first, piece = 1ull << b.shift;
+            const uint64_t k = i - first, m = left < piece ? left : piece;
+            char* out = b.hits + 16 * first;
+            reinterpret_cast<double*>(out)[k] = t;
+            reinterpret_cast<uint32_t*>(out + 8 * m)[k] = hit ? h.boundary : (s == kTraceOverflow ? kNone - 1u : kNone);
+            reinterpret_cast<uint32_t*>(out + 12 * m)[k] = hit ? h.prim : 0u;
         });
 }
 
@@ -1212,11 +1220,10 @@ void launchFilm(const DeviceScene& sc, const PassParams& pp, const PathBuffers<R
 }
 static int castGrid(uint64_t n, int grid) { return int(std::min<uint64_t>(uint64_t(grid), (n + 127) / 128)); }
 template <int M>
-void launchCastRays(const DeviceScene& sc, uint64_t n, const double* o, const double* d, uint32_t* b, uint32_t* p,
-                    double* t, int grid, cudaStream_t s) {
-    grid = castGrid(n, grid);
-    if (sc.fullFeatures) kCastRays<M, true><<<grid, 128, traversalSharedBytes(128), s>>>(sc, n, o, d, b, p, t);
-    else kCastRays<M, false><<<grid, 128, persistentSharedBytes<M>(128), s>>>(sc, n, o, d, b, p, t);
+void launchCastRays(const DeviceScene& sc, const CastPieces& b, int grid, cudaStream_t s) {
+    grid = castGrid(b.n, grid);
+    if (sc.fullFeatures) kCastRays<M, true><<<grid, 128, traversalSharedBytes(128), s>>>(sc, b);
+    else kCastRays<M, false><<<grid, 128, persistentSharedBytes<M>(128), s>>>(sc, b);
 }
 void launchCastRaysF(const DeviceScene& sc, uint64_t n, const float* o, const float* d, uint32_t* b, uint32_t* p,
                      float* t, int grid, cudaStream_t s) {
@@ -1247,8 +1254,7 @@ void launchMaterialize(const uint32_t* leafOrder, uint32_t n, const float4* tri,
                                    StatCounters*, uint8_t*, const SplatTarget&, int, cudaStream_t);                 \
     template void launchFilm<M>(const DeviceScene&, const PassParams&, const PathBuffers<RT<M>>&, double*, double*,  \
                                 double*, uint32_t, cudaStream_t);                                                   \
-    template void launchCastRays<M>(const DeviceScene&, uint64_t, const double*, const double*, uint32_t*,          \
-                                    uint32_t*, double*, int, cudaStream_t);
+    template void launchCastRays<M>(const DeviceScene&, const CastPieces&, int, cudaStream_t);
 
 OWEC_INSTANTIATE(0)
 OWEC_INSTANTIATE(1)

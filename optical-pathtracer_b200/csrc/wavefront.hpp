@@ -40,9 +40,17 @@ void launchFoldFilm(const double* film, const double* comp, double* out, size_t 
 template <int M>
 void launchFilm(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, double* film, double* comp,
                 double* samples, uint32_t spp, cudaStream_t);
+// n rays in device memory in pieces of 2^shift (the last one shorter): a piece of m rays from ray `first` on is m
+// origins and m directions (world, FP64) at rays + 48 first, and its hits m distances, m boundaries and m
+// primitives at hits + 16 first.
+struct CastPieces {
+    uint64_t n;
+    const char* rays;
+    char* hits;
+    int shift;
+};
 template <int M>
-void launchCastRays(const DeviceScene&, uint64_t n, const double* o, const double* d, uint32_t* b, uint32_t* p,
-                    double* t, int grid, cudaStream_t);
+void launchCastRays(const DeviceScene&, const CastPieces&, int grid, cudaStream_t);
 void launchCastRaysF(const DeviceScene&, uint64_t n, const float* o, const float* d, uint32_t* b, uint32_t* p, float* t,
                      int grid, cudaStream_t);
 void launchMaterialize(const uint32_t* leafOrder, uint32_t n, const float4* tri, const double* tri64, PrimRec* prims,
