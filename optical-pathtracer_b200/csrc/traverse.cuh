@@ -74,6 +74,9 @@ struct HitRec {
     uint32_t slot;        // leaf-order primitive slot
     uint32_t flags;       // kHitFront, kHitAmbiguous (kept by the contact-resolving traversal only)
 };
+// What FP64 rays' slab tests read from the record: the inverse direction (intersectChildren).
+template <class T> struct SlabRay {};
+template <> struct SlabRay<double> { double inv[3], pad; };
 // The part of a query that the node loop does not touch: what a primitive test, an accepted
 // crossing or the query's end needs. The persistent kernels keep it in shared memory, one record per
 // thread, which leaves the registers to the node test (at 128 registers kIntersect's spill stores go
@@ -81,7 +84,7 @@ struct HitRec {
 // blocks still spill in the node loop and run 10 to 18 % slower). The record is an odd number of
 // 8-byte words, so that a warp's accesses to one field spread over the banks.
 template <class T>
-struct ColdRay {
+struct ColdRay : SlabRay<T> {
     double od[3];
     ShearedRay<T> sh;
     T tmax, errN;
@@ -291,15 +294,18 @@ __device__ __forceinline__ void loadNode(const WideNode* nodes, uint32_t i, Node
 }
 
 
-// Decoded child boxes of a node, slab-tested against the ray. Returns the hit mask (slot order). The test is
-// in FP32 in every mode: it only has to be conservative. FromDouble: the ray is an FP64 one, whose origin's
-// and direction's rounding the slabs are widened by (a couple of ulps of each plane's and the origin's
-// distances along the ray), where the FP32 modes' boxes are padded for their rays. 641 x 359 room in FP64 at
-// 3 spp: 8.21 -> 6.74 ms a pass, kIntersect 5.35 -> 4.10 ms, films the same to the bit.
-template <bool FromDouble>
-__device__ __forceinline__ uint32_t intersectChildren(const NodeWords& nd, const V3<float>& inv, const V3<float>& oinv, float tmin,
-                                                      float tmax) {
+// Decoded child boxes of a node, slab-tested against the ray over (0, tmax). Returns the hit mask (slot order).
+// The planes' distances are FP32 in every mode: the test only has to be conservative. For an FP64 ray the
+// distance b of the node's origin is taken in FP64 from its FP64 origin and inverse direction and then rounded,
+// so that the slabs are as tight as the FP64 test's wherever the ray starts: taken in FP32, with slabs widened by
+// the rounding of the ray's origin, rays from 1e6 m away met ten times the nodes' work (2^18 rays into the room
+// of 2^18 triangles: 184 ms, against 8.4). The origin and the inverse are read from the cold record, which spares the
+// node loop ten registers: 641 x 359 room in FP64 at 3 spp 6.5 ms a pass either way (8.2 with FP64 slabs).
+template <class TR>
+__device__ __forceinline__ uint32_t intersectChildren(const NodeWords& nd, const ColdRay<TR>& ray, const V3<float>& inv,
+                                                      const V3<float>& oinv, float tmax) {
     using T = float;
+    constexpr bool FromDouble = sizeof(TR) == sizeof(double);
     const T sx = T(__uint_as_float((nd.a.w & 0xFFu) << 23));
     const T sy = T(__uint_as_float(((nd.a.w >> 8) & 0xFFu) << 23));
     const T sz = T(__uint_as_float(((nd.a.w >> 16) & 0xFFu) << 23));
@@ -311,22 +317,31 @@ __device__ __forceinline__ uint32_t intersectChildren(const NodeWords& nd, const
     // rounding), so the boxes stay conservative and grow by well under a percent of a quantum.
     const T ax = sx * inv.x, ay = sy * inv.y, az = sz * inv.z;
     const T ax8 = ax * T(0.00390625), ay8 = ay * T(0.00390625), az8 = az * T(0.00390625);
-    const T b0x = T(__uint_as_float(nd.a.x)) * inv.x - oinv.x;
-    const T b0y = T(__uint_as_float(nd.a.y)) * inv.y - oinv.y;
-    const T b0z = T(__uint_as_float(nd.a.z)) * inv.z - oinv.z;
-    const T bx = b0x - T(32768) * ax, by = b0y - T(32768) * ay, bz = b0z - T(32768) * az;
-    T mx = T(0.00390625) * fabs(ax) + T(2.4e-7) * fabs(bx);
-    T my = T(0.00390625) * fabs(ay) + T(2.4e-7) * fabs(by);
-    T mz = T(0.00390625) * fabs(az) + T(2.4e-7) * fabs(bz);
-    if (FromDouble) {
-        mx += T(3e-7) * (fabs(oinv.x) + fabs(b0x));
-        my += T(3e-7) * (fabs(oinv.y) + fabs(b0y));
-        mz += T(3e-7) * (fabs(oinv.z) + fabs(b0z));
+    T b0x, b0y, b0z;
+    if constexpr (FromDouble) {
+        b0x = T((double(__uint_as_float(nd.a.x)) - ray.od[0]) * ray.inv[0]);
+        b0y = T((double(__uint_as_float(nd.a.y)) - ray.od[1]) * ray.inv[1]);
+        b0z = T((double(__uint_as_float(nd.a.z)) - ray.od[2]) * ray.inv[2]);
+    } else {
+        b0x = T(__uint_as_float(nd.a.x)) * inv.x - oinv.x;
+        b0y = T(__uint_as_float(nd.a.y)) * inv.y - oinv.y;
+        b0z = T(__uint_as_float(nd.a.z)) * inv.z - oinv.z;
     }
+    const T bx = b0x - T(32768) * ax, by = b0y - T(32768) * ay, bz = b0z - T(32768) * az;
+    // FP64 rays: in units of u = 2^-24, b carries u |b| and a u |a|, the two roundings of the affine term 2 u |bx|
+    // and the FMA's own u (|b| + 255 |a|), and |b| <= |bx| + 2^15 |a|: 4 u |bx| + (2^-8 + 512 u) |a| in all, which
+    // 2.4e-7 |bx| + 0.004 |a| covers on both sides.
+    constexpr T quantum = FromDouble ? T(0.004) : T(0.00390625);
+    const T mx = quantum * fabs(ax) + T(2.4e-7) * fabs(bx);
+    const T my = quantum * fabs(ay) + T(2.4e-7) * fabs(by);
+    const T mz = quantum * fabs(az) + T(2.4e-7) * fabs(bz);
     const T nbx = bx - mx, nby = by - my, nbz = bz - mz;
-    const T fbx = bx + mx + (fabs(b0x) + T(255) * fabs(ax)) * kFarWiden;
-    const T fby = by + my + (fabs(b0y) + T(255) * fabs(ay)) * kFarWiden;
-    const T fbz = bz + mz + (fabs(b0z) + T(255) * fabs(az)) * kFarWiden;
+    T fbx = bx + mx, fby = by + my, fbz = bz + mz;
+    if constexpr (!FromDouble) {
+        fbx += (fabs(b0x) + T(255) * fabs(ax)) * kFarWiden;
+        fby += (fabs(b0y) + T(255) * fabs(ay)) * kFarWiden;
+        fbz += (fabs(b0z) + T(255) * fabs(az)) * kFarWiden;
+    }
     const bool nx = inv.x < T(0), ny = inv.y < T(0), nz = inv.z < T(0);
     // near and far planes per axis, chosen by the ray's direction on whole words
     const uint32_t nxl0 = nx ? nd.d.z : nd.c.x, nxl1 = nx ? nd.d.w : nd.c.y;
@@ -349,7 +364,7 @@ __device__ __forceinline__ uint32_t intersectChildren(const NodeWords& nd, const
         const T t0x = fma(lx, ax8, nbx), t1x = fma(hx, ax8, fbx);
         const T t0y = fma(ly, ay8, nby), t1y = fma(hy, ay8, fby);
         const T t0z = fma(lz, az8, nbz), t1z = fma(hz, az8, fbz);
-        const T te = fmax(fmax(t0x, t0y), fmax(t0z, tmin));
+        const T te = fmax(fmax(t0x, t0y), fmax(t0z, T(0)));
         const T tx = fmin(fmin(t1x, t1y), t1z);
         const T tl = fmin(tx, tmax);
         if (te <= tl) mask |= 1u << i;
@@ -427,7 +442,8 @@ __device__ __forceinline__ uint32_t permuteSlots(uint32_t m, uint32_t x) {
 // (fullCrossings).
 template <class T, class R, class Rr, bool AnyHit, class Stack = SharedStack, bool Count = true, bool Full = false>
 struct Traversal {
-    V3<T> o, d;           // the ray, camera-relative
+    V3<T> d;              // the ray's direction
+    V3<float> o;          // its origin, camera-relative (an FP64 ray's is the cold record's)
     V3<float> inv, oinv;  // for the slab tests
     T best;
     T bestCos;            // contact-resolving instantiation: |cos| of the closest crossing's incidence
@@ -454,10 +470,17 @@ struct Traversal {
         c->depB = q.depB;
         c->depP = q.depP;
         c->region = q.region;
-        o = q.o;
         d = q.d;
-        inv = V3<float>(safeInverse(float(d.x)), safeInverse(float(d.y)), safeInverse(float(d.z)));
-        oinv = V3<float>(float(o.x) * inv.x, float(o.y) * inv.y, float(o.z) * inv.z);
+        const V3<T> i(safeInverse(d.x), safeInverse(d.y), safeInverse(d.z));
+        inv = V3<float>(i);
+        if constexpr (sizeof(T) == sizeof(double)) {
+            c->inv[0] = i.x;
+            c->inv[1] = i.y;
+            c->inv[2] = i.z;
+        } else {
+            o = q.o;
+            oinv = V3<float>(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+        }
         best = q.tmax;
         bestCos = T(1);
         bestD = double(q.tmax);
@@ -475,10 +498,15 @@ struct Traversal {
         primBits = 0;
     }
 
+    __device__ __forceinline__ V3<T> origin() const {
+        if constexpr (sizeof(T) == sizeof(double)) return c->origin();
+        else return o;
+    }
+
     // The query as begin() took it.
     __device__ __forceinline__ RayQuery<T> query() const {
         RayQuery<T> q;
-        q.o = o;
+        q.o = origin();
         q.d = d;
         q.od = c->origin();
         q.tmax = c->tmax;
@@ -517,7 +545,7 @@ struct Traversal {
                 NodeWords nd;
                 loadNode(sc.nodes, node, nd);
                 if (Count) ++nodeVisits;
-                const uint32_t mask = intersectChildren<sizeof(T) == sizeof(double)>(nd, inv, oinv, 0.f, slabLimit((Full && !AnyHit) ? tieLimit() : best));
+                const uint32_t mask = intersectChildren<T>(nd, *c, inv, oinv, slabLimit((Full && !AnyHit) ? tieLimit() : best));
                 const uint32_t inner = nd.a.w >> 24;
                 nodeBase = nd.b.x;
                 nodeBits = permuteSlots(mask & inner, first) | (inner << 8);
@@ -544,7 +572,7 @@ struct Traversal {
     // A distance as the slab tests' FP32 limit, rounded up.
     __device__ __forceinline__ static float slabLimit(T t) {
         if constexpr (sizeof(T) == sizeof(float)) return t;
-        else return float(t) + 3e-7f * fabsf(float(t));
+        else return __double2float_ru(t);
     }
 
     // Contact decisions compare FP64 distances where the instantiation has them: the FP64 one, and
@@ -651,6 +679,7 @@ struct Traversal {
         const T limit = (Full && !AnyHit) ? tieLimit() : best;
         uint32_t flags = 0;
         if (kind == kPrimTriangle) {
+            const V3<T> o = origin();
             const V3<T> a0 = v0 - o, a1 = v1 - o, a2 = v2 - o;
             if (!lineCrossesTriangle(c->sh, a0, a1, a2)) return false;
             const V3<T> n = triangleNormal(v0, v1, v2);
