@@ -20,6 +20,7 @@
 // world hierarchy and of every mesh's own hierarchy with one hierarchy over all primitives.
 #include <cub/device/device_radix_sort.cuh>
 
+#include <algorithm>
 #include <vector>
 
 #include "bvh_build.hpp"
@@ -498,7 +499,10 @@ uint32_t buildWideBvh(const float4* primLo, const float4* primHi, uint32_t n, Bv
         if (err >= 0x10000u) throw std::runtime_error("BVH build: malformed radix tree");
         s.nodeCount = h[0];
         s.placedPrims = h[1];
-        if (h[2 + level] == 0) break;
+        if (h[2 + level] == 0) {
+            s.levels = uint32_t(std::find(h.begin() + 2, h.end(), 0u) - (h.begin() + 2));
+            break;
+        }
         if (level + batch > int(kMaxLevels)) throw std::runtime_error("BVH collapse did not terminate");
     }
     if (s.placedPrims != n) throw std::runtime_error("BVH collapse placed " + std::to_string(s.placedPrims) +

@@ -17,7 +17,7 @@ struct BvhScratch {
     DBuf<float4> boxLo, boxHi;
     DBuf<uint2> work, next;
     DBuf<int> bounds;
-    uint32_t nodeCount = 0, placedPrims = 0;
+    uint32_t nodeCount = 0, placedPrims = 0, levels = 0;
 };
 
 // Builds the wide BVH over n primitive boxes (camera-relative, padded outward). Fills `nodes`

@@ -1143,6 +1143,7 @@ void buildBvh(owec_ctx& c) {
         c.ds.prims64 = nullptr;
         c.ds.nNodes = 0;
         c.ds.nPrims = 0;
+        c.ds.stackDepth = kMinStackDepth;
         c.bvhDirty = false;
         c.prims64Ready = true;
         return;
@@ -1151,6 +1152,7 @@ void buildBvh(owec_ctx& c) {
     c.ds.nodes = c.dNodes.get();
     c.ds.nNodes = c.nNodes;
     c.ds.nPrims = c.nPrims;
+    c.ds.stackDepth = std::min(kMaxStackDepth, std::max(kMinStackDepth, int(c.scratch.levels)));
     materializePrims(c, c.settings.precision != OWEC_PRECISION_FP32);
     c.bvhDirty = false;
 }

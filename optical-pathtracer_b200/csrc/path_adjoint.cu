@@ -914,7 +914,8 @@ template <int M>
 void launchMode(const DeviceScene& sc, const AdjointParams& P, const void* ckpt, const uint32_t* count, int grid,
                 cudaStream_t s) {
     using C = PathCheckpoint<typename Mode<M>::R>;
-    const size_t smem = traversalSharedBytes(kAdjointBlock);
+    static_assert(kAdjointBlock * kMaxStackDepth * sizeof(StackEntry) <= 48 * 1024, "what a kernel gets unasked");
+    const size_t smem = traversalSharedBytes(sc, kAdjointBlock);
     if (ckpt) {
         if (sc.fullFeatures) kPathAdjointResume<M, true><<<grid, kAdjointBlock, smem, s>>>(sc, P, static_cast<const C*>(ckpt), count);
         else kPathAdjointResume<M, false><<<grid, kAdjointBlock, smem, s>>>(sc, P, static_cast<const C*>(ckpt), count);

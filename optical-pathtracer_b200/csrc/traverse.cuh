@@ -20,13 +20,6 @@
 
 namespace owec {
 
-#ifndef OWEC_STACK_DEPTH
-#define OWEC_STACK_DEPTH 16
-#endif
-// Group entries per thread in shared memory, one per level: 16 levels of eight children cover any tree
-// that is near balanced, and half the former 32 leaves the shared memory to the queries' cold records
-// and the L1.
-constexpr int kStackDepth = OWEC_STACK_DEPTH;
 constexpr int kDeepStackDepth = 96;  // the rare query of a deeper tree is traversed again with a stack
                                      // of this depth in local memory; beyond it the query ends and is
                                      // counted as a fault
@@ -41,7 +34,7 @@ struct StackEntry {
 // The short traversal stack: this thread's column of the block's shared-memory stack (stride =
 // block size), so that a warp's entries of one level are consecutive words.
 struct SharedStack {
-    static constexpr int kDepth = kStackDepth;
+    __device__ __forceinline__ static int depth(const DeviceScene& sc) { return sc.stackDepth; }
     StackEntry* sh;
     int stride;
     __device__ __forceinline__ void init(StackEntry* stack, int s) { sh = stack; stride = s; }
@@ -50,7 +43,7 @@ struct SharedStack {
 };
 // The deep stack, in local memory, for the queries that overflow the short one.
 struct LocalStack {
-    static constexpr int kDepth = kDeepStackDepth;
+    __device__ __forceinline__ static int depth(const DeviceScene&) { return kDeepStackDepth; }
     StackEntry e[kDeepStackDepth];
     __device__ __forceinline__ void init(StackEntry*, int) {}
     __device__ __forceinline__ StackEntry get(int i) const { return e[i]; }
@@ -538,7 +531,7 @@ struct Traversal {
                 const uint32_t slot = pos ^ first;
                 const uint32_t node = nodeBase + uint32_t(__popc((nodeBits >> 8) & ((1u << slot) - 1u)));
                 if (nodeBits & 0xFFu) {
-                    if (sp >= Stack::kDepth) return kTraceOverflow;
+                    if (sp >= Stack::depth(sc)) return kTraceOverflow;
                     st.set(sp, {nodeBase, nodeBits});
                     ++sp;
                 }

@@ -446,7 +446,7 @@ template <int M, bool ADJ, bool Full>
 void walkKernelOf(const DeviceScene& sc, const WalkParams& P, unsigned long long* bins, unsigned long long* stats,
                   const double* g, double* dH, int numSMs, cudaStream_t s) {
     constexpr int block = kWalkBlock<Full>;
-    const size_t smem = traversalSharedBytes(block);
+    const size_t smem = traversalSharedBytes(sc, block);
     OWEC_CUDA(cudaFuncSetAttribute(kWalk<M, ADJ, Full>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     unsigned long long* fetch = stats + kWalkFetchWord;
     OWEC_CUDA(cudaMemsetAsync(fetch, 0, sizeof(*fetch), s));

@@ -96,8 +96,8 @@ __device__ __forceinline__ uint32_t refillLanes(bool idle, uint32_t* fetch, uint
 
 // This thread's record behind the block's traversal stacks (persistentSharedBytes).
 template <class R>
-__device__ __forceinline__ ColdRay<R>* coldRay(StackEntry* stackMem) {
-    return reinterpret_cast<ColdRay<R>*>(stackMem + size_t(kStackDepth) * blockDim.x) + threadIdx.x;
+__device__ __forceinline__ ColdRay<R>* coldRay(const DeviceScene& sc, StackEntry* stackMem) {
+    return reinterpret_cast<ColdRay<R>*>(stackMem + size_t(sc.stackDepth) * blockDim.x) + threadIdx.x;
 }
 
 // Adds a per-lane count to a counter, one atomic per warp (all lanes of the warp present).
@@ -115,7 +115,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kIntersect(DeviceScene sc, PathBuffers<RT<
     using R = RT<M>;
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
-    ColdRay<R>* cold = coldRay<R>(stackMem);
+    ColdRay<R>* cold = coldRay<R>(sc, stackMem);
     if (firstThread()) stampIntersect(q);
     const uint32_t n = q.counts[kCountActive];
     Traversal<R, typename Mode<M>::Ro, typename Mode<M>::Rr, false, SharedStack, Count, Full> tr;
@@ -629,7 +629,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadow(DeviceScene sc, PassParams pp, Pat
     using Rr = typename Mode<M>::Rr;
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
-    ColdRay<R>* cold = coldRay<R>(stackMem);
+    ColdRay<R>* cold = coldRay<R>(sc, stackMem);
     if (firstThread()) stampShadow(q);
     const uint32_t n = q.counts[kCountShadow];
     Traversal<R, Ro, Rr, AnyHit, SharedStack, Count, Full> tr;
@@ -787,7 +787,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadowVis(DeviceScene sc, PathBuffers<RT<
     using Rr = typename Mode<M>::Rr;
     extern __shared__ StackEntry stackMem[];
     StackEntry* stack = stackMem + threadIdx.x;
-    ColdRay<R>* cold = coldRay<R>(stackMem);
+    ColdRay<R>* cold = coldRay<R>(sc, stackMem);
     if (firstThread()) stampShadow(q);
     const uint32_t n = q.counts[kCountShadow];
     Traversal<R, Ro, Rr, true, SharedStack, Count, Full> tr;
@@ -992,7 +992,7 @@ __device__ __forceinline__ void castQueries(const DeviceScene& sc, uint64_t n, c
         __shared__ uint32_t fetch;
         if (threadIdx.x == 0) fetch = 0;
         __syncthreads();
-        ColdRay<T>* cold = coldRay<T>(stackMem);
+        ColdRay<T>* cold = coldRay<T>(sc, stackMem);
         Traversal<T, R, Rr, false, SharedStack, false, false> tr;
         const uint64_t share = (n + gridDim.x - 1) / gridDim.x, first = share * blockIdx.x;
         const uint32_t count = first < n ? uint32_t(share < n - first ? share : n - first) : 0u;
@@ -1127,10 +1127,13 @@ __global__ void __launch_bounds__(256) kResolve(const double* film, const double
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
-size_t traversalSharedBytes(int block) { return size_t(block) * kStackDepth * sizeof(StackEntry); }
-// The persistent kernels': the stacks and the queries' cold records.
+size_t traversalSharedBytes(const DeviceScene& sc, int block) { return size_t(block) * sc.stackDepth * sizeof(StackEntry); }
+// The persistent kernels': the stacks and the queries' cold records, at most what a kernel gets unasked.
 template <int M>
-size_t persistentSharedBytes(int block) { return traversalSharedBytes(block) + size_t(block) * sizeof(ColdRay<RT<M>>); }
+size_t persistentSharedBytes(const DeviceScene& sc, int block) {
+    return traversalSharedBytes(sc, block) + size_t(block) * sizeof(ColdRay<RT<M>>);
+}
+static_assert(128 * (kMaxStackDepth * sizeof(StackEntry) + sizeof(ColdRay<double>)) + 16 <= 48 * 1024, "stacks and records fit");
 
 template <int M>
 void launchGenerate(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
@@ -1141,7 +1144,7 @@ template <int M>
 void launchIntersect(const DeviceScene& sc, const PathBuffers<RT<M>>& pb, const Queues& q, StatCounters* st,
                      int grid, cudaStream_t s) {
     uint32_t* fetch = q.counts + kFetchIntersect;
-    const size_t smem = persistentSharedBytes<M>(128);
+    const size_t smem = persistentSharedBytes<M>(sc, 128);
     if (sc.fullFeatures) {
         if (sc.travCounters) kIntersect<M, true, true><<<grid, 128, smem, s>>>(sc, pb, q, st, fetch);
         else kIntersect<M, false, true><<<grid, 128, smem, s>>>(sc, pb, q, st, fetch);
@@ -1172,7 +1175,7 @@ void launchSurface(const DeviceScene& sc, const PassParams& pp, const PathBuffer
 template <int M, bool Splat, bool Count, bool Full>
 void shadowKernelsOf(const DeviceScene& sc, const PassParams& pp, const PathBuffers<RT<M>>& pb, const Queues& q,
                      StatCounters* st, uint32_t* fetch, uint8_t* vis, const SplatTarget& film, int grid, cudaStream_t s) {
-    const size_t smem = persistentSharedBytes<M>(128);
+    const size_t smem = persistentSharedBytes<M>(sc, 128);
     // next-event rays of a scene with contacts take the ordered walk, where the light point's
     // identity decides what lies at its end
     if (pp.anyHitShadows && !(Full && !Splat)) {
@@ -1222,14 +1225,14 @@ static int castGrid(uint64_t n, int grid) { return int(std::min<uint64_t>(uint64
 template <int M>
 void launchCastRays(const DeviceScene& sc, const CastPieces& b, int grid, cudaStream_t s) {
     grid = castGrid(b.n, grid);
-    if (sc.fullFeatures) kCastRays<M, true><<<grid, 128, traversalSharedBytes(128), s>>>(sc, b);
-    else kCastRays<M, false><<<grid, 128, persistentSharedBytes<M>(128), s>>>(sc, b);
+    if (sc.fullFeatures) kCastRays<M, true><<<grid, 128, traversalSharedBytes(sc, 128), s>>>(sc, b);
+    else kCastRays<M, false><<<grid, 128, persistentSharedBytes<M>(sc, 128), s>>>(sc, b);
 }
 void launchCastRaysF(const DeviceScene& sc, uint64_t n, const float* o, const float* d, uint32_t* b, uint32_t* p,
                      float* t, int grid, cudaStream_t s) {
     grid = castGrid(n, grid);
-    if (sc.fullFeatures) kCastRaysF<true><<<grid, 128, traversalSharedBytes(128), s>>>(sc, n, o, d, b, p, t);
-    else kCastRaysF<false><<<grid, 128, persistentSharedBytes<OWEC_PRECISION_MIXED>(128), s>>>(sc, n, o, d, b, p, t);
+    if (sc.fullFeatures) kCastRaysF<true><<<grid, 128, traversalSharedBytes(sc, 128), s>>>(sc, n, o, d, b, p, t);
+    else kCastRaysF<false><<<grid, 128, persistentSharedBytes<OWEC_PRECISION_MIXED>(sc, 128), s>>>(sc, n, o, d, b, p, t);
 }
 void launchResolve(const double* film, const double* comp, const double* samples, uint32_t nPixels, double* xyz,
                    cudaStream_t s) {

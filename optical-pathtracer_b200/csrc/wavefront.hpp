@@ -11,7 +11,7 @@ namespace owec {
 template <int M>
 using ModeR = typename Mode<M>::R;
 
-size_t traversalSharedBytes(int block);
+size_t traversalSharedBytes(const DeviceScene&, int block);
 
 template <int M>
 void launchGenerate(const DeviceScene&, const PassParams&, const PathBuffers<ModeR<M>>&, const Queues&, StatCounters*,
