@@ -508,8 +508,9 @@ typedef struct owec_adjoint_stats {
     uint64_t faults;      /* bounded loops that ran out */
     double seconds;       /* device time of the call */
     uint64_t device_bytes;/* device memory of the call's buffers: loss gradient, height gradient,
-                           * checkpoints, replayed film (the context keeps all but the last for the next
-                           * call) */
+                           * checkpoints, replayed film. The context keeps all but the last for the next
+                           * call, until another scene is uploaded. Not counted: the path state, which the
+                           * passes use too, and the replay kernel's local-memory stacks */
     double replay_seconds;/* of seconds, the device time of the derivative replay alone (the rest is the
                            * wavefront phase that runs the paths to their first heightfield crossing) */
 } owec_adjoint_stats;

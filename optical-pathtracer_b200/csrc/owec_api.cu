@@ -1098,9 +1098,13 @@ void uploadScene(owec_ctx& c, const owec_scene_desc& d) {
     c.bvhDirty = true;
     c.prims64Ready = false;
     c.tri64Ready = false;
-    // a new scene has no heightfield until owec_set_heightfield names one of its boundaries
-    c.hf.boundary = kNone;
+    // a new scene has no heightfield until owec_set_heightfield names one of its boundaries, and needs none of
+    // what the adjoints kept for the last one
+    c.hf = HeightfieldParams{kNone, nullptr, {0, 0, 1}};
     c.hfVertices = 0;
+    c.dHfTris.release();
+    for (DBuf<double>* b : {&c.dHfVerts, &c.dHfHeights, &c.dLossGrad, &c.dHeightGrad}) b->release();
+    c.dCheckpoints.release();
     c.passCount = 0;
     c.dFilm.release();
     c.dComp.release();

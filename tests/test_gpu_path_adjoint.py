@@ -179,3 +179,26 @@ def test_gradient_descent_recovers_the_heights():
     save_artifact("path_adjoint_descent", target=target_h, final=final.reshape(N, N), losses=np.array([loss0, loss1]))
     assert rmse1 < 0.5 * rmse0, (rmse0, rmse1, loss0, loss1)
     assert loss1 < loss0, (loss0, loss1)
+
+
+def test_a_new_scene_gives_back_what_the_adjoint_kept():
+    import torch
+    sb, info = scenes.caustic_room(width=640, height=360, n_lon=32, n_lat=16, panel_n=32)
+    desc = sb.desc()
+    other = scenes.bvh_stress_room(640, 360, 32, 16).desc()
+    with owe_cuda.Context(0) as c:
+        c.set_settings(A.make_settings(seed=2, max_depth=8, rr_depth=6))
+        c.upload(desc)
+        c.set_heightfield(info["heightfield"], info["base_z"], np.zeros(32 * 32))
+        c.run_pass(4)
+        g = np.zeros((360, 640, 3))
+        _, st, _ = c.path_adjoint(0, 4, g, with_stats=True)
+        held = torch.cuda.mem_get_info(0)[0]
+        c.upload(other)
+        # allocations come in steps of 2 MB
+        assert torch.cuda.mem_get_info(0)[0] - held >= st["device_bytes"] - (16 << 20) > (100 << 20)
+        c.run_pass(1)
+        c.upload(desc)
+        c.set_heightfield(info["heightfield"], info["base_z"], np.zeros(32 * 32))
+        c.run_pass(4)
+        c.path_adjoint(0, 4, g)
