@@ -1302,8 +1302,8 @@ void runBounces(owec_ctx& c, Queues q, int maxDepth, uint32_t nPaths, int& bounc
 
 // The shadow kernels of a bounce run beside the next bounce's closest-hit kernel: neither reads what the
 // other writes (radiance and connections; hits), and each leaves the GPU to its last long rays for a
-// quarter of its time (kIntersect's SMs were active for 73 % of it). shadowsBegin: on the shadow stream
-// from here, after the events queued so far; shadowsEnd: the pass's stream waits for them.
+// quarter of its time (kIntersect's SMs were active for 73 % of it). queueShadows: on the shadow stream,
+// after the events queued so far; joinShadows: the pass's stream waits for them.
 template <class Launch>
 void queueShadows(owec_ctx& c, const Launch& launch) {
     OWEC_CUDA(cudaEventRecord(c.eventsDone, c.stream));
@@ -1525,18 +1525,6 @@ uint64_t runAdjointCheckpointed(owec_ctx& c, PassParams pp, uint64_t firstPass, 
     return hs.paths;
 }
 
-// Share k of n of a result buffer's whole pages, faulted in while the rays are traced (a kernel without the advice
-// faults them in under the workers' copies). What the pages hold stays: a worker done with its share may already be
-// writing hits into another's.
-void populateShare(void* dst, size_t bytes, size_t k, size_t n) {
-    constexpr size_t kPage = 4096;
-    char* first = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(dst) + kPage - 1) & ~uintptr_t(kPage - 1));
-    char* end = static_cast<char*>(dst) + bytes;
-    if (end <= first) return;
-    const size_t pages = size_t(end - first) / kPage, from = pages * k / n, to = pages * (k + 1) / n;
-    if (from < to) (void)madvise(first + from * kPage, (to - from) * kPage, MADV_POPULATE_WRITE);
-}
-
 // One batch of host rays: pieces of 2^shift rays, dealt to the workers as they come for them and traced by the
 // group. A piece travels to the device as its origins and then its directions, its hits come back as distances,
 // boundaries, primitives (CastPieces, the layout launchCastRays reads and writes).
@@ -1639,12 +1627,7 @@ void castBatch(owec_ctx& c, CastBatch& b, int workers) {
             if (k) OWEC_CUDA(cudaSetDevice(c.device));
             uploadPieces<M>(c, b, k, k ? c.castStaging + size_t(k - 1) * kCastSlot : own);
         },
-        [&](int k, int n) {
-            populateShare(b.t, 8 * b.n, size_t(k), size_t(n));
-            populateShare(b.boundary, 4 * b.n, size_t(k), size_t(n));
-            populateShare(b.prim, 4 * b.n, size_t(k), size_t(n));
-            downloadPieces(c, b, k, k ? c.castStaging + size_t(k - 1) * kCastSlot : own);
-        });
+        [&](int k) { downloadPieces(c, b, k, k ? c.castStaging + size_t(k - 1) * kCastSlot : own); });
 }
 
 // The slots, events and stream that a call with several workers needs besides; false where they cannot be had.
@@ -1670,7 +1653,8 @@ bool castStagingReady(owec_ctx& c) {
 // Host rays: packed and copied by the workers, traced by the group, copied back and unpacked. One core's packing
 // of a ray's 64 bytes, the driver's own staging of pageable copies, the faults of the results' fresh pages and
 // five allocations a call took ten times the kernel's time (2^20 rays into the room of 2^18 triangles: 10.5 ms
-// around a 0.97 ms kernel). The groups' launches, each on its own stream, overlap the copies and each other's
+// around a 0.97 ms kernel; faulting the results' pages in while the rays are traced, on top of this, changed
+// nothing). The groups' launches, each on its own stream, overlap the copies and each other's
 // last rays, and each has the rays to fill the GPU: launches of 16,384 rays, one after another on four streams,
 // left most of it idle where the tracing is the longer part (2^20 rays into the FP32 wave pool: 50.3 ms, against
 // 23.6 in one launch). Device memory for

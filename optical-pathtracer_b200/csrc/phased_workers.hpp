@@ -10,8 +10,8 @@
 
 namespace owec {
 
-// run(first, second): first(worker) on every worker, and once all of them are done with it second(worker, workers)
-// on every worker. The calling thread is worker 0; the others are started here, as many as the system gives
+// run(first, second): first(worker) on every worker, and once all of them are done with it second(worker) on every
+// worker. The calling thread is worker 0; the others are started here, as many as the system gives
 // (with none, the calling thread does all the work, which the callers deal out piece by piece). After a failure
 // no further phase starts; the first one is rethrown once all threads have ended. Thread: std::thread, or a
 // test's.
@@ -20,7 +20,7 @@ class PhasedWorkersOf {
 public:
     explicit PhasedWorkersOf(int workers) : wanted_(workers) {}
 
-    void run(const std::function<void(int)>& first, const std::function<void(int, int)>& second) {
+    void run(const std::function<void(int)>& first, const std::function<void(int)>& second) {
         threads_.reserve(size_t(wanted_));
         for (int k = 1; k < wanted_; ++k) {
             try {
@@ -32,21 +32,20 @@ public:
                         changed_.notify_all();
                         changed_.wait(lock, [&] { return open_; });
                     }
-                    attempt([&] { second(k, workers_); });
+                    attempt([&] { second(k); });
                 });
             } catch (...) {  // no more threads to be had
                 break;
             }
         }
-        workers_ = int(threads_.size()) + 1;
         attempt([&] { first(0); });
         {
             std::unique_lock<std::mutex> lock(mutex_);
-            changed_.wait(lock, [&] { return arrived_ == workers_ - 1; });
+            changed_.wait(lock, [&] { return arrived_ == int(threads_.size()); });
             open_ = true;
             changed_.notify_all();
         }
-        attempt([&] { second(0, workers_); });
+        attempt([&] { second(0); });
         for (Thread& t : threads_) t.join();
         if (failure_) std::rethrow_exception(failure_);
     }
@@ -66,7 +65,7 @@ private:
         }
     }
 
-    int wanted_, workers_ = 1, arrived_ = 0;
+    int wanted_, arrived_ = 0;
     bool open_ = false;
     std::mutex mutex_;
     std::condition_variable changed_;

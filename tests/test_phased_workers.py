@@ -39,7 +39,7 @@ PROGRAM = textwrap.dedent(r"""
             bool threw = false;
             try {
                 gang.run([&](int k) { for (int i; (i = up++) < 1000;) { if (fail == 1 && i == 500) throw std::runtime_error("up"); ++upDone; } (void)k; },
-                         [&](int k, int n) { if (n != expect || k >= n || upDone != 1000) order = false; for (int i; (i = down++) < 1000;) { if (fail == 2 && i == 500) throw std::runtime_error("down"); ++downDone; } });
+                         [&](int k) { if (k >= expect || upDone != 1000) order = false; for (int i; (i = down++) < 1000;) { if (fail == 2 && i == 500) throw std::runtime_error("down"); ++downDone; } });
             } catch (const std::runtime_error&) { threw = true; }
             if (!order) { std::puts("order"); return 1; }
             if (threw != (fail != 0)) { std::puts("exception"); return 1; }
