@@ -1,5 +1,6 @@
-"""The bounce loop at its edges: depths from none to far beyond any path's end, films from one pixel up,
-several passes in flight through one context, and paths through null boundaries that outlive the depth."""
+"""The bounce loop at its edges: depths from none to far beyond any path's end, films from one pixel up, passes in
+one call and in several, batches of one pass after another, images still being copied when the film is cleared,
+and paths through null boundaries that outlive the depth."""
 import numpy as np
 import pytest
 
@@ -52,3 +53,39 @@ def test_times_of_a_pass(precision):
             # the two kinds of kernel overlap each other but not themselves (20 us: the timer's steps)
             assert 0 < intersect < total + 2e-5 and 0 < shadow < total + 2e-5
             assert launches >= 7
+
+
+@pytest.mark.parametrize("size,spp", [((33, 17), 3), ((64, 64), 1030)])
+@pytest.mark.parametrize("precision", [A.PRECISION_MIXED, A.PRECISION_FP32, A.PRECISION_FP64])
+def test_light_passes_repeat_to_the_bit(size, spp, precision):
+    """Splats are fixed-point sums: a connection lost or counted twice beside the next bounce's closest-hit kernel
+    would show in any bit. The larger pass takes three batches of 2^21 particles."""
+    desc = scenes.materials_gallery(*size).desc()
+    with owe_cuda.Context(0) as c:
+        c.upload(desc)
+        c.set_settings(A.make_settings(seed=2, max_depth=12, rr_depth=4, precision=precision, integrator="light"))
+        a = render(c, [spp])
+        b = render(c, [spp])
+    assert a[0].max() > 0 and a[2]["device_faults"] == 0
+    assert a[2] == b[2]
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("integrator", ["path", "light"])
+def test_film_cleared_while_its_image_is_copied(integrator):
+    desc = scenes.bvh_stress_room(641, 359, 64, 32).desc()
+    with owe_cuda.Context(0) as c:
+        c.upload(desc)
+        c.set_settings(A.make_settings(seed=6, max_depth=5, integrator=integrator))
+        want = render(c, [1])
+        c.reset_film()
+        c.run_pass(1)
+        out = np.zeros((359, 641, 3))
+        samples = np.zeros((359, 641))
+        c.resolve_async(out, samples)
+        c.reset_film()
+        c.run_pass(1)
+        c.resolve_wait()
+        again = c.resolve()
+    assert np.array_equal(out, want[0]) and np.array_equal(samples, want[1])
+    assert np.array_equal(again[0], want[0]) and np.array_equal(again[1], want[1])
