@@ -381,7 +381,7 @@ constexpr uint64_t kCastSerial = 65536;
 constexpr uint64_t kCastKept = 1ull << 21, kCastBatch = 1ull << 24;  // see castRays
 constexpr size_t kCastSlot = (size_t(1) << kCastPieceShift) * 48;
 constexpr int kCastGroups = 4;  // launches of a batch at most, of at least kCastGroupPieces pieces each
-constexpr uint64_t kCastGroupPieces = 8;
+constexpr uint64_t kCastGroupPieces = 2;
 constexpr size_t kHostReports = 4096;  // the context block's first part: what kernels report to the host
 constexpr size_t kHostBlock = kHostReports + kCastSlot;
 
@@ -1548,14 +1548,14 @@ void traceGroup(owec_ctx& c, CastBatch& b, uint64_t g) {
     const uint64_t first = g * b.groupPieces << b.shift, n = std::min(b.groupPieces << b.shift, b.n - first);
     const CastPieces pieces{n, b.device + 48 * first, b.hits() + 16 * first, b.shift};
     if (b.groups() == 1) {
-        launchCastRays<M>(c.ds, pieces, c.numSMs * 8, c.stream);
+        launchCastRays<M>(c.ds, pieces, c.numSMs, c.stream);
         checkLaunch();
         return;
     }
     const cudaStream_t s = g ? c.castStreams[g - 1] : c.shadowStream;
     OWEC_CUDA(cudaEventRecord(c.castUp[g], c.stream));
     OWEC_CUDA(cudaStreamWaitEvent(s, c.castUp[g], 0));
-    launchCastRays<M>(c.ds, pieces, c.numSMs * 4, s);
+    launchCastRays<M>(c.ds, pieces, c.numSMs, s);
     checkLaunch();
     OWEC_CUDA(cudaEventRecord(c.castTraced[g], s));
 }
@@ -1653,13 +1653,12 @@ bool castStagingReady(owec_ctx& c) {
 // Host rays: packed and copied by the workers, traced by the group, copied back and unpacked. One core's packing
 // of a ray's 64 bytes, the driver's own staging of pageable copies, the faults of the results' fresh pages and
 // five allocations a call took ten times the kernel's time (2^20 rays into the room of 2^18 triangles: 10.5 ms
-// around a 0.97 ms kernel; faulting the results' pages in while the rays are traced, on top of this, changed
-// nothing). The groups' launches, each on its own stream, overlap the copies and each other's
-// last rays, and each has the rays to fill the GPU: launches of 16,384 rays, one after another on four streams,
-// left most of it idle where the tracing is the longer part (2^20 rays into the FP32 wave pool: 50.3 ms, against
-// 23.6 in one launch). Device memory for
-// up to kCastKept rays (128 MB) stays with the context; larger calls allocate theirs, for kCastBatch rays
-// (1 GB) at a time.
+// around a 0.97 ms kernel; now 4.3, of which the rays' copies take 2.1; faulting the results' pages in while the rays
+// are traced changed nothing). The groups are traced on streams of their own and so all at once, each as its rays
+// arrive (120,000 rays 0.58 ms, against 0.81 in one launch). Launches of 16,384 rays one after another on four
+// streams left most of the GPU idle where the tracing is the longer part (2^20 rays into the FP32 wave pool: 50.3 ms,
+// against 23.6 in one launch and 13.0 now). Device memory for up to kCastKept rays (128 MB) stays with the context;
+// larger calls allocate theirs, for kCastBatch rays (1 GB) at a time.
 template <int M>
 void castRays(owec_ctx& c, uint64_t n, const double* o, const double* d, uint32_t* boundary, uint32_t* prim, double* t) {
     const uint64_t batch = std::min(n, kCastBatch);
@@ -2102,7 +2101,7 @@ int owec_cast_rays_device(owec_ctx* ctx, uint64_t n, const float* o, const float
         OWEC_CUDA(cudaSetDevice(ctx->device));
         ensureReady(*ctx);
         OWEC_CUDA(cudaEventRecord(ctx->passStart, ctx->stream));
-        launchCastRaysF(ctx->ds, n, o, d, b, p, t, ctx->numSMs * 8, ctx->stream);
+        launchCastRaysF(ctx->ds, n, o, d, b, p, t, ctx->numSMs, ctx->stream);
         checkLaunch();
         OWEC_CUDA(cudaEventRecord(ctx->passStop, ctx->stream));
         if (seconds) {

@@ -1,9 +1,10 @@
 // Host threads that work in two phases, the second starting when all of them are done with the first.
 #pragma once
 
-#include <condition_variable>
+#include <atomic>
 #include <exception>
 #include <functional>
+#include <limits>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -26,31 +27,28 @@ public:
             try {
                 threads_.emplace_back([this, k, &first, &second] {
                     attempt([&] { first(k); });
-                    {
-                        std::unique_lock<std::mutex> lock(mutex_);
-                        ++arrived_;
-                        changed_.notify_all();
-                        changed_.wait(lock, [&] { return open_; });
-                    }
+                    waitForAll();
                     attempt([&] { second(k); });
                 });
             } catch (...) {  // no more threads to be had
                 break;
             }
         }
+        expected_ = int(threads_.size()) + 1;
         attempt([&] { first(0); });
-        {
-            std::unique_lock<std::mutex> lock(mutex_);
-            changed_.wait(lock, [&] { return arrived_ == int(threads_.size()); });
-            open_ = true;
-            changed_.notify_all();
-        }
+        waitForAll();
         attempt([&] { second(0); });
         for (Thread& t : threads_) t.join();
         if (failure_) std::rethrow_exception(failure_);
     }
 
 private:
+    // The phases' ends lie microseconds apart, less than waking a sleeping thread takes.
+    void waitForAll() {
+        ++arrived_;
+        while (arrived_ < expected_) std::this_thread::yield();
+    }
+
     // f(), unless something has failed before.
     void attempt(const std::function<void()>& f) {
         {
@@ -65,10 +63,9 @@ private:
         }
     }
 
-    int wanted_, arrived_ = 0;
-    bool open_ = false;
+    int wanted_;
+    std::atomic<int> arrived_{0}, expected_{std::numeric_limits<int>::max()};
     std::mutex mutex_;
-    std::condition_variable changed_;
     std::exception_ptr failure_;
     std::vector<Thread> threads_;
 };

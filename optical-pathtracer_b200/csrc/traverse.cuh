@@ -72,8 +72,8 @@ template <class T> struct SlabRay {};
 template <> struct SlabRay<double> { double inv[3], pad; };
 // The part of a query that the node loop does not touch: what a primitive test, an accepted
 // crossing or the query's end needs. The persistent kernels keep it in shared memory, one record per
-// thread, which leaves the registers to the node test (at 128 registers kIntersect's spill stores go
-// from 126 to 40 bytes and its local-memory reads to a fifth; 96 or 80 registers for five or six
+// thread, which leaves the registers to the node test (at 128 registers the mixed kIntersect spills 92
+// bytes and reads 80 back, where it spilled 126; 96 or 80 registers for five or six
 // blocks still spill in the node loop and run 10 to 18 % slower). The record is an odd number of
 // 8-byte words, so that a warp's accesses to one field spread over the banks.
 template <class T>

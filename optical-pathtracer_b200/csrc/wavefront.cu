@@ -373,8 +373,8 @@ __global__ void __launch_bounds__(128, OWEC_SHADING_MIN_BLOCKS) kMedium(DeviceSc
 }
 
 // kMedium for a scene without any absorbing or scattering medium: a segment that met a boundary goes to
-// its surface queue on the hit record alone, and one that met none gathers the sky. 64 registers instead
-// of kMedium's 164: it waits on scattered loads, which twice the resident warps hide. With the surface
+// its surface queue on the hit record alone, and one that met none gathers the sky. 64 registers (80 in
+// FP64) instead of kMedium's 164 (168): it waits on scattered loads, which twice the resident warps hide. With the surface
 // kernels' next index loaded ahead, the 256 x 256 glass film at 64 spp: 5.45 -> 5.09 ms a pass, the
 // 1920 x 1080 room 14.35 -> 13.91 ms (prefetching the next records as well gained nothing).
 template <int M>
@@ -972,120 +972,137 @@ __global__ void __launch_bounds__(256) kFoldFilm(const double* film, const doubl
 }
 
 // ------------------------------------------------------------------ ray casts
-// The closest hits of rays 0 .. n - 1, load(i) giving the query of ray i and store(i, status, hit) taking its
-// answer. The lean instantiations run as kIntersect does: a block takes its share of the rays, and a lane whose
-// query ends takes the share's next ray. 2^21 device rays into the room of 2^20 triangles: 1.64 ms, against
-// 2.39 with each lane's query run to its end at the 146 registers the compiler takes unbounded (three blocks
-// to an SM), 2.09 so at 128. In the Full ones a refill waits on the others' numeric roots and walks with
-// contacts: with a cone in that room 6.83 ms refilled, 5.14 run to their ends at 128 registers (6.19 unbounded).
-template <class T, class R, class Rr, bool Full, class Load, class Store>
-__device__ __forceinline__ void castQueries(const DeviceScene& sc, uint64_t n, const Load& load, const Store& store) {
-    extern __shared__ StackEntry stackMem[];
-    StackEntry* stack = stackMem + threadIdx.x;
-    if constexpr (Full) {
-        for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
-            HitRec h;
-            const int s = traceRay<T, R, Rr, false, true>(sc, load(i), stack, blockDim.x, h);
-            store(i, s, h);
-        }
-    } else {
-        __shared__ uint32_t fetch;
-        if (threadIdx.x == 0) fetch = 0;
-        __syncthreads();
-        ColdRay<T>* cold = coldRay<T>(sc, stackMem);
-        Traversal<T, R, Rr, false, SharedStack, false, false> tr;
-        const uint64_t share = (n + gridDim.x - 1) / gridDim.x, first = share * blockIdx.x;
-        const uint32_t count = first < n ? uint32_t(share < n - first ? share : n - first) : 0u;
-        uint32_t k = 0;
-        bool alive = false, exhausted = false;
-        for (;;) {
-            const uint32_t next = refillLanes(!alive, &fetch, count, exhausted);
-            if (!alive && next < count) {
-                k = next;
-                tr.begin(load(first + k), stack, blockDim.x, cold);
-                alive = true;
-            }
-            if (__ballot_sync(0xFFFFFFFFu, alive) == 0) break;
-            if (!alive) continue;
-            int s = tr.run(sc, kRefillBudget);
-            if (s == kTraceRunning) continue;
-            HitRec h = cold->hit;
-            if (s == kTraceOverflow) {
-                const DeepResult d = traceRayDeep<T, R, Rr, false, false>(sc.self, tr.query(), h);
-                s = d.status;
-                h = d.hit;
-            }
-            store(first + k, s, h);
-            alive = false;
-        }
+// What a cast reads and writes: rays 0 .. n - 1, each one's query and where its answer goes. Host rays in their
+// pieces:
+template <int M>
+struct HostRays {
+    using T = RT<M>;
+    using Ro = typename Mode<M>::Ro;
+    using Rr = typename Mode<M>::Rr;
+    CastPieces b;
+    __device__ uint64_t n() const { return b.n; }
+    // Ray i's piece: its first ray and how many it has.
+    __device__ uint64_t piece(uint64_t i, uint64_t& m) const {
+        const uint64_t first = i >> b.shift << b.shift, left = b.n - first;
+        m = left < 1ull << b.shift ? left : 1ull << b.shift;
+        return first;
     }
-}
-
-template <int M, bool Full>
-__global__ void OWEC_TRAVERSAL_BOUNDS kCastRays(DeviceScene sc, CastPieces b) {
-    using R = RT<M>;
-    // ray i's origin and direction, in its piece of the batch
-    auto ray = [&](uint64_t i, V3<double>& od, V3<double>& d) {
-        const uint64_t first = i >> b.shift << b.shift, left = b.n - first, piece = 1ull << b.shift;
+    __device__ void ray(const DeviceScene& sc, uint64_t i, V3<double>& od, V3<double>& d) const {
+        uint64_t m;
+        const uint64_t first = piece(i, m);
         const double* o = reinterpret_cast<const double*>(b.rays + 48 * first) + 3 * (i - first);
-        const double* v = o + 3 * (left < piece ? left : piece);
+        const double* v = o + 3 * m;
         od = V3<double>(o[0] - sc.origin[0], o[1] - sc.origin[1], o[2] - sc.origin[2]);
         if (Mode<M>::plainOrigin) od = V3<double>(V3<float>(od));
         d = V3<double>(v[0], v[1], v[2]);
-    };
-    castQueries<R, typename Mode<M>::Ro, typename Mode<M>::Rr, Full>(
-        sc, b.n,
-        [&](uint64_t i) {
-            RayQuery<R> rq;
-            V3<double> d;
-            ray(i, rq.od, d);
-            rq.o = V3<R>(rq.od);
-            rq.d = V3<R>(d);
-            rq.tmax = R(INFINITY);
-            rq.depB = rq.depP = kNone;
-            rq.region = kNone;
-            rq.errN = R(0);
-            return rq;
-        },
-        [&](uint64_t i, int s, const HitRec& h) {
-            const bool hit = s == kTraceHit;
-            double t = hit ? h.t : INFINITY;
-            if (hit && sizeof(typename Mode<M>::Rr) == sizeof(double) && sc.boundaries[h.boundary].shape == OWEC_SHAPE_MESH) {
-                V3<double> od, d;
-                ray(i, od, d);
-                t = refineTriangleT(sc, h.slot, od, d, h.t);
-            }
-            const uint64_t first = i >> b.shift << b.shift, left = b.n - first, piece = 1ull << b.shift;
-            const uint64_t k = i - first, m = left < piece ? left : piece;
-            char* out = b.hits + 16 * first;
-            reinterpret_cast<double*>(out)[k] = t;
-            reinterpret_cast<uint32_t*>(out + 8 * m)[k] = hit ? h.boundary : (s == kTraceOverflow ? kNone - 1u : kNone);
-            reinterpret_cast<uint32_t*>(out + 12 * m)[k] = hit ? h.prim : 0u;
-        });
-}
+    }
+    __device__ RayQuery<T> load(const DeviceScene& sc, uint64_t i) const {
+        RayQuery<T> rq;
+        V3<double> d;
+        ray(sc, i, rq.od, d);
+        rq.o = V3<T>(rq.od);
+        rq.d = V3<T>(d);
+        rq.tmax = T(INFINITY);
+        rq.depB = rq.depP = kNone;
+        rq.region = kNone;
+        rq.errN = T(0);
+        return rq;
+    }
+    __device__ void store(const DeviceScene& sc, uint64_t i, int s, const HitRec& h) const {
+        const bool hit = s == kTraceHit;
+        double t = hit ? h.t : INFINITY;
+        if (hit && sizeof(Rr) == sizeof(double) && sc.boundaries[h.boundary].shape == OWEC_SHAPE_MESH) {
+            V3<double> od, d;
+            ray(sc, i, od, d);
+            t = refineTriangleT(sc, h.slot, od, d, h.t);
+        }
+        uint64_t m;
+        const uint64_t first = piece(i, m), k = i - first;
+        char* out = b.hits + 16 * first;
+        reinterpret_cast<double*>(out)[k] = t;
+        reinterpret_cast<uint32_t*>(out + 8 * m)[k] = hit ? h.boundary : (s == kTraceOverflow ? kNone - 1u : kNone);
+        reinterpret_cast<uint32_t*>(out + 12 * m)[k] = hit ? h.prim : 0u;
+    }
+};
+// Device-resident FP32 camera-relative rays (the benchmark's ray-cast workload):
+struct DeviceRays {
+    using T = float;
+    using Ro = float;
+    using Rr = double;
+    uint64_t count;
+    const float *o, *d;
+    uint32_t *boundary, *prim;
+    float* t;
+    __device__ uint64_t n() const { return count; }
+    __device__ RayQuery<float> load(const DeviceScene&, uint64_t i) const {
+        RayQuery<float> rq;
+        rq.o = V3<float>(o[3 * i], o[3 * i + 1], o[3 * i + 2]);
+        rq.od = V3<double>(rq.o);
+        rq.d = V3<float>(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
+        rq.tmax = INFINITY;
+        rq.depB = rq.depP = kNone;
+        rq.region = kNone;
+        rq.errN = 0.f;
+        return rq;
+    }
+    __device__ void store(const DeviceScene&, uint64_t i, int s, const HitRec& h) const {
+        boundary[i] = s == kTraceHit ? h.boundary : (s == kTraceOverflow ? kNone - 1u : kNone);
+        prim[i] = s == kTraceHit ? h.prim : 0u;
+        t[i] = s == kTraceHit ? float(h.t) : INFINITY;
+    }
+};
 
-// Device-resident FP32 camera-relative rays (the benchmark's ray-cast workload).
-template <bool Full>
-__global__ void OWEC_TRAVERSAL_BOUNDS kCastRaysF(DeviceScene sc, uint64_t n, const float* o, const float* d,
-                                                 uint32_t* boundary, uint32_t* prim, float* t) {
-    castQueries<float, float, double, Full>(
-        sc, n,
-        [&](uint64_t i) {
-            RayQuery<float> rq;
-            rq.o = V3<float>(o[3 * i], o[3 * i + 1], o[3 * i + 2]);
-            rq.od = V3<double>(rq.o);
-            rq.d = V3<float>(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
-            rq.tmax = INFINITY;
-            rq.depB = rq.depP = kNone;
-            rq.region = kNone;
-            rq.errN = 0.f;
-            return rq;
-        },
-        [&](uint64_t i, int s, const HitRec& h) {
-            boundary[i] = s == kTraceHit ? h.boundary : (s == kTraceOverflow ? kNone - 1u : kNone);
-            prim[i] = s == kTraceHit ? h.prim : 0u;
-            t[i] = s == kTraceHit ? float(h.t) : INFINITY;
-        });
+// Every lane runs its rays' queries to their ends.
+template <class Rays, bool Full>
+__device__ __forceinline__ void castWhole(const DeviceScene& sc, const Rays& rays) {
+    extern __shared__ StackEntry stackMem[];
+    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < rays.n(); i += uint64_t(gridDim.x) * blockDim.x) {
+        HitRec h;
+        const int s = traceRay<typename Rays::T, typename Rays::Ro, typename Rays::Rr, false, Full>(
+            sc, rays.load(sc, i), stackMem + threadIdx.x, blockDim.x, h);
+        rays.store(sc, i, s, h);
+    }
+}
+template <class Rays, bool Full>
+__global__ void __launch_bounds__(128) kCastFew(DeviceScene sc, Rays rays) { castWhole<Rays, Full>(sc, rays); }
+template <class Rays, bool Full>
+__global__ void OWEC_TRAVERSAL_BOUNDS kCastWhole(DeviceScene sc, Rays rays) { castWhole<Rays, Full>(sc, rays); }
+
+// As kIntersect: a block takes its share of the rays, and a lane whose query ends takes the share's next ray.
+template <class Rays>
+__global__ void OWEC_TRAVERSAL_BOUNDS kCastRefilled(DeviceScene sc, Rays rays) {
+    using T = typename Rays::T;
+    extern __shared__ StackEntry stackMem[];
+    __shared__ uint32_t fetch;
+    StackEntry* stack = stackMem + threadIdx.x;
+    ColdRay<T>* cold = coldRay<T>(sc, stackMem);
+    if (threadIdx.x == 0) fetch = 0;
+    __syncthreads();
+    Traversal<T, typename Rays::Ro, typename Rays::Rr, false, SharedStack, false, false> tr;
+    const uint64_t n = rays.n(), share = (n + gridDim.x - 1) / gridDim.x, first = share * blockIdx.x;
+    const uint32_t count = first < n ? uint32_t(share < n - first ? share : n - first) : 0u;
+    uint32_t k = 0;
+    bool alive = false, exhausted = false;
+    for (;;) {
+        const uint32_t next = refillLanes(!alive, &fetch, count, exhausted);
+        if (!alive && next < count) {
+            k = next;
+            tr.begin(rays.load(sc, first + k), stack, blockDim.x, cold);
+            alive = true;
+        }
+        if (__ballot_sync(0xFFFFFFFFu, alive) == 0) break;
+        if (!alive) continue;
+        int s = tr.run(sc, kRefillBudget);
+        if (s == kTraceRunning) continue;
+        HitRec h = cold->hit;
+        if (s == kTraceOverflow) {
+            const DeepResult d = traceRayDeep<T, typename Rays::Ro, typename Rays::Rr, false, false>(sc.self, tr.query(), h);
+            s = d.status;
+            h = d.hit;
+        }
+        rays.store(sc, first + k, s, h);
+        alive = false;
+    }
 }
 
 // Primitive records in leaf order (the triangles' camera-relative vertices and identities).
@@ -1221,18 +1238,36 @@ void launchFilm(const DeviceScene& sc, const PassParams& pp, const PathBuffers<R
     else
         kFilm<M><<<(pp.nPixels + 255) / 256, 256, 0, s>>>(sc, pp, pb, film, comp, samples, spp);
 }
-static int castGrid(uint64_t n, int grid) { return int(std::min<uint64_t>(uint64_t(grid), (n + 127) / 128)); }
+// Which cast kernel for n rays. Few: up to the rays that are resident at once at the 146 registers the compiler
+// takes unbounded (three blocks to an SM), where a query's own latency counts, which the bound to 128 and the
+// refills lengthen: 257 rays into the room of 2^17 triangles 47 us, 49 bound, 57 refilled. Whole, at 128
+// registers: to a second wave of blocks, where nothing is left to refill with (65,536 rays: 95 us, against 110
+// unbounded and 103 refilled; 120,000: 184, 175, 200). Refilled beyond: 400,000 rays 300 us with as many blocks as
+// are resident, 333 with twice as many, 354 whole; 2^21 into 2^20 triangles 1.64 ms, against 2.09 whole and
+// 2.39 unbounded. With general shapes a refill waits on the others' numeric roots and contacts, and casts stay
+// whole (2^21 rays, a cone in that room: 5.2 ms, against 6.8 refilled and 6.2 unbounded).
+template <int M, class Rays>
+void launchCast(const DeviceScene& sc, const Rays& rays, uint64_t n, int numSMs, cudaStream_t s) {
+    const size_t smem = traversalSharedBytes(sc, 128);
+    const uint64_t blocks = (n + 127) / 128, sms = uint64_t(numSMs);
+    if (blocks <= 3 * sms) {
+        if (sc.fullFeatures) kCastFew<Rays, true><<<int(blocks), 128, smem, s>>>(sc, rays);
+        else kCastFew<Rays, false><<<int(blocks), 128, smem, s>>>(sc, rays);
+    } else if (sc.fullFeatures) {
+        kCastWhole<Rays, true><<<int(std::min(blocks, 8 * sms)), 128, smem, s>>>(sc, rays);
+    } else if (blocks <= 8 * sms) {
+        kCastWhole<Rays, false><<<int(blocks), 128, smem, s>>>(sc, rays);
+    } else {
+        kCastRefilled<Rays><<<int(4 * sms), 128, persistentSharedBytes<M>(sc, 128), s>>>(sc, rays);
+    }
+}
 template <int M>
-void launchCastRays(const DeviceScene& sc, const CastPieces& b, int grid, cudaStream_t s) {
-    grid = castGrid(b.n, grid);
-    if (sc.fullFeatures) kCastRays<M, true><<<grid, 128, traversalSharedBytes(sc, 128), s>>>(sc, b);
-    else kCastRays<M, false><<<grid, 128, persistentSharedBytes<M>(sc, 128), s>>>(sc, b);
+void launchCastRays(const DeviceScene& sc, const CastPieces& b, int numSMs, cudaStream_t s) {
+    launchCast<M>(sc, HostRays<M>{b}, b.n, numSMs, s);
 }
 void launchCastRaysF(const DeviceScene& sc, uint64_t n, const float* o, const float* d, uint32_t* b, uint32_t* p,
-                     float* t, int grid, cudaStream_t s) {
-    grid = castGrid(n, grid);
-    if (sc.fullFeatures) kCastRaysF<true><<<grid, 128, traversalSharedBytes(sc, 128), s>>>(sc, n, o, d, b, p, t);
-    else kCastRaysF<false><<<grid, 128, persistentSharedBytes<OWEC_PRECISION_MIXED>(sc, 128), s>>>(sc, n, o, d, b, p, t);
+                     float* t, int numSMs, cudaStream_t s) {
+    launchCast<OWEC_PRECISION_MIXED>(sc, DeviceRays{n, o, d, b, p, t}, n, numSMs, s);
 }
 void launchResolve(const double* film, const double* comp, const double* samples, uint32_t nPixels, double* xyz,
                    cudaStream_t s) {

@@ -50,9 +50,9 @@ struct CastPieces {
     int shift;
 };
 template <int M>
-void launchCastRays(const DeviceScene&, const CastPieces&, int grid, cudaStream_t);
+void launchCastRays(const DeviceScene&, const CastPieces&, int numSMs, cudaStream_t);
 void launchCastRaysF(const DeviceScene&, uint64_t n, const float* o, const float* d, uint32_t* b, uint32_t* p, float* t,
-                     int grid, cudaStream_t);
+                     int numSMs, cudaStream_t);
 void launchMaterialize(const uint32_t* leafOrder, uint32_t n, const float4* tri, const double* tri64, PrimRec* prims,
                        PrimRec64* prims64, cudaStream_t);
 

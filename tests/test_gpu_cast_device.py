@@ -25,7 +25,7 @@ def cast_device(c, o, d):
 
 
 @pytest.mark.parametrize("full", [False, True])
-@pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 148 * 8 * 128 - 1, 148 * 8 * 128 + 1, 400001])
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 148 * 3 * 128, 148 * 3 * 128 + 1, 148 * 8 * 128, 148 * 8 * 128 + 1, 400001])
 def test_device_batches_match_their_rays_in_small_calls(n, full):
     sb = scenes.bvh_stress_room(16, 16, 64, 32)
     if full:
