@@ -308,8 +308,9 @@ def c5_study(device, spp_timing=1024, steps=0, spp_step=8, width=1920, height=10
         c.set_heightfield(info["heightfield"], info["base_z"], np.zeros(n * n))
         out["triangles"] = c.bvh_info()["triangles"]
         c.run_pass(1)
-        c.path_adjoint(0, 1, np.zeros((height, width, 3)))  # warm-up: buffers, the replay's stacks
         free1, _ = torch.cuda.mem_get_info(device)
+        c.path_adjoint(0, 1, np.zeros((height, width, 3)))  # warm-up: buffers, the replay's stacks
+        free2, _ = torch.cuda.mem_get_info(device)
         c.reset_film()
         c.set_pass_index(100)
         c.run_pass(spp_timing)
@@ -323,7 +324,10 @@ def c5_study(device, spp_timing=1024, steps=0, spp_step=8, width=1920, height=10
                     "forward_paths_per_s": width * height * spp_timing / fwd,
                     "paths_met_heightfield": st["heightfield"] / max(1, st["paths"]),
                     "dropped_of_those": st["dropped"] / max(1, st["heightfield"]), "faults": st["faults"],
-                    "context_bytes": int(free0 - free1), "adjoint_call_bytes": int(st["device_bytes"]),
+                    # the context with its scene and passes; what its first adjoint adds and keeps (buffers and
+                    # the replay's stacks), of which the call's own buffers
+                    "context_bytes": int(free0 - free1), "adjoint_held_bytes": int(free1 - free2),
+                    "adjoint_call_bytes": int(st["device_bytes"]),
                     "device_total_bytes": int(total)})
         if steps > 0:
             out["optimisation"] = c5_optimise(c, info, n, steps, spp_step, width, height)
@@ -536,7 +540,8 @@ def run_cuda(args):
     ctx.run_pass(1)
     launch_queries = ctx.trace_launch_queries()
     cnt = ctx.trace_counters(0)
-    _, isec_prof, _, launches_prof = ctx.last_pass_timing()
+    # the closest-hit launches of a pass that had paths: one or two more are queued behind the last
+    launches_prof = sum(1 for n in launch_queries if n > 0) or ctx.last_pass_timing()[3]
 
     stats0 = ctx.stats()
     times, isec, shadow = [], [], []
@@ -618,10 +623,11 @@ def run_cuda(args):
         hbm, peak_kind = peaks()
         q, nodes, prims = cnt[0], cnt[1], cnt[2]
         bytes_isec = nodes * NODE_BYTES + prims * PRIM_BYTES + q * RAY_STATE_BYTES
-        # algorithmic bytes of an average launch (from the counting pass's visit counts) over the
-        # average device time of the timed passes' intersect launches
+        # algorithmic bytes of a pass (from the counting pass's visit counts) over the device time of the
+        # timed passes' closest-hit kernels, each from its first thread to its last warp (the shadow kernels
+        # of the bounce before run beside it); both per launch that had paths
         per_launch_bytes = bytes_isec / max(1, launches_prof)
-        per_launch_s = sum(isec) / max(1, launches)
+        per_launch_s = sum(isec) / args.steps / max(1, launches_prof)
         achieved = per_launch_bytes / per_launch_s / 1e9
         # DRAM traffic per launch: the ncu-measured bytes per query (profiles/) times this launch's queries
         traffic = None

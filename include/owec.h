@@ -364,9 +364,11 @@ int owec_set_pass_index(owec_ctx* ctx, uint64_t pass_index);
 /* Discards the film and the pass count (Renderer::resetObserver, src/owe/render/renderer.hpp:60). */
 int owec_reset_film(owec_ctx* ctx);
 int owec_read_stats(owec_ctx* ctx, owec_stats* stats);
-/* Timing of the last owec_pass, measured with CUDA events on the context's stream:
- * out[0] device seconds of the whole pass, out[1] of its closest-hit (intersect) kernels,
- * out[2] of its shadow-ray kernels, out[3] the number of intersect launches. */
+/* Timing of the last owec_pass: out[0] device seconds of the whole pass (CUDA events on the context's
+ * stream), out[1] of its closest-hit (intersect) kernels and out[2] of its shadow-ray kernels (the device's
+ * timer, from a kernel's first thread to its last warp), out[3] the number of intersect launches. A bounce's
+ * shadow kernels run beside the next bounce's intersect kernel, so out[1] + out[2] may exceed out[0]; the
+ * launches include one or two a batch that were queued behind the last bounce and found no paths. */
 int owec_last_pass_timing(owec_ctx* ctx, double out[4]);
 
 /* Closest hits of n rays given in world coordinates (World::intersect,
