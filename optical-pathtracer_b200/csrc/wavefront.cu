@@ -1240,7 +1240,7 @@ void launchFilm(const DeviceScene& sc, const PassParams& pp, const PathBuffers<R
 }
 // Which cast kernel for n rays. Few: up to the rays that are resident at once at the 146 registers the compiler
 // takes unbounded (three blocks to an SM), where a query's own latency counts, which the bound to 128 and the
-// refills lengthen: 257 rays into the room of 2^17 triangles 47 us, 49 bound, 57 refilled. Whole, at 128
+// refills lengthen: 257 rays into the room of 2^16 triangles 47 us, 49 bound, 57 refilled. Whole, at 128
 // registers: to a second wave of blocks, where nothing is left to refill with (65,536 rays: 95 us, against 110
 // unbounded and 103 refilled; 120,000: 184, 175, 200). Refilled beyond: 400,000 rays 300 us with as many blocks as
 // are resident, 333 with twice as many, 354 whole; 2^21 into 2^20 triangles 1.64 ms, against 2.09 whole and
