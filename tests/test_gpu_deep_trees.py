@@ -138,3 +138,57 @@ def test_deep_levels_are_not_traversed_twice(precision):
     deep, nodes = node_visits_per_query(nested_octants(20), precision)
     assert nodes > 100
     assert deep - middle <= 2 * (middle - shallow) + 4, (shallow, middle, deep)
+
+
+def cell_of_triangles(count, shallow=False):
+    """Octants nested over twenty octaves of 10 km, and `count` triangles in a row along the diagonal of the smallest
+    one's corner, all within one Morton cell: split by their order, they add six levels of their own."""
+    v = 1e4 * nested_vertices(20)
+    s = 1e4 * 2.0 ** -23  # about a millimetre: a quarter of a cell
+    at = (np.arange(count) + 0.5)[:, None] / count * s * np.ones(3)
+    size = 0.3 * s / count
+    row = np.stack([at, at + [size, 0.0, -size], at + [-size, size, 0.0]], 1).reshape(-1, 3)
+    v = np.concatenate([v, row])
+    if shallow:
+        v = np.concatenate([v, np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0]]) - [0.0, 0.0, 1e11]])
+    sb = scenes.SceneBuilder()
+    sb.boundary(A.SHAPE_MESH, [], scenes.pose(), 0, 0, sb.diffuse(0.5), -1,
+                sb.mesh(v, np.arange(len(v), dtype=np.uint32).reshape(-1, 3)))
+    sb.uniform_sky(1.0)
+    e = 1e4 * 2.0 ** -25
+    sb.observer(16, 16, (-1.0 * e, -1.1 * e, -0.9 * e), (1e4, 1e4, 1e4), fov_y_deg=4.0)
+    sb.frame_origin((0.0, 0.0, 0.0))
+    return sb.desc()
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_levels_beyond_the_shared_stack(precision):
+    """More pending levels than the shared stack ever holds: the query starts again with the deep one."""
+    count = 8 ** 6
+    rng = np.random.default_rng(3)
+    n = 512
+    e = 1e4 * 2.0 ** -25
+    o = -e * rng.uniform(0.5, 1.5, (n, 3))
+    d = 1.0 + 0.02 * rng.uniform(-1.0, 1.0, (n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    got = []
+    for shallow in (False, True):
+        with owe_cuda.Context(0) as c:
+            c.set_settings(A.make_settings(precision=precision))
+            c.upload(cell_of_triangles(count, shallow))
+            got.append(c.cast_rays(o, d))
+    (b0, p0, t0), (b1, p1, t1) = got
+    assert np.array_equal(b0, b1) and (b0 < 1).any()
+    if precision != A.PRECISION_MIXED:
+        assert np.array_equal(t0, t1)
+    if precision == A.PRECISION_FP64:
+        assert np.array_equal(p0, p1)
+    desc = cell_of_triangles(count)
+    few, _ = node_visits_per_query(cell_of_triangles(1), precision)
+    many, _ = node_visits_per_query(desc, precision)
+    print("node visits per query", few, many)
+    with owe_cuda.Context(0) as c:
+        c.upload(desc)
+        c.set_settings(A.make_settings(seed=5, max_depth=3, precision=precision))
+        c.run_pass(1)
+        assert c.stats()["device_faults"] == 0
