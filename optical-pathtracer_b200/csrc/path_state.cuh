@@ -129,12 +129,13 @@ static_assert(sizeof(ShadowRay<float>) == 96, "a mixed-precision shadow record s
 // global timer, from a kernel's first thread to its last warp. The two kinds overlap: a bounce's shadow
 // kernels run beside the next bounce's closest-hit kernel.
 struct BounceClock {
-    unsigned long long intersectStart, intersect, shadowStart, shadow;
+    unsigned long long intersect, shadow;
 };
 
 // Counters of one bounce; every bounce of a batch has its own set, all cleared at once before it.
-constexpr int kCountActive = 0, kWarpsIntersect = 1, kCountSurface = 2, kCountShadow = 3, kFetchIntersect = 4, kFetchShadow = 5,
-              kCountSimple = 6, kWarpsShadow = 7, kBounceCounters = 8, kCountNext = kBounceCounters + kCountActive;
+constexpr int kCountActive = 0, kCountSurface = 2, kCountShadow = 3, kFetchIntersect = 4, kFetchShadow = 5, kCountSimple = 6,
+              kClockIntersect = 8, kClockShadow = 10,  // 64-bit words (stampStart)
+              kBounceCounters = 12, kCountNext = kBounceCounters + kCountActive;
 // The paths a bounce started with, as the closest-hit kernel reports them to the host (Queues::progress):
 // the bounce's number in the upper half, so that a stale word is never taken for it.
 constexpr int kProgressSlots = 64;
@@ -156,23 +157,26 @@ __device__ __forceinline__ unsigned long long globalTimer() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+__device__ __forceinline__ bool firstThread() { return blockIdx.x == 0 && threadIdx.x == 0; }
+// A kernel's time in one 64-bit word of its bounce's counters: the first thread adds the time it starts at (modulo
+// 2^44 ns) above kClockBits, one lane of each warp adds one at the warp's end, and the last one finds the start
+// beside the count. One word needs no fence, which cost the FP32 room half a percent of a pass.
+constexpr int kClockBits = 20;
+__device__ __forceinline__ void stampStart(uint32_t* word) {
+    atomicAdd(reinterpret_cast<unsigned long long*>(word), globalTimer() << kClockBits);
+}
+__device__ __forceinline__ void stampEnd(uint32_t* word, unsigned long long& sum) {
+    const unsigned long long before = atomicAdd(reinterpret_cast<unsigned long long*>(word), 1ull);
+    if ((before & ((1ull << kClockBits) - 1)) + 1 != gridDim.x * (blockDim.x >> 5)) return;
+    sum += (globalTimer() - (before >> kClockBits)) & (~0ull >> kClockBits);
+}
 // The first thread of a bounce's closest-hit kernel, and of its first shadow kernel.
 __device__ __forceinline__ void stampIntersect(const Queues& q) {
     *reinterpret_cast<volatile unsigned long long*>(q.progress) = (uint64_t(q.bounce) << 32) | q.counts[kCountActive];
-    if (q.clock) q.clock->intersectStart = globalTimer();
+    if (q.clock) stampStart(q.counts + kClockIntersect);
 }
 __device__ __forceinline__ void stampShadow(const Queues& q) {
-    if (q.clock) q.clock->shadowStart = globalTimer();
-}
-__device__ __forceinline__ bool firstThread() { return blockIdx.x == 0 && threadIdx.x == 0; }
-// One lane of each warp of a kernel at its end, counted in warps: the last one adds the time since start. The first
-// thread, which may have stamped that, orders its stamp before its count (a fence in every warp cost the gallery
-// and the glass sphere 1 to 3 % of a pass).
-__device__ __forceinline__ void stampEnd(uint32_t* warps, const unsigned long long& start, unsigned long long& sum) {
-    if (firstThread()) __threadfence();
-    if (atomicAdd(warps, 1u) + 1 != gridDim.x * (blockDim.x >> 5)) return;
-    __threadfence();
-    sum += globalTimer() - *const_cast<const volatile unsigned long long*>(&start);
+    if (q.clock) stampStart(q.counts + kClockShadow);
 }
 #endif
 

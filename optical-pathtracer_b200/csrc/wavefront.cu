@@ -165,7 +165,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kIntersect(DeviceScene sc, PathBuffers<RT<
     }
     warpFlush(&st->segments, segments);
     warpFlush(&st->faults, faults);
-    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kWarpsIntersect, q.clock->intersectStart, q.clock->intersect);
+    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kClockIntersect, q.clock->intersect);
 }
 
 // ------------------------------------------------------------------ next-event estimation
@@ -771,7 +771,7 @@ __global__ void OWEC_TRAVERSAL_BOUNDS kShadow(DeviceScene sc, PassParams pp, Pat
     }
     warpFlush(&st->shadowRays, rays);
     warpFlush(&st->faults, faults);
-    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kWarpsShadow, q.clock->shadowStart, q.clock->shadow);
+    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kClockShadow, q.clock->shadow);
 }
 
 // Without null boundaries a shadow ray is one any-hit query, and its bookkeeping (the medium's
@@ -875,7 +875,7 @@ __global__ void __launch_bounds__(256) kShadowApply(DeviceScene sc, PathBuffers<
         warpCount(&st->shadowRays, true);
         warpCount(&st->faults, v == 2);
     }
-    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kWarpsShadow, q.clock->shadowStart, q.clock->shadow);
+    if (q.clock && (threadIdx.x & 31) == 0) stampEnd(q.counts + kClockShadow, q.clock->shadow);
 }
 
 // ------------------------------------------------------------------ film
